@@ -120,6 +120,11 @@ cudaError_t launch_sub(evp1d_t *h, int from, bool last, bool after_sub) {
   return cudaGetLastError();
 }
 
+// Subcycles from which a call takes the resident launch: a single subcycle
+// costs as much in either form (about 11 us with its launch), and its results
+// would land in the set that other blocks still read.
+constexpr int kResidentMin = 2;
+
 // A bounded device-side wait that ran out leaves a code in the error word.
 int check_device_error(evp1d_t *h) {
   int code = 0;
@@ -282,6 +287,23 @@ int init_common(evp1d_t **handle, int na, int navel, const int32_t *const idx[6]
                   first.c_str());
   }
 
+  // The resident plan, unless a setting of the subcycle kernel asks for that
+  // kernel (EVP1D_RESIDENT=0: never)
+  evp::ResidentPlan res;
+  bool resident = g_tile_points.load() == evp::kTileCompute;
+  for (const char *name : {"EVP1D_PATH", "EVP1D_PERSIST", "EVP1D_PDL", "EVP1D_COMPACT", "EVP1D_RUNS",
+                           "EVP1D_STRIP_W", "EVP1D_PREFETCH", "EVP1D_TRACE"})
+    resident = resident && !getenv(name);
+  if (const char *e = getenv("EVP1D_RESIDENT")) resident = resident && atoi(e) != 0;
+  if (resident && evp::build_resident_plan(na, nbp, plan, sms, &res) &&
+      getenv("EVP1D_CHECK_PLAN")) {
+    std::string first;
+    const long long bad = evp::verify_resident_plan(res, na, nbp, plan, &first);
+    if (bad)
+      return fail(EVP1D_ERR_INDEX, "resident plan: %lld violations, the first: %s", bad,
+                  first.c_str());
+  }
+
   evp1d_t *h = new evp1d_handle();
   h->p = to_params(*params);
   if (const char *e = getenv("EVP1D_PATH")) {
@@ -297,13 +319,14 @@ int init_common(evp1d_t **handle, int na, int navel, const int32_t *const idx[6]
     const int v = atoi(e);
     h->prefetch = v < 0 ? 0 : (v > 8 ? 8 : v);
   }
-  int rc = evp::problem_create(&h->d, device, plan, geo);
+  int rc = evp::problem_create(&h->d, device, plan, res, geo);
   if (rc != EVP1D_OK) {
     evp::problem_destroy(&h->d);
     if (h->trace) cudaFree(h->trace);
     delete h;
     return rc;
   }
+  h->resident = h->d.res_blocks > 0;
   // EVP1D_PERSIST=1: a call's subcycles in one launch where the device keeps
   // every run's CTA resident (asked after problem_create has allowed the
   // kernel's shared memory).  Off by default: on grid1600x1200 it measured
@@ -504,6 +527,15 @@ int evp1d_upload(evp1d_t *h, const evp1d_fields *io) {
 
 }  // extern "C"
 
+namespace evp {
+bool use_resident(const evp1d_handle *h, int n) {
+  if (h->path != kPathTma || !h->resident || n < kResidentMin) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->d.stream, &cs) == cudaSuccess &&
+         cs == cudaStreamCaptureStatusNone;
+}
+}  // namespace evp
+
 namespace {
 // ndte subcycles; `ends` = the last one ends the call (writes strintx,
 // strinty, Cb and str).
@@ -514,6 +546,17 @@ int run_subcycles(evp1d_t *h, int ndte, bool ends) {
   if (h->d.ntiles == 0 || ndte == 0) return EVP1D_OK;
   CHECK(select_device(h));
   cudaStream_t st = h->d.stream;
+  if (evp::use_resident(h, ndte)) {
+    // the state on chip for the whole call; the sets alternate as if each
+    // subcycle had been a launch of its own
+    DeviceProblem &d = h->d;
+    const int c = d.cur, to = (ndte & 1) ? 1 - c : c;
+    CUDA_TRY(evp::problem_launch_resident(&d, h->p, ndte, ends, d.stress[c], d.stress[to], d.u[c],
+                                          d.v[c], d.u[to], d.v[to], 0));
+    d.cur = to;
+    h->launches++;
+    return EVP1D_OK;
+  }
   if (h->path == kPathTma && h->persist && ndte > 1) {
     // the whole call in one launch; the per-tile counters start at zero
     CUDA_TRY(cudaMemsetAsync(h->d.epoch, 0, sizeof(unsigned) * (size_t)h->d.ntiles, st));
@@ -707,14 +750,15 @@ int evp1d_autotune(evp1d_t *h, int nsub, char *chosen, int len) {
   copy_all(true);
   struct Cand {
     int path, prefetch;
-    bool persist;
+    bool persist, resident;
   };
   // the multi-subcycle launch (EVP1D_PERSIST) stays a caller's choice: it is
   // far slower with the strip-ordered runs
-  const Cand all[] = {{kPathTma, 0, false}, {kPathTma, 2, false}, {kPathFused, 0, false}};
-  std::vector<Cand> cands(all, all + 3);
+  const Cand all[] = {{kPathTma, 0, false, false}, {kPathTma, 2, false, false},
+                      {kPathFused, 0, false, false}, {kPathTma, 0, false, true}};
+  std::vector<Cand> cands(all, all + (d.res_blocks > 0 ? 4 : 3));
   const int old_path = h->path, old_pf = h->prefetch;
-  const bool old_persist = h->persist;
+  const bool old_persist = h->persist, old_resident = h->resident;
   int best = -1;
   float best_ms = 0.f;
   cudaEvent_t e0, e1;
@@ -725,6 +769,7 @@ int evp1d_autotune(evp1d_t *h, int nsub, char *chosen, int len) {
     h->path = cands[c].path;
     h->prefetch = cands[c].prefetch;
     h->persist = cands[c].persist;
+    h->resident = cands[c].resident;
     drop_graphs(h);
     rc = evp1d_subcycles(h, 2);  // warm-up (also builds nothing: < one chunk)
     if (rc == EVP1D_OK) {
@@ -757,16 +802,18 @@ int evp1d_autotune(evp1d_t *h, int nsub, char *chosen, int len) {
     h->path = old_path;
     h->prefetch = old_pf;
     h->persist = old_persist;
+    h->resident = old_resident;
     return rc != EVP1D_OK ? rc : fail(EVP1D_ERR_CUDA, "autotune found no candidate");
   }
   CHECK(check_device_error(h));
   h->path = cands[best].path;
   h->prefetch = cands[best].prefetch;
   h->persist = cands[best].persist;
+  h->resident = cands[best].resident;
   char buf[128];
   snprintf(buf, sizeof buf, "%s%s prefetch=%d (%.2f us/subcycle)",
            h->path == kPathTma ? "fused-tile-tma" : "fused-tile",
-           h->persist ? " multi-subcycle" : "", h->prefetch, 1000.0 * best_ms / nsub);
+           h->resident ? " resident" : h->persist ? " multi-subcycle" : "", h->prefetch, 1000.0 * best_ms / nsub);
   h->tuned = buf;
   if (chosen && len > 0) {
     strncpy(chosen, buf, (size_t)len - 1);

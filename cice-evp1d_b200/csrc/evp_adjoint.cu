@@ -549,6 +549,12 @@ void launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], doubl
                    double *tv0, size_t entry_step, int len, bool last) {
   DeviceProblem &d = h->d;
   if (len <= 0) return;
+  if (use_resident(h, len)) {
+    problem_launch_resident(&d, h->p, len, last, s0, (len & 1) ? s1 : s0, tu0, tv0, tu0, tv0,
+                            entry_step);
+    h->launches++;
+    return;
+  }
   if (h->path == kPathTma && h->persist && len > 1) {
     cudaMemsetAsync(d.epoch, 0, sizeof(unsigned) * (size_t)d.ntiles, d.stream);
     TmaArgs a = problem_tma_args(d, 0);

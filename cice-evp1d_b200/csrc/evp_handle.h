@@ -16,6 +16,10 @@ void adjoint_release(AdjointState *a);
 void exchange_release(evp1d_handle *h);
 // Forget the recorded forward (the inputs or parameters changed).
 void adjoint_invalidate(AdjointState *a);
+// Whether a call of n subcycles, queued now on the handle's stream, takes the
+// resident launch.  Not under stream capture: its mailbox numbers are launch
+// arguments, and a replay would find the previous replay's messages.
+bool use_resident(const evp1d_handle *h, int n);
 }  // namespace evp
 
 // Kernel paths of the fused subcycle.
@@ -29,6 +33,9 @@ struct evp1d_handle {
   // TMA path: a call's subcycles in one launch whose CTAs stay resident
   // (cooperative), instead of one launch per subcycle in CUDA graphs
   bool persist = false;
+  // TMA path: calls of at least kResidentMin subcycles in one launch that
+  // keeps the state on chip (d.res_blocks > 0)
+  bool resident = false;
   // TMA path: each subcycle's launch after the first of a call (and of a
   // captured chunk) is a programmatic dependent of the one before, so that
   // its prologue overlaps the previous launch's last tiles (EVP1D_PDL=0

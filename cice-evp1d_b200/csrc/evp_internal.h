@@ -10,6 +10,7 @@
 
 #include "evp1d.h"
 #include "evp_kernels.cuh"
+#include "evp_resident.h"
 #include "evp_tiles.h"
 
 namespace evp {
@@ -83,12 +84,18 @@ struct DeviceProblem {
   double *str[8] = {};
   double *stage = nullptr;  // reference-order staging, 32 x navel doubles
   int cur = 0;              // buffer holding the current state
+  // resident plan (evp_resident.h), res_blocks == 0: none
+  int res_blocks = 0, res_threads = 0, res_cls = 0;
+  int32_t *res_slot = nullptr, *res_cnt = nullptr, *res_corner = nullptr;
+  uint32_t *res_str = nullptr;
+  double4 *res_mail = nullptr;  // 2 x nslots velocity mailboxes
+  unsigned res_seq = 1;         // number of the next launch's first subcycle
 };
 
 // Allocate and fill the static part from a tile plan and reference-order
 // geometry (host).  Creates the stream.
 int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
-                   const double *const geo[kNumGeo]);
+                   const ResidentPlan &res, const double *const geo[kNumGeo]);
 void problem_destroy(DeviceProblem *d);
 
 // Per-call fields host -> device (through the staging area); str zeroed;
@@ -115,6 +122,13 @@ int problem_download(DeviceProblem *d, const evp1d_fields *io);
 DevState problem_inplace_view(const DeviceProblem &d);
 FusedArgs problem_fused_args(const DeviceProblem &d, int from);
 TmaArgs problem_tma_args(const DeviceProblem &d, int from);
+// One resident launch of nsub subcycles from the state (u_in, v_in, s_in) to
+// s_out and, uv_step == 0, (u_out, v_out); see ResidentArgs.  Takes nsub
+// mailbox numbers.
+cudaError_t problem_launch_resident(DeviceProblem *d, const Params &p, int nsub, bool last,
+                                    double *const s_in[12], double *const s_out[12],
+                                    const double *u_in, const double *v_in, double *u_out,
+                                    double *v_out, size_t uv_step);
 // Read and clear the device error word (0 if no bounded wait ran out).
 int problem_take_error(DeviceProblem *d, int *code);
 

@@ -187,6 +187,37 @@ cudaError_t launch_tma(const TmaArgs &a, const Params &p, cudaStream_t st);
 // with one CTA per run resident on every SM).
 bool tma_can_persist(int device, int nruns);
 
+// ---- a call's subcycles in one launch, state on chip (evp_kernels_resident.cu)
+struct ResidentArgs {
+  int nslots = 0;
+  // the resident plan (evp_resident.h)
+  const int32_t *slot = nullptr, *cnt = nullptr, *corner = nullptr;
+  const uint32_t *str_idx = nullptr;
+  const uint8_t *flags = nullptr;
+  const double *sg[7] = {};   // dxT, dyT, HTE, HTN, HTEm1, HTNm1, strength by slot
+  const double *uf[kTmaStepuFields] = {};  // the stepu inputs by slot, order as above
+  const double *s_in[12] = {};
+  double *s_out[12] = {};     // may be s_in when nsub >= 2
+  const double *u_in = nullptr, *v_in = nullptr;
+  // uv_step == 0: the final velocities; else subcycle k's result goes to
+  // u_out + (k + 1) * uv_step (the adjoint's tape; u_in is its entry 0)
+  double *u_out = nullptr, *v_out = nullptr;
+  size_t uv_step = 0;
+  // written on the last subcycle when `last` is set
+  double *strintx = nullptr, *strinty = nullptr, *Cb = nullptr;
+  double *str_out[8] = {};
+  int nsub = 1;
+  bool last = false;
+  double4 *mail = nullptr;    // 2 x nslots mailboxes
+  unsigned seq = 0;           // number of the launch's first subcycle
+  int *err = nullptr;
+};
+// Enable the variant of width class `cls` and tell whether `nblocks` of its
+// CTAs are resident at once (1) or the plan cannot run here (0).
+int resident_prepare(int device, int cls, int nblocks);
+cudaError_t launch_resident(const ResidentArgs &a, const Params &p, int cls, int threads,
+                            int nblocks, cudaStream_t st);
+
 // ---- layout conversion between the reference 1D order and slots ----------
 constexpr int kMaxBatch = 32;
 struct PermBatch {

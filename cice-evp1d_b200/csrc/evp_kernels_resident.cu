@@ -1,0 +1,486 @@
+// evp_kernels_resident.cu -- a call's subcycles in one launch, for problems
+// small enough to stay on chip (evp_resident.h).
+//
+// One CTA per block of the resident plan, one thread per compute point (owned
+// points, then the forward halo).  A thread keeps its point's 12 stresses in
+// registers (kSmemStress: in shared memory) and its constants in shared memory
+// from the first subcycle to the last; only velocities move between blocks.
+// Per subcycle:
+//   stress  reads the corner velocities from shared memory, or, where another
+//           block owns the point, from that point's mailbox; writes six of
+//           str1..str8 to the block's str table (str1 and str5 are read only
+//           by their own point and stay in its registers);
+//   barrier
+//   stepu   (owned points) writes the new velocity to shared memory and, for
+//           a point other blocks read, to its mailbox;
+//   barrier
+// A mailbox is 32 bytes in L2: the four 32-bit halves of u and v, each beside
+// the 32-bit number of the subcycle they belong to.  A 64-bit access is
+// atomic, so a word whose number matches carries its half: the reader polls
+// the data themselves, and a subcycle's exchange costs one trip to L2 each
+// way, with no fence, no flag and no barrier between blocks.  Numbers grow
+// across launches, so that nothing stale ever matches.  Each point has two
+// mailboxes, for even and odd subcycles.  One can be written again without
+// looking: a block writes number n+2 only after it has read number n+1 from
+// every block it reads from; those had then passed the barrier after their
+// stress n, and they include every block that reads this one (the plan
+// requires the symmetry).
+// The CTAs wait on one another, so the launch is cooperative (all resident or
+// none).  Every wait is bounded: on expiry the code goes to the error word,
+// the CTA leaves together at the next barrier, and its neighbours' waits run
+// out in turn.
+//
+// What bounds it: the FP64 pipe (about 535 operations a point, two issue
+// cycles each, 64 lanes an SM) for full blocks, the dependent chain through
+// stress, stepu and the exchange for small ones; no HBM traffic per subcycle.
+// Measured, us per subcycle, against the one-launch-per-subcycle kernel:
+// 2.0k points 3.0 / 4.8, 18k 3.5 / 5.0, 51k 3.6 / 7.8, 64k 4.2 / 8.0,
+// 74k 6.4 / 10.4.
+#include <cstdint>
+
+#include "evp_kernels.cuh"
+#include "evp_resident.h"
+
+namespace evp {
+
+namespace {
+
+constexpr int kResGeo = 10;  // dxT dyT cxp cyp cxm cym DminTarea dxhy dyhx strength
+constexpr unsigned long long kResWaitNs = 2000000000ull;  // 2 s
+constexpr int kResCode = 15;
+
+template <int NT, bool kSmemStress>
+struct ResSmem {
+  double2 uv[NT];           // velocities of the owned points
+  double2 str[3][NT + 1];   // (str2, str7), (str3, str6), (str4, str8); [NT] stays 0
+  double geo[kResGeo][NT];
+  double cst[kTmaStepuFields][NT];
+  double s[kSmemStress ? 12 : 1][kSmemStress ? NT : 1];
+};
+
+__device__ __forceinline__ void mail_put(double4 *box, double u, double v, unsigned seq) {
+  const unsigned long long a = (unsigned long long)__double_as_longlong(u);
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long n = (unsigned long long)seq << 32;
+  const unsigned long long m = 0xffffffffull;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(box), "l"((a & m) | n),
+               "l"((a >> 32) | n)
+               : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0+16], {%1, %2};" ::"l"(box), "l"((b & m) | n),
+               "l"((b >> 32) | n)
+               : "memory");
+}
+
+struct Mail {
+  unsigned long long a0, a1, b0, b1;
+};
+
+__device__ __forceinline__ Mail mail_get(const double4 *box) {
+  Mail w;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+               : "=l"(w.a0), "=l"(w.a1)
+               : "l"(box)
+               : "memory");
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2+16];"
+               : "=l"(w.b0), "=l"(w.b1)
+               : "l"(box)
+               : "memory");
+  return w;
+}
+
+__device__ __forceinline__ bool mail_is(const Mail &w, unsigned seq) {
+  return (unsigned)(w.a0 >> 32) == seq && (unsigned)(w.a1 >> 32) == seq &&
+         (unsigned)(w.b0 >> 32) == seq && (unsigned)(w.b1 >> 32) == seq;
+}
+
+__device__ __forceinline__ double2 mail_value(const Mail &w) {
+  const unsigned long long m = 0xffffffffull;
+  return make_double2(__longlong_as_double((long long)((w.a0 & m) | (w.a1 << 32))),
+                      __longlong_as_double((long long)((w.b0 & m) | (w.b1 << 32))));
+}
+
+__device__ __forceinline__ unsigned long long res_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Keeps the compiler from moving shared-memory accesses across: the lean
+// stress below is written so that few values are live at once.
+__device__ __forceinline__ void hold() { asm volatile("" ::: "memory"); }
+
+// stress_update (evp_math.cuh) on a point's 12 stresses in shared memory
+// (`s`, `stride` doubles apart), for the widths that leave a thread 96
+// registers: corner by corner, then the x and the y half of str_combine with
+// the stresses read again.  Every operation is stress_update's own, in its
+// order (corner_strain and corner_update; the sums of str_combine), so the
+// bits are the same.
+template <bool kStd>
+__device__ __forceinline__ void stress_lean(double *s, int stride, double (&out)[8],
+                                            const double2 (&w)[4], const double *geo, int gs,
+                                            const Params &p) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int p2 = k ^ 1, p4 = 3 - k;
+    Geom g;
+    g.dxT = geo[0 * gs];
+    g.dyT = geo[1 * gs];
+    g.cxp = geo[2 * gs];
+    g.cyp = geo[3 * gs];
+    g.cxm = geo[4 * gs];
+    g.cym = geo[5 * gs];
+    double div, ten, shr, Delta;
+    corner_strain(k, w[k].x, w[k].y, w[p2].x, w[p2].y, w[p4].x, w[p4].y, g, p.e_factor, div, ten,
+                  shr, Delta);
+    const double strength = geo[9 * gs], least = geo[6 * gs];
+    double sp = s[k * stride], sm = s[(4 + k) * stride], st = s[(8 + k) * stride];
+    if (kStd && least > 0.0 && fabs(strength) < 1e300 * least && Delta == Delta) {
+      const double z = strength / fmax_ref(Delta, least);
+      const double r = z * Delta;
+      const double e = p.epp2i * z;
+      sp = (sp + p.arlx1i * (z * div - r)) * p.denom1;
+      sm = (sm + p.arlx1i * e * ten) * p.denom1;
+      st = (st + p.arlx1i * kP5 * e * shr) * p.denom1;
+    } else {
+      corner_update(sp, sm, st, div, ten, shr, Delta, strength, least, p);
+    }
+    s[k * stride] = sp;
+    s[(4 + k) * stride] = sm;
+    s[(8 + k) * stride] = st;
+    hold();
+  }
+#pragma unroll
+  for (int half = 0; half < 2; half++) {
+    double A[4], D[4];
+    {
+      const double a0 = s[0], a1 = s[stride], a2 = s[2 * stride], a3 = s[3 * stride];
+      const double b0 = s[4 * stride], b1 = s[5 * stride], b2 = s[6 * stride],
+                   b3 = s[7 * stride];
+      const double d = kP25 * geo[(half == 0 ? 1 : 0) * gs];  // dyT for x, dxT for y
+      const double pa = half == 0 ? a0 + a1 : a0 + a3, pb = half == 0 ? a2 + a3 : a1 + a2;
+      const double ma = half == 0 ? b0 + b1 : b0 + b3, mb = half == 0 ? b2 + b3 : b1 + b2;
+      const double strp = d * (kP333 * pa + kP166 * pb), strm = d * (kP333 * ma + kP166 * mb);
+      const double strq = d * (kP333 * pb + kP166 * pa), strn = d * (kP333 * mb + kP166 * ma);
+      if (half == 0) {
+        A[0] = -strp - strm;
+        A[1] = strp + strm;
+        A[2] = -strq - strn;
+        A[3] = strq + strn;
+      } else {
+        A[0] = -strp + strm;
+        A[1] = strp - strm;
+        A[2] = -strq + strn;
+        A[3] = strq - strn;
+      }
+      const double p1 = (a0 + a2) * kP055, p2 = (a1 + a3) * kP055;
+      const double m1 = (b0 + b2) * kP055, m2 = (b1 + b3) * kP055;
+      const double pne = kP111 * a0 + p2 + kP027 * a2, pnw = kP111 * a1 + p1 + kP027 * a3;
+      const double psw = kP111 * a2 + p2 + kP027 * a0, pse = kP111 * a3 + p1 + kP027 * a1;
+      const double mne = kP111 * b0 + m2 + kP027 * b2, mnw = kP111 * b1 + m1 + kP027 * b3;
+      const double msw = kP111 * b2 + m2 + kP027 * b0, mse = kP111 * b3 + m1 + kP027 * b1;
+      if (half == 0) {  // str1..4: ne, nw, se, sw
+        D[0] = -pne + mne;
+        D[1] = -pnw + mnw;
+        D[2] = -pse + mse;
+        D[3] = -psw + msw;
+      } else {  // str5..8: ne, se, nw, sw
+        D[0] = pne + mne;
+        D[1] = pse + mse;
+        D[2] = pnw + mnw;
+        D[3] = psw + msw;
+      }
+    }
+    hold();
+    const double c0 = s[8 * stride], c1 = s[9 * stride], c2 = s[10 * stride], c3 = s[11 * stride];
+    const double t1 = (c0 + c2) * kP111, t2 = (c1 + c3) * kP111;
+    const double tne = kP222 * c0 + t2 + kP055 * c2, tnw = kP222 * c1 + t1 + kP055 * c3;
+    const double tsw = kP222 * c2 + t2 + kP055 * c0, tse = kP222 * c3 + t1 + kP055 * c1;
+    const double dxhy = geo[7 * gs], dyhx = geo[8 * gs];
+    const double h = kP5 * geo[(half == 0 ? 0 : 1) * gs];  // dxT for x, dyT for y
+    const double ta = half == 0 ? c0 + c3 : c0 + c1;       // e, n
+    const double tb = half == 0 ? c1 + c2 : c2 + c3;       // w, s
+    const double ew = h * (kP333 * ta + kP166 * tb), we = h * (kP333 * tb + kP166 * ta);
+    if (half == 0) {
+      out[0] = A[0] - ew + dxhy * D[0] + dyhx * tne;
+      out[1] = A[1] - we + dxhy * D[1] + dyhx * tnw;
+      out[2] = A[2] + ew + dxhy * D[2] + dyhx * tse;
+      out[3] = A[3] + we + dxhy * D[3] + dyhx * tsw;
+    } else {
+      out[4] = A[0] - ew - dyhx * D[0] + dxhy * tne;
+      out[5] = A[1] - we - dyhx * D[1] + dxhy * tse;
+      out[6] = A[2] + ew - dyhx * D[2] + dxhy * tnw;
+      out[7] = A[3] + we - dyhx * D[3] + dxhy * tsw;
+    }
+    hold();
+  }
+}
+
+template <int NT, bool kStd, bool kSmemStress>
+__global__ void __launch_bounds__(NT, 1) k_resident(ResidentArgs a, Params p) {
+  extern __shared__ __align__(16) unsigned char res_raw[];
+  using S_t = ResSmem<NT, kSmemStress>;
+  S_t &S = *reinterpret_cast<S_t *>(res_raw);
+  const int c = threadIdx.x;
+  const size_t at = (size_t)blockIdx.x * blockDim.x + c;
+  const int slot = a.slot[at];
+  const bool own = c < a.cnt[blockIdx.x];
+  const uint32_t nbr = a.str_idx[at];
+  const uint8_t fl = slot >= 0 ? a.flags[slot] : (uint8_t)(kSkipT | kSkipU);
+  const bool actT = !(fl & kSkipT), actU = own && !(fl & kSkipU);
+  const bool exported = own && (nbr & kResExport);
+
+  // ---- the point's constants and state ------------------------------------
+  int ref[4] = {0, 0, 0, 0};
+  double sreg[12];
+  if (slot >= 0) {
+    const int4 q = reinterpret_cast<const int4 *>(a.corner)[at];
+    ref[0] = q.x;
+    ref[1] = q.y;
+    ref[2] = q.z;
+    ref[3] = q.w;
+    const Geom g = make_geom(a.sg[0][slot], a.sg[1][slot], a.sg[2][slot], a.sg[3][slot],
+                             a.sg[4][slot], a.sg[5][slot], p.deltaminEVP);
+    S.geo[0][c] = g.dxT;
+    S.geo[1][c] = g.dyT;
+    S.geo[2][c] = g.cxp;
+    S.geo[3][c] = g.cyp;
+    S.geo[4][c] = g.cxm;
+    S.geo[5][c] = g.cym;
+    S.geo[6][c] = g.DminTarea;
+    S.geo[7][c] = g.dxhy;
+    S.geo[8][c] = g.dyhx;
+    S.geo[9][c] = a.sg[6][slot];
+#pragma unroll
+    for (int k = 0; k < 12; k++) sreg[k] = a.s_in[k][slot];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 12; k++) sreg[k] = 0.0;
+  }
+  if (own) {
+#pragma unroll
+    for (int k = 0; k < kTmaStepuFields; k++) S.cst[k][c] = a.uf[k][slot];
+    S.uv[c] = make_double2(a.u_in[slot], a.v_in[slot]);
+  }
+  if constexpr (kSmemStress) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) S.s[k][c] = sreg[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    S.str[k][c] = make_double2(0.0, 0.0);  // skipped T points keep str = 0
+    if (c == 0) S.str[k][NT] = make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+
+  unsigned polled = 0;  // corners whose velocity another block owns
+#pragma unroll
+  for (int k = 0; k < 4; k++) polled |= (ref[k] < 0 && ~ref[k] < a.nslots) ? 1u << k : 0u;
+  bool fail = false;
+  double2 own_str = make_double2(0.0, 0.0);  // str1, str5
+  for (int sub = 0; sub < a.nsub; sub++) {
+    const bool wlast = a.last && sub == a.nsub - 1;
+    // ---- stress ------------------------------------------------------------
+    if (actT) {
+      double2 w[4];
+      // Velocities other blocks own: the corners are polled together, so that a
+      // round of reads costs one trip to L2; the words stay as they came until
+      // every corner has its own (fewer registers than the values beside them).
+      Mail m[4];
+      if (sub > 0 && polled) {
+        const unsigned seq = a.seq + (unsigned)sub;
+        const double4 *box = a.mail + (size_t)(sub & 1) * (size_t)a.nslots;
+        unsigned left = polled;
+        unsigned long long t0 = 0;
+        for (unsigned tries = 1;; tries++) {
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            if (left >> k & 1) m[k] = mail_get(box + ~ref[k]);
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            if ((left >> k & 1) && mail_is(m[k], seq)) left &= ~(1u << k);
+          if (!left) break;
+          if ((tries & 63u) == 0) {
+            const unsigned long long t = res_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > kResWaitNs) {
+              fail = true;
+              break;
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (ref[k] >= 0)
+          w[k] = S.uv[ref[k]];
+        else if (sub > 0 && (polled >> k & 1))
+          w[k] = mail_value(m[k]);
+        else
+          w[k] = make_double2(a.u_in[~ref[k]], a.v_in[~ref[k]]);
+      }
+      double out[8];
+      if constexpr (kSmemStress) {
+        stress_lean<kStd>(&S.s[0][c], NT, out, w, &S.geo[0][c], NT, p);
+      } else {
+        Corners cr;
+        cr.ucc = w[0].x;
+        cr.vcc = w[0].y;
+        cr.uee = w[1].x;
+        cr.vee = w[1].y;
+        cr.une = w[2].x;
+        cr.vne = w[2].y;
+        cr.use = w[3].x;
+        cr.vse = w[3].y;
+        Geom g;
+        g.dxT = S.geo[0][c];
+        g.dyT = S.geo[1][c];
+        g.cxp = S.geo[2][c];
+        g.cyp = S.geo[3][c];
+        g.cxm = S.geo[4][c];
+        g.cym = S.geo[5][c];
+        g.DminTarea = S.geo[6][c];
+        g.dxhy = S.geo[7][c];
+        g.dyhx = S.geo[8][c];
+        const Strain sr = strain_rates(cr, g, p.e_factor);
+        if (kStd)
+          stress_update_std(sreg, out, sr, S.geo[9][c], g, p);
+        else
+          stress_update(sreg, out, sr, S.geo[9][c], g, p);
+      }
+      S.str[0][c] = make_double2(out[1], out[6]);
+      S.str[1][c] = make_double2(out[2], out[5]);
+      S.str[2][c] = make_double2(out[3], out[7]);
+      own_str = make_double2(out[0], out[4]);
+      if (wlast && own) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) a.str_out[k][slot] = out[k];
+      }
+    }
+    if (fail) atomicMax(a.err, kResCode);
+    if (__syncthreads_or(fail)) return;
+    // ---- stepu -------------------------------------------------------------
+    if (own) {
+      double2 z = S.uv[c];
+      if (actU) {
+        StepuIn in;
+        in.uold = z.x;
+        in.vold = z.y;
+        in.kvrel = S.cst[0][c];
+        in.uocn = S.cst[1][c];
+        in.vocn = S.cst[2][c];
+        in.waterx = S.cst[3][c];
+        in.watery = S.cst[4][c];
+        in.forcex = S.cst[5][c];
+        in.forcey = S.cst[6][c];
+        in.umassdti = S.cst[7][c];
+        in.fm = S.cst[8][c];
+        in.uarear = S.cst[9][c];
+        in.Tbu = S.cst[10][c];
+        in.uinit = S.cst[11][c];
+        in.vinit = S.cst[12][c];
+        const double2 nw = S.str[0][nbr & 1023], sse = S.str[1][(nbr >> 20) & 1023];
+        const double2 sw = S.str[2][(nbr >> 10) & 1023];
+        in.s1 = own_str.x;
+        in.s5 = own_str.y;
+        in.s2nw = nw.x;
+        in.s7nw = nw.y;
+        in.s3sse = sse.x;
+        in.s6sse = sse.y;
+        in.s4sw = sw.x;
+        in.s8sw = sw.y;
+        const StepuOut o = stepu_point(in, p);
+        z = make_double2(o.u, o.v);
+        S.uv[c] = z;
+        if (wlast) {
+          a.strintx[slot] = o.strintx;
+          a.strinty[slot] = o.strinty;
+          a.Cb[slot] = o.Cb;
+        }
+      }
+      if (sub + 1 < a.nsub) {
+        if (exported)
+          mail_put(a.mail + (size_t)((sub + 1) & 1) * (size_t)a.nslots + slot, z.x, z.y,
+                   a.seq + (unsigned)sub + 1u);
+        if (actU && a.uv_step) {
+          a.u_out[(size_t)(sub + 1) * a.uv_step + slot] = z.x;
+          a.v_out[(size_t)(sub + 1) * a.uv_step + slot] = z.y;
+        }
+      } else if (actU) {
+        a.u_out[(size_t)a.nsub * a.uv_step + slot] = z.x;
+        a.v_out[(size_t)a.nsub * a.uv_step + slot] = z.y;
+      }
+    }
+    __syncthreads();
+  }
+  // A block comes here only after its neighbours have read its starting state
+  // (they sent it a later subcycle's velocities), or writes the other set.
+  if (own && actT) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      if constexpr (kSmemStress)
+        a.s_out[k][slot] = S.s[k][c];
+      else
+        a.s_out[k][slot] = sreg[k];
+    }
+  }
+}
+
+using ResKernel = void (*)(ResidentArgs, Params);
+struct ResVariant {
+  int width;
+  ResKernel k[2];  // [kStd]
+  size_t smem;
+};
+template <int NT, bool kSmemStress>
+constexpr ResVariant variant() {
+  return {NT, {k_resident<NT, false, kSmemStress>, k_resident<NT, true, kSmemStress>},
+          sizeof(ResSmem<NT, kSmemStress>)};
+}
+// 640 threads leave 96 registers each: the stresses go to shared memory there.
+// At 512 they stay in registers (4.2 us per subcycle against 5.6 from shared
+// memory, 63.8k points: the extra 48 shared-memory accesses a point cost more
+// than 36 bytes of spills).
+const ResVariant kVariants[] = {variant<128, false>(), variant<256, false>(),
+                                variant<384, false>(), variant<512, false>(),
+                                variant<640, true>()};
+static_assert(sizeof(ResSmem<640, true>) <= 227 * 1024, "shared memory per block");
+
+const ResVariant *find_variant(int cls) {
+  for (const ResVariant &v : kVariants)
+    if (v.width == cls) return &v;
+  return nullptr;
+}
+
+}  // namespace
+
+int resident_prepare(int device, int cls, int nblocks) {
+  const ResVariant *v = find_variant(cls);
+  if (!v) return 0;
+  int coop = 0, sms = 0, per_sm = 0;
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 2 && e == cudaSuccess; k++)
+    e = cudaFuncSetAttribute(v->k[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v->smem);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v->k[1], v->width, v->smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return coop && nblocks <= sms * per_sm ? 1 : 0;
+}
+
+cudaError_t launch_resident(const ResidentArgs &given, const Params &p, int cls, int threads,
+                            int nblocks, cudaStream_t st) {
+  const ResVariant *v = find_variant(cls);
+  if (!v || nblocks <= 0 || given.nsub <= 0) return cudaErrorInvalidValue;
+  ResidentArgs a = given;
+  Params pp = p;
+  void *args[] = {&a, &pp};
+  return cudaLaunchCooperativeKernel((const void *)v->k[std_params(p) ? 1 : 0], dim3(nblocks),
+                                     dim3(threads), args, v->smem, st);
+}
+
+}  // namespace evp

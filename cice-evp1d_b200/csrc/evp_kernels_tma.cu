@@ -873,6 +873,7 @@ const char *tma_wait_name(int code) {
     case 10: return "the stepu-part warp waited for its last copy";
     case 11: return "a consumer waited for a tile's stepu inputs";
     case 13: return "the producer waited for neighbouring tiles to finish a subcycle";
+    case 15: return "a resident block waited for another block's velocities";
     case kProbeCode: return "the wait probe (evp1d_debug_wait_timeout)";
     case kDepProbeCode: return "the dependency-wait probe (evp1d_debug_dep_wait_timeout)";
     default: return "unknown";

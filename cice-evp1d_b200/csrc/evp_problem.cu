@@ -52,6 +52,7 @@ int d2h(void *dst, const void *src, size_t bytes, cudaStream_t st) {
 
 void layout(DeviceProblem *d, Carve &c, size_t nhalo_total, size_t nuvx_total,
             size_t ndep_total) {
+  const size_t R = (size_t)d->res_blocks * (size_t)d->res_threads;
   const size_t S = (size_t)d->nslots, U = (size_t)d->nuv, T = (size_t)d->ntiles;
   c.take(&d->err, 1);
   c.take(&d->cflags, 1);
@@ -90,13 +91,20 @@ void layout(DeviceProblem *d, Carve &c, size_t nhalo_total, size_t nuvx_total,
   c.take(&d->strinty, S);
   c.take(&d->Cb, S);
   for (int k = 0; k < 8; k++) c.take(&d->str[k], U);
+  if (d->res_blocks > 0) {
+    c.take(&d->res_slot, R);
+    c.take(&d->res_cnt, (size_t)d->res_blocks);
+    c.take(&d->res_corner, 4 * R);
+    c.take(&d->res_str, R);
+    c.take(&d->res_mail, 2 * S);
+  }
   c.take(&d->stage, (size_t)32 * (size_t)(d->navel > 0 ? d->navel : 1));
 }
 
 }  // namespace
 
 int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
-                   const double *const geo[kNumGeo]) {
+                   const ResidentPlan &res, const double *const geo[kNumGeo]) {
   d->device = device;
   d->na = plan.na;
   d->navel = plan.navel;
@@ -111,6 +119,11 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
   CUDA_TRY(cudaDeviceGetAttribute(&d->nctas, cudaDevAttrMultiProcessorCount, device));
   if (tma_prepare(device) != 0)
     return error(EVP1D_ERR_CUDA, "cannot enable %d bytes of shared memory", 0);
+  if (res.nblocks > 0 && resident_prepare(device, res.cls, res.nblocks)) {
+    d->res_blocks = res.nblocks;
+    d->res_threads = res.threads;
+    d->res_cls = res.cls;
+  }
   Carve sizing;
   layout(d, sizing, plan.halo_idx.size(), plan.uvx_idx.size(), plan.dep_idx.size());
   CUDA_TRY(device_alloc(&d->arena, sizing.off));
@@ -175,6 +188,12 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
     }
   }
   TRY(h2d(d->tile_rec, rec.data(), rec.size() * sizeof(int32_t), st));
+  if (d->res_blocks > 0) {
+    TRY(h2d(d->res_slot, res.slot.data(), res.slot.size() * sizeof(int32_t), st));
+    TRY(h2d(d->res_cnt, res.cnt.data(), res.cnt.size() * sizeof(int32_t), st));
+    TRY(h2d(d->res_corner, res.corner.data(), res.corner.size() * sizeof(int32_t), st));
+    TRY(h2d(d->res_str, res.str.data(), res.str.size() * sizeof(uint32_t), st));
+  }
   // geometry: reference order -> staging -> slots
   PermBatch b;
   for (int k = 0; k < kNumGeo; k++) {
@@ -507,6 +526,48 @@ TmaArgs problem_tma_args(const DeviceProblem &d, int from) {
   a.dep_idx = d.dep_idx;
   a.err = d.err;
   return a;
+}
+
+cudaError_t problem_launch_resident(DeviceProblem *d, const Params &p, int nsub, bool last,
+                                    double *const s_in[12], double *const s_out[12],
+                                    const double *u_in, const double *v_in, double *u_out,
+                                    double *v_out, size_t uv_step) {
+  ResidentArgs a;
+  a.nslots = d->nslots;
+  a.slot = d->res_slot;
+  a.cnt = d->res_cnt;
+  a.corner = d->res_corner;
+  a.str_idx = d->res_str;
+  a.flags = d->flags;
+  const int geo_order[6] = {kDxT, kDyT, kHTE, kHTN, kHTEm1, kHTNm1};
+  for (int k = 0; k < 6; k++) a.sg[k] = d->geo[geo_order[k]];
+  a.sg[6] = d->dyn[kStrength];
+  const double *uf[kTmaStepuFields] = {
+      d->dyn[kKvrel],  d->dyn[kUocn],     d->dyn[kVocn], d->dyn[kWaterx],
+      d->dyn[kWatery], d->dyn[kForcex],   d->dyn[kForcey], d->dyn[kUmassdti],
+      d->dyn[kFm],     d->geo[kUarear],   d->dyn[kTbu],  d->dyn[kUinit],
+      d->dyn[kVinit]};
+  for (int k = 0; k < kTmaStepuFields; k++) a.uf[k] = uf[k];
+  for (int k = 0; k < 12; k++) {
+    a.s_in[k] = s_in[k];
+    a.s_out[k] = s_out[k];
+  }
+  a.u_in = u_in;
+  a.v_in = v_in;
+  a.u_out = u_out;
+  a.v_out = v_out;
+  a.uv_step = uv_step;
+  a.strintx = d->strintx;
+  a.strinty = d->strinty;
+  a.Cb = d->Cb;
+  for (int k = 0; k < 8; k++) a.str_out[k] = d->str[k];
+  a.nsub = nsub;
+  a.last = last;
+  a.mail = d->res_mail;
+  a.seq = d->res_seq;
+  a.err = d->err;
+  d->res_seq += (unsigned)nsub;
+  return launch_resident(a, p, d->res_cls, d->res_threads, d->res_blocks, d->stream);
 }
 
 int problem_take_error(DeviceProblem *d, int *code) {

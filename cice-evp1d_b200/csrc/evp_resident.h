@@ -1,0 +1,58 @@
+// evp_resident.h -- host-side plan of the resident solver (internal).
+//
+// Where a problem is small enough for one point per thread, a call's
+// subcycles run in one launch whose CTAs keep their points on chip from the
+// first subcycle to the last (evp_kernels_resident.cu).  The list is cut into
+// blocks, one per CTA.  A block owns its points and recomputes `stress` at
+// its forward halo, the nw/sw/sse neighbours other blocks own, so that only
+// velocities travel between blocks: those of points that another block's
+// stress reads ("exported" points).
+#pragma once
+
+#include <cstdint>
+#include <string>
+#include <vector>
+
+#include "evp_tiles.h"
+
+namespace evp {
+
+// Launch widths the kernel is compiled for; a block's compute set (owned
+// points, then forward halo) has at most that many points, one thread each.
+constexpr int kResWidths[] = {128, 256, 384, 512, 640};
+constexpr int kResMaxWidth = 640;
+constexpr int kResMinWidth = 128;  // four warps, one per scheduler
+// ResidentPlan::str bits
+constexpr uint32_t kResExport = 1u << 30;
+
+struct ResidentPlan {
+  int nblocks = 0;
+  int threads = 0;  // per block: compute positions, a multiple of 32
+  int cls = 0;      // the kResWidths entry the kernel runs at
+  std::vector<int32_t> cnt;   // [nblocks] owned points; positions below cnt are owned
+  // [nblocks * threads]: device slot of each position, -1 for none
+  std::vector<int32_t> slot;
+  // [nblocks * threads * 4]: where a position's stress reads the velocities of
+  // cc, ee, ne, se: >= 0 an owned position of the block; < 0 the u/v slot ~x:
+  // another block's point (~x < nslots), or one of the reference's halo slots,
+  // whose velocities stay as given
+  std::vector<int32_t> corner;
+  // [nblocks * threads] owned positions: str positions of nw, sw, sse (10 bits
+  // each; `cls` = the zero slot) and kResExport
+  std::vector<uint32_t> str;
+};
+
+// Plan for at most `max_blocks` CTAs from the problem's tile plan (its slots
+// and rebuilt coordinates) and 0-based neighbour vectors.  False where the
+// problem does not fit one point per thread, has no grid layout, or where a
+// block would read from a block that does not read from it (the kernel's
+// two-deep mailboxes need the symmetry; grids have it).
+bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &tiles,
+                         int max_blocks, ResidentPlan *plan);
+
+// Decode every index of `plan` and compare it with the neighbour vectors.
+// Returns the number of violations; *first (if not null) describes the first.
+long long verify_resident_plan(const ResidentPlan &plan, int na, const int32_t *const nb0[6],
+                               const TilePlan &tiles, std::string *first);
+
+}  // namespace evp

@@ -308,6 +308,11 @@ void build_tile_plan(int na, int navel, const int32_t *const nb0[6],
     if ((int)T.run_off.size() - 1 <= want_runs) break;
   }
   std::vector<std::vector<int32_t>> &tiles = T.tiles;
+  if (have) {
+    P.ci = std::move(ci);
+    P.cj = std::move(cj);
+    P.piece = std::move(comp);
+  }
   P.nruns = (int)T.run_off.size() - 1;
   P.run_off = T.run_off;
 

@@ -66,6 +66,9 @@ struct TilePlan {
   int nslots = 0;        // owned slots incl. alignment padding
   int nhalo_slots = 0;   // navel - na: the reference's halo slots, appended
   bool from_coords = false;  // points ordered by reconstructed (i,j); else list order
+  // with from_coords, per list point: its piece (connected part of the list)
+  // and its coordinates from the piece's corner
+  std::vector<int32_t> ci, cj, piece;
   std::vector<int32_t> slot_of_point;  // [na]
   std::vector<int32_t> point_of_slot;  // [nslots], -1 for padding
   std::vector<int32_t> run_off;        // [nruns + 1] tile ranges of the runs

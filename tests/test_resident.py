@@ -1,0 +1,119 @@
+"""The resident solver: a call's subcycles in one launch, one point per thread.
+
+CPU: the resident plan's indices against the neighbour vectors, over grids at
+the edges of the kernel's width classes, and mistakes planted in a plan.
+GPU: the launch against the oracle, bit for bit (zero tolerance: the same
+operations in the same order), at sizes around the class edges, over counts
+around the smallest it takes, and against the one-launch-per-subcycle form.
+"""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import evp1d
+from evp1d import synth
+
+from conftest import PKG, ROOT
+
+NEIGHBOURS = ("ee", "ne", "se", "nw", "sw", "sse")
+BLOCKS = 148
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("resident") / "resident_plan_shim.so")
+    csrc = os.path.join(PKG, "csrc")
+    subprocess.run(["g++", "-O2", "-fPIC", "-shared", "-std=c++17", "-I", csrc,
+                    os.path.join(csrc, "evp_tiles.cpp"), os.path.join(csrc, "evp_resident.cpp"),
+                    os.path.join(ROOT, "tests", "native", "resident_plan_shim.cpp"), "-o", out],
+                   check=True)
+    L = C.CDLL(out)
+    L.resident_plan.restype = C.c_longlong
+    return L
+
+
+def plan(L, pr, blocks=BLOCKS, plant=0):
+    nb = np.ascontiguousarray(np.stack([pr.idx[k] - 1 for k in NEIGHBOURS]).astype(np.int32))
+    st = (C.c_longlong * 6)()
+    bad = L.resident_plan(pr.na, pr.navel, nb.ctypes.data_as(C.POINTER(C.c_int32)), blocks, plant, st)
+    return bad, list(st)
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 2), (64, 48), (131, 77), (203, 151), (45, 550), (300, 200),
+                                   (330, 250), (400, 300), (416, 312)])
+def test_plan_indices(shim, nx, ny):
+    pr = synth.to_1d(synth.make_grid(nx, ny, seed=3, ndte=2))
+    bad, (nb, threads, cls, most, halo, exported) = plan(shim, pr)
+    assert bad == 0
+    assert nb <= BLOCKS and most <= threads <= cls
+    assert pr.na + halo <= nb * threads
+
+
+def test_plan_refuses_what_does_not_fit(shim):
+    # more points than one per thread, and a graph without a grid layout
+    assert plan(shim, synth.to_1d(synth.make_grid(700, 500, seed=3, ndte=2)))[0] == -1
+    rng = np.random.default_rng(2)
+    pr = synth.to_1d(synth.make_grid(40, 30, seed=3, ndte=2))
+    for k in NEIGHBOURS:
+        pr.idx[k] = rng.integers(1, pr.navel + 1, pr.na).astype(np.int32)
+    assert plan(shim, pr)[0] == -1
+
+
+@pytest.mark.parametrize("plant", [1, 2, 3, 4, 5])
+def test_plan_verifier_catches(shim, plant):
+    pr = synth.to_1d(synth.make_grid(131, 77, seed=3, ndte=2))
+    assert plan(shim, pr, plant=plant)[0] > 0
+
+
+def _params(ndte, general):
+    p = evp1d.set_evp_parameters(ndte)
+    if general:
+        p.revp, p.Ktens, p.capping = 1.0, 0.2, 0.0
+        p.cosw, p.sinw = np.cos(0.4), np.sin(0.4)
+    return p
+
+
+# widths 128, 256, 384, 512, 640 of the kernel
+@pytest.mark.gpu
+@pytest.mark.parametrize("general", [False, True])
+@pytest.mark.parametrize("nx,ny,ndte", [(3, 2, 5), (64, 48, 24), (200, 150, 5), (300, 200, 5),
+                                        (330, 250, 4), (400, 300, 4)])
+def test_launch_bitwise(oracle_mod, nx, ny, ndte, general):
+    from test_gpu_parity import assert_same, gpu_run, oracle_run
+    g = synth.make_grid(nx, ny, seed=13, ndte=ndte, curvilinear=True)
+    if general:
+        rng = np.random.default_rng(5)
+        g.f["Tbu"] = np.asfortranarray(rng.uniform(0.0, 5.0, g.f["Tbu"].shape))
+    pr = synth.to_1d(g)
+    p = _params(ndte, general)
+    fs = gpu_run(pr, ndte, params=p, explicit_init=general)
+    assert_same(fs, oracle_run(oracle_mod, pr, ndte, params=p), pr)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 101])
+def test_same_as_one_launch_per_subcycle(monkeypatch, n):
+    """The same bits as the subcycle kernel in every output, over three calls
+    on one handle (mailbox numbers go on, both buffer sets are used), and the
+    call that does not end (evp1d_subcycles_inner) between them."""
+    pr = synth.to_1d(synth.make_grid(203, 151, seed=5, ndte=n, curvilinear=True))
+    got = []
+    for resident in ("1", "0"):
+        monkeypatch.setenv("EVP1D_RESIDENT", resident)
+        fs = evp1d.FieldSet.from_problem(pr, want_str=True)
+        with evp1d.EVP1D.from_problem(pr, ndte=n) as s:
+            s.upload(fs)
+            s.launch_count(reset=True)
+            s.subcycles(n)
+            launches = s.launch_count()
+            s.subcycles_inner(n)
+            s.subcycles(n)
+            s.download(fs)
+        assert launches == (1 if resident == "1" else n)
+        got.append(fs)
+    for k in ("stress", "uvel", "vvel", "strintx", "strinty", "Cb", "str"):
+        a, b = (np.asarray(getattr(f, k)).view(np.int64) for f in got)
+        assert np.array_equal(a, b), k

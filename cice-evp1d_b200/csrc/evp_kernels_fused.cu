@@ -61,11 +61,10 @@ k_fused(FusedArgs a, Params p) {
         cr.vse = a.v_in[ise];
         const Geom gm = make_geom(a.dxT[g], a.dyT[g], a.HTE[g], a.HTN[g],
                                   a.HTEm1[g], a.HTNm1[g], p.deltaminEVP);
-        const Strain sr = strain_rates(cr, gm, p.e_factor);
         double st[12];
 #pragma unroll
         for (int k = 0; k < 12; k++) st[k] = a.s_in[k][g];
-        stress_update(st, out, sr, a.strength[g], gm, p);
+        stress_point<false>(cr, gm, a.strength[g], st, out, p);
         if (owned) {
 #pragma unroll
           for (int k = 0; k < 12; k++) a.s_out[k][g] = st[k];

@@ -34,14 +34,10 @@ k_stress_ref(DevState s, Params p) {
     c.vse = s.v[ise];
     const Geom g = make_geom(s.dxT[w], s.dyT[w], s.HTE[w], s.HTN[w],
                              s.HTEm1[w], s.HTNm1[w], p.deltaminEVP);
-    const Strain sr = strain_rates(c, g, p.e_factor);
     double st[12], out[8];
 #pragma unroll
     for (int k = 0; k < 12; k++) st[k] = s.stress[k][w];
-    if (kStd)
-      stress_update_std(st, out, sr, s.strength[w], g, p);
-    else
-      stress_update(st, out, sr, s.strength[w], g, p);
+    stress_point<kStd>(c, g, s.strength[w], st, out, p);
 #pragma unroll
     for (int k = 0; k < 12; k++) s.stress[k][w] = st[k];
 #pragma unroll

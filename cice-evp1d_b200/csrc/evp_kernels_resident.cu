@@ -109,19 +109,16 @@ __device__ __forceinline__ unsigned long long res_ns() {
 // stress below is written so that few values are live at once.
 __device__ __forceinline__ void hold() { asm volatile("" ::: "memory"); }
 
-// stress_update (evp_math.cuh) on a point's 12 stresses in shared memory
-// (`s`, `stride` doubles apart), for the widths that leave a thread 96
-// registers: corner by corner, then the x and the y half of str_combine with
-// the stresses read again.  Every operation is stress_update's own, in its
-// order (corner_strain and corner_update; the sums of str_combine), so the
-// bits are the same.
+// stress_point (evp_math.cuh) on a point's 12 stresses in shared memory (`s`,
+// `stride` doubles apart), for the width that leaves a thread 96 registers:
+// the relaxations corner by corner, then the x and the y half of str_combine
+// with the stresses read again.  Every operation is stress_point's own, in its
+// order, so the bits are the same.
 template <bool kStd>
 __device__ __forceinline__ void stress_lean(double *s, int stride, double (&out)[8],
-                                            const double2 (&w)[4], const double *geo, int gs,
+                                            const Corners &c, const double *geo, int gs,
                                             const Params &p) {
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int p2 = k ^ 1, p4 = 3 - k;
+  {
     Geom g;
     g.dxT = geo[0 * gs];
     g.dyT = geo[1 * gs];
@@ -129,25 +126,34 @@ __device__ __forceinline__ void stress_lean(double *s, int stride, double (&out)
     g.cyp = geo[3 * gs];
     g.cxm = geo[4 * gs];
     g.cym = geo[5 * gs];
-    double div, ten, shr, Delta;
-    corner_strain(k, w[k].x, w[k].y, w[p2].x, w[p2].y, w[p4].x, w[p4].y, g, p.e_factor, div, ten,
-                  shr, Delta);
-    const double strength = geo[9 * gs], least = geo[6 * gs];
-    double sp = s[k * stride], sm = s[(4 + k) * stride], st = s[(8 + k) * stride];
-    if (kStd && least > 0.0 && fabs(strength) < 1e300 * least && Delta == Delta) {
-      const double z = strength / fmax_ref(Delta, least);
-      const double r = z * Delta;
-      const double e = p.epp2i * z;
-      sp = (sp + p.arlx1i * (z * div - r)) * p.denom1;
-      sm = (sm + p.arlx1i * e * ten) * p.denom1;
-      st = (st + p.arlx1i * kP5 * e * shr) * p.denom1;
-    } else {
-      corner_update(sp, sm, st, div, ten, shr, Delta, strength, least, p);
-    }
-    s[k * stride] = sp;
-    s[(4 + k) * stride] = sm;
-    s[(8 + k) * stride] = st;
+    const StrainSq q = strain_squares(c, g, p.e_factor);
     hold();
+    const double strength = geo[9 * gs], least = geo[6 * gs];
+    if (stress_in_range(strength, least, q.sq) &&
+        (kStd || p.capping == kC1 || p.capping == 0.0)) {
+      double Delta[4], visc[4];
+      viscosities(strength, least, kStd || p.capping == kC1, q.sq, Delta, visc);
+      hold();
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        double sp = s[k * stride], sm = s[(4 + k) * stride], st = s[(8 + k) * stride];
+        corner_relax<kStd>(sp, sm, st, q.div[k], q.ten[k], q.shr[k], Delta[k], visc[k], p);
+        s[k * stride] = sp;
+        s[(4 + k) * stride] = sm;
+        s[(8 + k) * stride] = st;
+        hold();
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        double sp = s[k * stride], sm = s[(4 + k) * stride], st = s[(8 + k) * stride];
+        corner_update(sp, sm, st, q.div[k], q.ten[k], q.shr[k], sqrt(q.sq[k]), strength, least, p);
+        s[k * stride] = sp;
+        s[(4 + k) * stride] = sm;
+        s[(8 + k) * stride] = st;
+        hold();
+      }
+    }
   }
 #pragma unroll
   for (int half = 0; half < 2; half++) {
@@ -318,19 +324,19 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResidentArgs a, Params p) {
         else
           w[k] = make_double2(a.u_in[~ref[k]], a.v_in[~ref[k]]);
       }
+      Corners cr;
+      cr.ucc = w[0].x;
+      cr.vcc = w[0].y;
+      cr.uee = w[1].x;
+      cr.vee = w[1].y;
+      cr.une = w[2].x;
+      cr.vne = w[2].y;
+      cr.use = w[3].x;
+      cr.vse = w[3].y;
       double out[8];
       if constexpr (kSmemStress) {
-        stress_lean<kStd>(&S.s[0][c], NT, out, w, &S.geo[0][c], NT, p);
+        stress_lean<kStd>(&S.s[0][c], NT, out, cr, &S.geo[0][c], NT, p);
       } else {
-        Corners cr;
-        cr.ucc = w[0].x;
-        cr.vcc = w[0].y;
-        cr.uee = w[1].x;
-        cr.vee = w[1].y;
-        cr.une = w[2].x;
-        cr.vne = w[2].y;
-        cr.use = w[3].x;
-        cr.vse = w[3].y;
         Geom g;
         g.dxT = S.geo[0][c];
         g.dyT = S.geo[1][c];
@@ -341,11 +347,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResidentArgs a, Params p) {
         g.DminTarea = S.geo[6][c];
         g.dxhy = S.geo[7][c];
         g.dyhx = S.geo[8][c];
-        const Strain sr = strain_rates(cr, g, p.e_factor);
-        if (kStd)
-          stress_update_std(sreg, out, sr, S.geo[9][c], g, p);
-        else
-          stress_update(sreg, out, sr, S.geo[9][c], g, p);
+        stress_point<kStd>(cr, g, S.geo[9][c], sreg, out, p);
       }
       S.str[0][c] = make_double2(out[1], out[6]);
       S.str[1][c] = make_double2(out[2], out[5]);

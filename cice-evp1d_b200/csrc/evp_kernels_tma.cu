@@ -706,14 +706,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
           cr.vse = st.v[ise];
           const Geom gm = make_geom(F[0 * fs], F[1 * fs], F[2 * fs], F[3 * fs], F[4 * fs],
                                     F[5 * fs], p.deltaminEVP);
-          const Strain sr = strain_rates(cr, gm, p.e_factor);
           double s12[12];
 #pragma unroll
           for (int k = 0; k < 12; k++) s12[k] = F12[k * fs];
-          if (kStd)
-            stress_update_std(s12, out, sr, F[6 * fs], gm, p);
-          else
-            stress_update(s12, out, sr, F[6 * fs], gm, p);
+          stress_point<kStd>(cr, gm, F[6 * fs], s12, out, p);
           if (own) {
 #pragma unroll
             for (int k = 0; k < 12; k++) a.s[to][k][cy.off + c] = s12[k];

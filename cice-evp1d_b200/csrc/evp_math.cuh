@@ -4,15 +4,17 @@
 // operation order (left to right within a precedence level, parentheses kept,
 // x**2 as x*x, sign(1,x) as copysign).  The translation unit is compiled with
 // -fmad=false, so every +, -, * is a separately rounded IEEE FP64 operation
-// and / and sqrt are the IEEE correctly rounded CUDA FP64 operations: the
-// results are bit-identical to the reference's -fp-model precise -no-fma
-// builds.  Build flag EVP_FMA (set only in the FMA flavour of the library)
+// and / and sqrt are correctly rounded (CUDA's FP64 operations, or
+// evp_fp64.cuh's): the results are bit-identical to the reference's
+// -fp-model precise -no-fma builds.  Build flag EVP_FMA (set only in the FMA flavour of the library)
 // changes nothing here; the compiler then contracts a*b+c itself.
 #pragma once
 
 #include <cmath>
 
 #include <cuda_runtime.h>
+
+#include "evp_fp64.cuh"
 
 namespace evp {
 
@@ -68,15 +70,15 @@ __host__ __device__ __forceinline__ double fmax_ref(double a, double b) {
   return a > b ? a : b;
 }
 
-// strain_rates (src/bench_v2b.F90:321-397) and Delta.
-struct Strain {
-  double div[4], ten[4], shr[4], Delta[4];  // corners ne, nw, sw, se
+// strain_rates (src/bench_v2b.F90:321-397) and the square of Delta.
+struct StrainSq {
+  double div[4], ten[4], shr[4], sq[4];  // corners ne, nw, sw, se
 };
 
-__host__ __device__ __forceinline__ Strain strain_rates(const Corners &c,
-                                                        const Geom &g,
-                                                        double e_factor) {
-  Strain s;
+__host__ __device__ __forceinline__ StrainSq strain_squares(const Corners &c,
+                                                            const Geom &g,
+                                                            double e_factor) {
+  StrainSq s;
   const double ucc = c.ucc, vcc = c.vcc, uee = c.uee, vee = c.vee;
   const double une = c.une, vne = c.vne, use = c.use, vse = c.vse;
   const double dxT = g.dxT, dyT = g.dyT, cxp = g.cxp, cyp = g.cyp;
@@ -97,9 +99,32 @@ __host__ __device__ __forceinline__ Strain strain_rates(const Corners &c,
   s.shr[3] = -(cym * vse) - dyT * vne - cxp * use + dxT * ucc;
 #pragma unroll
   for (int k = 0; k < 4; k++)
-    s.Delta[k] = sqrt(s.div[k] * s.div[k] +
-                      e_factor * (s.ten[k] * s.ten[k] + s.shr[k] * s.shr[k]));
+    s.sq[k] = s.div[k] * s.div[k] +
+              e_factor * (s.ten[k] * s.ten[k] + s.shr[k] * s.shr[k]);
   return s;
+}
+
+// strain_rates and Delta.
+struct Strain {
+  double div[4], ten[4], shr[4], Delta[4];  // corners ne, nw, sw, se
+};
+
+__host__ __device__ __forceinline__ Strain strain_delta(const StrainSq &q) {
+  Strain s;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    s.div[k] = q.div[k];
+    s.ten[k] = q.ten[k];
+    s.shr[k] = q.shr[k];
+    s.Delta[k] = sqrt(q.sq[k]);
+  }
+  return s;
+}
+
+__host__ __device__ __forceinline__ Strain strain_rates(const Corners &c,
+                                                        const Geom &g,
+                                                        double e_factor) {
+  return strain_delta(strain_squares(c, g, e_factor));
 }
 
 // visc_replpress (src/bench_v2b.F90:415-437).
@@ -235,6 +260,81 @@ __host__ __device__ __forceinline__ void stress_update_std(
   str_combine(s, out, g);
 }
 
+// Whether the straight-line stress below holds at a point: strength, DminArea
+// and the four squared Deltas in the ranges of evp_fp64.cuh.
+__host__ __device__ __forceinline__ bool stress_in_range(double strength, double DminArea,
+                                                         const double (&sq)[4]) {
+  return fp64_dividend(strength) & fp64_mid(DminArea) & fp64_radicand(sq[0]) &
+         fp64_radicand(sq[1]) & fp64_radicand(sq[2]) & fp64_radicand(sq[3]);
+}
+
+// The viscosity strength/max(Delta, DminArea), or without capping
+// strength/(Delta + DminArea), of the four corners, and their Deltas
+// (stress_in_range): the square roots and divisions side by side.  The other
+// viscosity's share, 0 times a finite quotient of the same sign, leaves the
+// sum at the first (capping is 1 or 0).
+__host__ __device__ __forceinline__ void viscosities(double strength, double DminArea,
+                                                     bool capped, const double (&sq)[4],
+                                                     double (&Delta)[4], double (&visc)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) Delta[k] = fp64_sqrt(sq[k]);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const double den = capped ? fmax_ref(Delta[k], DminArea) : Delta[k] + DminArea;
+    visc[k] = fp64_quot(strength, den, fp64_recip(den));
+  }
+}
+
+// One corner's relaxation from its viscosity (corner_update's expressions;
+// kStd: Ktens == 0 and revp == 0, whose factors are exactly 1).
+template <bool kStd>
+__host__ __device__ __forceinline__ void corner_relax(double &sp, double &sm, double &s12,
+                                                      double div, double ten, double shr,
+                                                      double Delta, double visc,
+                                                      const Params &p) {
+  const double arlx1i = p.arlx1i, denom1 = p.denom1;
+  const double z = kStd ? visc : (kC1 + p.Ktens) * visc;
+  const double r = kStd ? visc * Delta : (kC1 - p.Ktens) * visc * Delta;
+  const double e = p.epp2i * z;
+  if (kStd) {
+    sp = (sp + arlx1i * (z * div - r)) * denom1;
+    sm = (sm + arlx1i * e * ten) * denom1;
+    s12 = (s12 + arlx1i * kP5 * e * shr) * denom1;
+  } else {
+    const double keep = kC1 - arlx1i * p.revp;
+    sp = (sp * keep + arlx1i * (z * div - r)) * denom1;
+    sm = (sm * keep + arlx1i * e * ten) * denom1;
+    s12 = (s12 * keep + arlx1i * kP5 * e * shr) * denom1;
+  }
+}
+
+// `stress` at one T point (src/bench_v2b.F90:137-310): strain rates, the 12
+// relaxations in place, str1..str8.  The bits of strain_rates followed by
+// stress_update (kStd: stress_update_std), which run where the point's values
+// are out of range (never in normal runs) or capping is neither 0 nor 1.
+template <bool kStd>
+__host__ __device__ __forceinline__ void stress_point(const Corners &c, const Geom &g,
+                                                      double strength, double (&s)[12],
+                                                      double (&out)[8], const Params &p) {
+  const StrainSq q = strain_squares(c, g, p.e_factor);
+  if (!stress_in_range(strength, g.DminTarea, q.sq) ||
+      (!kStd && p.capping != kC1 && p.capping != 0.0)) {
+    const Strain sr = strain_delta(q);
+    if (kStd)
+      stress_update_std(s, out, sr, strength, g, p);
+    else
+      stress_update(s, out, sr, strength, g, p);
+    return;
+  }
+  double Delta[4], visc[4];
+  viscosities(strength, g.DminTarea, kStd || p.capping == kC1, q.sq, Delta, visc);
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    corner_relax<kStd>(s[k], s[4 + k], s[8 + k], q.div[k], q.ten[k], q.shr[k], Delta[k], visc[k],
+                       p);
+  str_combine(s, out, g);
+}
+
 __host__ __device__ __forceinline__ void str_combine(const double (&s)[12],
                                                      double (&out)[8],
                                                      const Geom &g) {
@@ -342,17 +442,30 @@ struct StepuOut {
 //    fm unless fm is -0 and the zero is +0, i.e. unless fm == -0 and
 //    vrel < 0; a NaN vrel takes the literal route; an infinite vrel makes u
 //    and v NaN on both routes, and strintx, strinty and Cb do not use ccb.
+// The square roots and divisions are evp_fp64.cuh's where their operands are
+// in range, CUDA's elsewhere: the same bits.
 __host__ __device__ __forceinline__ StepuOut stepu_point(const StepuIn &in,
                                                          const Params &p) {
   StepuOut o;
   const double uold = in.uold, vold = in.vold;
   const double du = in.uocn - uold, dv = in.vocn - vold;
-  const double vrel = in.kvrel * sqrt(du * du + dv * dv);
+  const double d2 = du * du + dv * dv;
+  double speed = fp64_sqrt(d2);
+  if (!fp64_radicand(d2)) speed = sqrt(d2);
+  const double vrel = in.kvrel * speed;
   const double taux = vrel * in.waterx;
   const double tauy = vrel * in.watery;
   const bool tbu_zero = in.Tbu == 0.0 && copysign(kC1, in.Tbu) > 0.0 && p.u0 > 0.0 &&
                         uold == uold && vold == vold;
-  o.Cb = tbu_zero ? 0.0 : in.Tbu / (sqrt(uold * uold + vold * vold) + p.u0);
+  o.Cb = 0.0;
+  if (!tbu_zero) {
+    const double w2 = uold * uold + vold * vold;
+    const double den = fp64_sqrt(w2) + p.u0;
+    if (fp64_radicand(w2) & fp64_divisor(den) & fp64_mid_abs(in.Tbu))
+      o.Cb = fp64_quot(in.Tbu, den, fp64_recip(den));
+    else
+      o.Cb = in.Tbu / (sqrt(w2) + p.u0);
+  }
   const double cca = (p.brlx + p.revp) * in.umassdti + (p.cosw == kC1 ? vrel : vrel * p.cosw) + o.Cb;
   const double ccb = p.sinw == 0.0 && (in.fm != 0.0 || vrel >= 0.0)
                          ? in.fm
@@ -364,8 +477,14 @@ __host__ __device__ __forceinline__ StepuOut stepu_point(const StepuIn &in,
                      in.umassdti * (p.brlx * uold + p.revp * in.uinit);
   const double cc2 = o.strinty + in.forcey + tauy +
                      in.umassdti * (p.brlx * vold + p.revp * in.vinit);
-  o.u = (cca * cc1 + ccb * cc2) / ab2;
-  o.v = (cca * cc2 - ccb * cc1) / ab2;
+  const double nu = cca * cc1 + ccb * cc2, nv = cca * cc2 - ccb * cc1;
+  const Recip r = fp64_recip(ab2);
+  o.u = fp64_quot(nu, ab2, r);
+  o.v = fp64_quot(nv, ab2, r);
+  if (!(fp64_divisor(ab2) & fp64_mid_abs(nu) & fp64_mid_abs(nv))) {
+    o.u = nu / ab2;
+    o.v = nv / ab2;
+  }
   return o;
 }
 

@@ -77,11 +77,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_na_stress(NaArgs a, Params p) {
     c.vse = a.v[ise];
     const Geom g = make_geom(a.dxT[w], a.dyT[w], a.HTE[w], a.HTN[w], a.HTEm1[w],
                              a.HTNm1[w], p.deltaminEVP);
-    const Strain sr = strain_rates(c, g, p.e_factor);
     double st[12], out[8];
 #pragma unroll
     for (int k = 0; k < 12; k++) st[k] = a.stress[k][w];
-    stress_update(st, out, sr, a.strength[w], g, p);
+    stress_point<false>(c, g, a.strength[w], st, out, p);
 #pragma unroll
     for (int k = 0; k < 12; k++) a.stress[k][w] = st[k];
 #pragma unroll

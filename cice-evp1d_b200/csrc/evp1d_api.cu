@@ -34,6 +34,12 @@ int error(int code, const char *fmt, ...) {
   return code;
 }
 
+int timeout_error(int code) {
+  return error(EVP1D_ERR_TIMEOUT,
+               "a bounded device-side wait ran out (code %d: %s); the results of this "
+               "call are not valid", code, tma_wait_name(code));
+}
+
 cudaError_t device_alloc(void **p, size_t bytes) {
   int n = g_fail_alloc.load();
   while (n > 0 && !g_fail_alloc.compare_exchange_weak(n, n - 1)) {
@@ -129,11 +135,7 @@ constexpr int kResidentMin = 2;
 int check_device_error(evp1d_t *h) {
   int code = 0;
   CHECK(evp::problem_take_error(&h->d, &code));
-  if (code)
-    return fail(EVP1D_ERR_TIMEOUT,
-                "a bounded device-side wait ran out (code %d: %s); the results of this "
-                "call are not valid", code, evp::tma_wait_name(code));
-  return EVP1D_OK;
+  return code ? evp::timeout_error(code) : EVP1D_OK;
 }
 
 // Capture kGraphChunk non-final fused subcycles starting from buffer `from`.
@@ -477,6 +479,19 @@ int evp1d_init_batched(evp1d_t **handle, int nmembers, const int32_t *na_m,
   for (int k = 0; k < 6; k++) cidx[k] = comb.data() + (size_t)k * NA;
   CHECK(init_common(handle, (int)NA, (int)NV, cidx, geo, params, device));
   (*handle)->nmembers = nmembers;
+  if (nmembers > 1 && NA > 0) {
+    std::vector<int32_t> pos(uv_pos.begin(), uv_pos.end());
+    int32_t **dst = &(*handle)->d.uv_pos;
+    cudaError_t e = evp::device_alloc(dst, pos.size() * sizeof(int32_t));
+    if (e == cudaSuccess)
+      e = cudaMemcpy(*dst, pos.data(), pos.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+      evp1d_finalize(*handle);
+      *handle = nullptr;
+      return fail(e == cudaErrorMemoryAllocation ? EVP1D_ERR_NOMEM : EVP1D_ERR_CUDA,
+                  "batched velocity positions: %s", cudaGetErrorString(e));
+    }
+  }
   (*handle)->uv_pos = std::move(uv_pos);
   return EVP1D_OK;
 }
@@ -509,25 +524,77 @@ int evp1d_set_params(evp1d_t *h, const evp1d_params *params) {
 }
 
 int evp1d_upload(evp1d_t *h, const evp1d_fields *io) {
-  evp::NvtxRange nvtx_range("evp1d_upload");
-  if (!h || !io) return fail(EVP1D_ERR_INVALID_ARG, "NULL argument");
-  CHECK(select_device(h));
-  evp::adjoint_invalidate(h->adj);
-  h->uinit_explicit = io->uvel_init != nullptr;
-  if (h->nmembers > 1 && h->d.na > 0) {
-    if (!io->uvel || !io->vvel) return fail(EVP1D_ERR_INVALID_ARG, "uvel/vvel are NULL");
-    const evp1d_fields c = combined_view(h, io, true);
-    CHECK(evp::problem_upload(&h->d, &c, h->p.rhow));
-  } else {
-    CHECK(evp::problem_upload(&h->d, io, h->p.rhow));
-  }
-  h->uploaded = true;
-  return EVP1D_OK;
+  return evp::upload_fields(h, io, true);
 }
 
 }  // extern "C"
 
 namespace evp {
+int upload_fields(evp1d_handle *h, const evp1d_fields *io, bool wait) {
+  NvtxRange nvtx_range("evp1d_upload");
+  if (!h || !io) return fail(EVP1D_ERR_INVALID_ARG, "NULL argument");
+  CHECK(select_device(h));
+  adjoint_invalidate(h->adj);
+  h->uinit_explicit = io->uvel_init != nullptr;
+  DeviceProblem &d = h->d;
+  evp1d_fields c = *io;
+  UploadFields f;
+  if (d.na > 0) {
+    const double *in[12] = {io->strength, io->Cw, io->aiu, io->uocn,
+                            io->vocn, io->waterx, io->watery, io->forcex,
+                            io->forcey, io->umassdti, io->fm, io->Tbu};
+    static const char *inname[12] = {"strength", "Cw", "aiu", "uocn",
+                                     "vocn", "waterx", "watery", "forcex",
+                                     "forcey", "umassdti", "fm", "Tbu"};
+    for (int k = 0; k < 12; k++)
+      if (!in[k]) return fail(EVP1D_ERR_INVALID_ARG, "field %s is NULL", inname[k]);
+    for (int k = 0; k < 12; k++)
+      if (!io->stress[k]) return fail(EVP1D_ERR_INVALID_ARG, "stress[%d] is NULL", k);
+    if (!io->skipT || !io->skipU || !io->uvel || !io->vvel || !io->strintx ||
+        !io->strinty || !io->Cb)
+      return fail(EVP1D_ERR_INVALID_ARG,
+                  "skipT/skipU/uvel/vvel/strintx/strinty/Cb must not be NULL");
+    const size_t bv = sizeof(double) * (size_t)d.navel;
+    void *dev;
+    if (h->nmembers > 1) {
+      // members' velocities at their own places, or put in order by the host
+      if (device_view(io->uvel, bv, sizeof(double), &dev) &&
+          device_view(io->vvel, bv, sizeof(double), &dev))
+        f.map_uv = d.uv_pos;
+      else
+        c = combined_view(h, io, true);
+    }
+    for (int k = 0; k < 12; k++) {
+      f.in[k] = in[k];
+      f.stress[k] = io->stress[k];
+    }
+    f.u = c.uvel;
+    f.v = c.vvel;
+    f.uinit = io->uvel_init;
+    f.vinit = io->vvel_init;
+    f.strintx = io->strintx;
+    f.strinty = io->strinty;
+    f.Cb = io->Cb;
+    f.skT = io->skipT;
+    f.skU = io->skipU;
+    f.n_f = (size_t)d.na;
+    f.n_uv = (size_t)d.navel;
+    f.stage = d.stage;
+    f.stage_step = (size_t)d.navel;
+    f.istage = reinterpret_cast<int32_t *>(d.stage + (size_t)31 * d.navel);
+    CHECK(problem_upload(&d, f, h->p.rhow, wait));
+  }
+  h->uploaded = true;
+  return EVP1D_OK;
+}
+
+int settle(evp1d_handle *h, int rc) {
+  // a call that fails while its arrays may still be read ends only when the
+  // stream has
+  if (rc != EVP1D_OK && h && h->d.stream) cudaStreamSynchronize(h->d.stream);
+  return rc;
+}
+
 bool use_resident(const evp1d_handle *h, int n) {
   if (h->path != kPathTma || !h->resident || n < kResidentMin) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -611,22 +678,55 @@ int evp1d_download(evp1d_t *h, const evp1d_fields *io) {
   if (!h || !io) return fail(EVP1D_ERR_INVALID_ARG, "NULL argument");
   if (!h->uploaded) return fail(EVP1D_ERR_STATE, "nothing uploaded");
   CHECK(select_device(h));
-  CHECK(check_device_error(h));
-  if (h->nmembers > 1 && h->d.na > 0) {
-    if (!io->uvel || !io->vvel) return fail(EVP1D_ERR_INVALID_ARG, "uvel/vvel are NULL");
-    const evp1d_fields c = combined_view(h, io, false);
-    CHECK(evp::problem_download(&h->d, &c));
-    scatter_combined(h, io, h->d.na);
-    return EVP1D_OK;
+  DeviceProblem &d = h->d;
+  if (d.na == 0) return check_device_error(h);
+  const bool batched = h->nmembers > 1;
+  if (batched && (!io->uvel || !io->vvel))
+    return fail(EVP1D_ERR_INVALID_ARG, "uvel/vvel are NULL");
+  evp::DownloadFields f;
+  evp1d_fields c = *io;
+  const size_t bv = sizeof(double) * (size_t)d.navel;
+  bool direct = batched;
+  void *dev;
+  if (batched) {
+    direct = evp::device_view(io->uvel, bv, sizeof(double), &dev) &&
+             evp::device_view(io->vvel, bv, sizeof(double), &dev);
+    for (int k = 0; k < 8 && direct; k++)
+      direct = !io->str[k] || evp::device_view(io->str[k], bv, sizeof(double), &dev);
+    if (direct)
+      f.map_uv = d.uv_pos;
+    else
+      c = combined_view(h, io, false);
   }
-  return evp::problem_download(&h->d, io);
+  for (int k = 0; k < 12; k++) f.stress[k] = io->stress[k];
+  f.u = c.uvel;
+  f.v = c.vvel;
+  f.strintx = io->strintx;
+  f.strinty = io->strinty;
+  f.Cb = io->Cb;
+  for (int k = 0; k < 8; k++) f.str[k] = c.str[k];
+  f.n_f = (size_t)d.na;
+  // in reference order the list points come first; a direct batched array is
+  // addressed whole
+  f.n_u = direct ? (size_t)d.navel : (size_t)d.na;
+  f.n_str = (size_t)d.navel;
+  f.stage = d.stage;
+  f.stage_step = (size_t)d.navel;
+  int code = 0;
+  CHECK(evp::problem_download(&d, f, &code));
+  if (code) return evp::timeout_error(code);
+  if (batched && !direct) scatter_combined(h, io, d.na);
+  return EVP1D_OK;
 }
 
 int evp1d_run(evp1d_t *h, int ndte, const evp1d_fields *io) {
   evp::NvtxRange nvtx_range("evp1d_run");
-  CHECK(evp1d_upload(h, io));
-  CHECK(evp1d_subcycles(h, ndte));
-  return evp1d_download(h, io);
+  // the results are written to the caller's arrays after the stream has read
+  // them, so the upload need not be waited for
+  int rc = evp::settle(h, evp::upload_fields(h, io, false));
+  if (rc == EVP1D_OK) rc = evp::settle(h, evp1d_subcycles(h, ndte));
+  if (rc == EVP1D_OK) rc = evp::settle(h, evp1d_download(h, io));
+  return rc;
 }
 
 int evp1d_stress_only(evp1d_t *h, int n) {

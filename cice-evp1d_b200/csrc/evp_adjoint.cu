@@ -723,9 +723,10 @@ int evp1d_record_subcycles(evp1d_t *h, int ndte, int interval) {
 }
 
 int evp1d_run_checkpointed(evp1d_t *h, int ndte, const evp1d_fields *io, int interval) {
-  ADJ_CHECK(evp1d_upload(h, io));
-  ADJ_CHECK(evp1d_record_subcycles(h, ndte, interval));
-  return evp1d_download(h, io);
+  int rc = settle(h, upload_fields(h, io, false));
+  if (rc == EVP1D_OK) rc = settle(h, evp1d_record_subcycles(h, ndte, interval));
+  if (rc == EVP1D_OK) rc = settle(h, evp1d_download(h, io));
+  return rc;
 }
 
 int evp1d_adjoint_seed(evp1d_t *h, const double *lam_uvel, const double *lam_vvel,

@@ -2,13 +2,13 @@
 // dyn_evp1d_init / dyn_evp1d_run / dyn_evp1d_finalize interface on global 2D
 // arrays, on top of the 1D solver.
 //
-// The per-timestep conversions run on the device: the caller's 2D arrays are
-// copied whole to the GPU, a gather kernel builds the 1D list fields and the
-// skip flags (convert_2d_1d_dyn and set_skipMe,
-// integration/ice_dyn_evp1d.F90:521-537, 818-882) straight into the solver's
-// staging area, and after the subcycles a scatter kernel writes the list
-// points' results back into the 2D arrays (convert_1d_2d_dyn, :884-947),
-// which are copied back whole.  Cells outside the list keep the values the
+// The per-timestep conversions are the transfer kernels' index map
+// (evp_transfer.cu): they read the list points' cells of the caller's arrays
+// and the ice masks (convert_2d_1d_dyn and set_skipMe,
+// integration/ice_dyn_evp1d.F90:521-537, 818-882), halo velocities 0
+// (:880-881), and write the results to the list points' cells
+// (convert_1d_2d_dyn, :884-947).  Arrays that the GPU cannot address are copied
+// whole to the device and back.  Cells outside the list keep the values the
 // caller passed.
 #include <cstdint>
 #include <string>
@@ -25,67 +25,6 @@ namespace {
 // umassdti, fmU, Tbu), the 12 stresses, strintxU, strintyU, Cb, uvel, vvel.
 constexpr int kIn2d = 12;
 constexpr int kF2d = kIn2d + 12 + 3 + 2;  // 29
-constexpr int kOut2d = 12 + 3 + 2;        // results: stresses, strint, Cb, u, v
-
-struct Gather2d {
-  const double *f[kF2d];
-  const int32_t *icet, *iceu;
-};
-
-// 2D -> reference-order staging (slots of problem_upload_staged): list points
-// from their cells, halo slots of u and v zero (:880-881), skip flags from the
-// ice masks (set_skipMe).
-__global__ void k_gather_2d(int na, int navel, const int32_t *__restrict__ cell, Gather2d g,
-                            double *stage) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < navel;
-       p += gridDim.x * blockDim.x) {
-    auto slot = [&](int k) { return stage + (size_t)k * navel; };
-    if (p >= na) {
-      slot(24)[p] = 0.0;
-      slot(25)[p] = 0.0;
-      continue;
-    }
-    const int c = cell[p];
-#pragma unroll
-    for (int k = 0; k < kIn2d; k++) slot(k)[p] = g.f[k][c];
-#pragma unroll
-    for (int k = 0; k < 12; k++) slot(12 + k)[p] = g.f[kIn2d + k][c];
-    slot(28)[p] = g.f[24][c];
-    slot(29)[p] = g.f[25][c];
-    slot(30)[p] = g.f[26][c];
-    slot(24)[p] = g.f[27][c];
-    slot(25)[p] = g.f[28][c];
-    int32_t *skT = reinterpret_cast<int32_t *>(slot(31));
-    skT[p] = g.icet[c] ? 0 : 1;
-    skT[navel + p] = g.iceu[c] ? 0 : 1;
-  }
-}
-
-struct Scatter2d {
-  double *f[kOut2d];
-};
-
-// Reference-order results (slots of problem_download_staged) -> their cells.
-__global__ void k_scatter_2d(int na, int navel, const int32_t *__restrict__ cell,
-                             const double *stage, Scatter2d o) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < na; p += gridDim.x * blockDim.x) {
-    const int c = cell[p];
-#pragma unroll
-    for (int k = 0; k < 12; k++) o.f[k][c] = stage[(size_t)k * navel + p];
-    o.f[12][c] = stage[(size_t)14 * navel + p];  // strintx
-    o.f[13][c] = stage[(size_t)15 * navel + p];  // strinty
-    o.f[14][c] = stage[(size_t)16 * navel + p];  // Cb
-    o.f[15][c] = stage[(size_t)12 * navel + p];  // uvel
-    o.f[16][c] = stage[(size_t)13 * navel + p];  // vvel
-  }
-}
-
-int grid_for(long long n) {
-  long long b = (n + 255) / 256;
-  if (b < 1) b = 1;
-  if (b > 148LL * 32) b = 148LL * 32;
-  return (int)b;
-}
 
 #define DYN_TRY(x)                                                         \
   do {                                                                     \
@@ -191,61 +130,38 @@ int evp1d_dyn_run(evp1d_dyn_t *d, int ndte, const evp1d_dyn_fields *io) {
   evp1d_t *h = d->h;
   evp::DeviceProblem &P = h->d;
   DYN_TRY(cudaSetDevice(P.device));
-  cudaStream_t st = P.stream;
-  const size_t cells = (size_t)d->nx * d->ny, bc = sizeof(double) * cells;
-  // whole 2D arrays to the device
-  const double *src[kF2d];
-  for (int k = 0; k < kIn2d; k++) src[k] = in[k];
-  for (int k = 0; k < 12; k++) src[kIn2d + k] = io->stress[k];
-  src[24] = io->strintxU;
-  src[25] = io->strintyU;
-  src[26] = io->Cb;
-  src[27] = io->uvel;
-  src[28] = io->vvel;
-  Gather2d g;
-  for (int k = 0; k < kF2d; k++) {
-    double *dst = d->f2d + (size_t)k * cells;
-    DYN_TRY(cudaMemcpyAsync(dst, src[k], bc, cudaMemcpyHostToDevice, st));
-    g.f[k] = dst;
+  const size_t cells = (size_t)d->nx * d->ny;
+  evp::UploadFields f;
+  evp::DownloadFields o;
+  for (int k = 0; k < 12; k++) {
+    f.in[k] = in[k];
+    f.stress[k] = io->stress[k];
+    o.stress[k] = io->stress[k];
   }
-  DYN_TRY(cudaMemcpyAsync(d->mask2d, io->icetmask, sizeof(int32_t) * cells,
-                          cudaMemcpyHostToDevice, st));
-  DYN_TRY(cudaMemcpyAsync(d->mask2d + cells, io->iceumask, sizeof(int32_t) * cells,
-                          cudaMemcpyHostToDevice, st));
-  g.icet = d->mask2d;
-  g.iceu = d->mask2d + cells;
-  // 2D -> 1D staging on the device, then the solver's own upload
-  k_gather_2d<<<grid_for(d->navel), 256, 0, st>>>(d->na, d->navel, d->cell, g, P.stage);
-  DYN_TRY(cudaGetLastError());
+  f.u = o.u = io->uvel;
+  f.v = o.v = io->vvel;
+  f.strintx = o.strintx = io->strintxU;
+  f.strinty = o.strinty = io->strintyU;
+  f.Cb = o.Cb = io->Cb;
+  f.skT = io->icetmask;
+  f.skU = io->iceumask;
+  f.mask = f.zero_halo = true;
+  f.n_f = f.n_uv = o.n_f = o.n_u = cells;
+  f.map_f = o.map_f = d->cell;
+  f.stage = o.stage = d->f2d;
+  f.stage_step = o.stage_step = cells;
+  f.istage = d->mask2d;
   evp::adjoint_invalidate(h->adj);
   h->uinit_explicit = false;
-  int rc = evp::problem_upload_staged(&P, false, false, h->p.rhow);
+  int rc = evp::settle(h, evp::problem_upload(&P, f, h->p.rhow, false));
   if (rc != EVP1D_OK) return rc;
   h->uploaded = true;
-  rc = evp1d_subcycles(h, ndte);
+  rc = evp::settle(h, evp1d_subcycles(h, ndte));
   if (rc != EVP1D_OK) return rc;
-  rc = evp1d_synchronize(h);  // also reports a bounded device wait that ran out
+  int code = 0;
+  rc = evp::settle(h, evp::problem_download(&P, o, &code));
   if (rc != EVP1D_OK) return rc;
-  // 1D results -> their cells of the device copies -> the caller's arrays
-  const bool no_str[8] = {false, false, false, false, false, false, false, false};
-  rc = evp::problem_download_staged(&P, no_str);
-  if (rc != EVP1D_OK) return rc;
-  Scatter2d o;
-  double *dst[kOut2d];
-  for (int k = 0; k < 12; k++) o.f[k] = d->f2d + (size_t)(kIn2d + k) * cells;
-  for (int k = 0; k < 5; k++) o.f[12 + k] = d->f2d + (size_t)(24 + k) * cells;
-  k_scatter_2d<<<grid_for(d->na), 256, 0, st>>>(d->na, d->navel, d->cell, P.stage, o);
-  DYN_TRY(cudaGetLastError());
-  for (int k = 0; k < 12; k++) dst[k] = io->stress[k];
-  dst[12] = io->strintxU;
-  dst[13] = io->strintyU;
-  dst[14] = io->Cb;
-  dst[15] = io->uvel;
-  dst[16] = io->vvel;
-  for (int k = 0; k < kOut2d; k++)
-    DYN_TRY(cudaMemcpyAsync(dst[k], o.f[k], bc, cudaMemcpyDeviceToHost, st));
-  DYN_TRY(cudaStreamSynchronize(st));
-  return EVP1D_OK;
+  return code ? evp::timeout_error(code) : EVP1D_OK;
 }
 
 int evp1d_dyn_finalize(evp1d_dyn_t *d) {

@@ -16,6 +16,10 @@ void adjoint_release(AdjointState *a);
 void exchange_release(evp1d_handle *h);
 // Forget the recorded forward (the inputs or parameters changed).
 void adjoint_invalidate(AdjointState *a);
+// evp1d_upload; without `wait` the arrays are still being read on return.
+int upload_fields(evp1d_handle *h, const evp1d_fields *io, bool wait);
+// rc; if it is an error, after the handle's stream has ended.
+int settle(evp1d_handle *h, int rc);
 // Whether a call of n subcycles, queued now on the handle's stream, takes the
 // resident launch.  Not under stream capture: its mailbox numbers are launch
 // arguments, and a replay would find the previous replay's messages.

@@ -17,6 +17,8 @@ namespace evp {
 
 // Record `fmt` as this thread's last error message and return `code`.
 int error(int code, const char *fmt, ...);
+// EVP1D_ERR_TIMEOUT for the error word's `code`.
+int timeout_error(int code);
 
 // A named NVTX range over a scope, so that the public calls show on a
 // profiler's timeline (header-only NVTX; without a profiler it does nothing).
@@ -58,6 +60,12 @@ struct DeviceProblem {
   int32_t *tile_off = nullptr, *tile_cnt = nullptr, *halo_off = nullptr;
   int32_t *halo_cnt = nullptr, *halo_idx = nullptr;
   int32_t *slot_of_point = nullptr, *point_of_slot = nullptr;
+  int32_t *tile_of_quad = nullptr;  // tile of slots 4q..4q+3
+  // batched: caller's position of each list point, then each halo slot
+  int32_t *uv_pos = nullptr;
+  // page-locked copy of the error word (pinned_word; null: none was left)
+  int *err_host = nullptr;
+  bool pins = false;        // holds a reference to the page-locked pool
   int32_t *nb[6] = {};  // ee ne se nw sw sse, slot space
   uint32_t *lnb = nullptr;   // static packed stepu neighbours
   uint32_t *meta = nullptr;  // lnb | skip flags << 30 (per call)
@@ -98,25 +106,55 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
                    const ResidentPlan &res, const double *const geo[kNumGeo]);
 void problem_destroy(DeviceProblem *d);
 
-// Per-call fields host -> device (through the staging area); str zeroed;
-// uvel_init/vvel_init default to the uploaded velocities; the drag factor
-// (aiu*rhow)*Cw is precomputed; cur = 0.
-int problem_upload(DeviceProblem *d, const evp1d_fields *io, double rhow);
-// The device half of problem_upload: from the reference-order staging area
-// (slots 0..11 per-call inputs, 12..23 stresses, 24 u, 25 v [navel], 26 uinit,
-// 27 vinit, 28 strintx, 29 strinty, 30 Cb, 31 skipT then skipU as int32) into
-// the slot-ordered state.
-int problem_upload_staged(DeviceProblem *d, bool uinit_given, bool vinit_given, double rhow);
-// The device half of problem_download: slot-ordered results into the staging
-// area in reference order (slots 0..11 stresses, 12 u, 13 v, 14 strintx,
-// 15 strinty, 16 Cb, 17 + k str_k when want_str[k]).
-int problem_download_staged(DeviceProblem *d, const bool want_str[8]);
+// The host arrays of one call.  Per-point fields have n_f elements, point p
+// at map_f[p] (null: at p); u and v have n_uv, at map_uv[p] (null: as the
+// fields; halo slots at their own index).  `stage` is device staging for
+// arrays the GPU cannot address, stage_step doubles apart: 0..11 the inputs,
+// 12..23 the stresses, strintx, strinty, Cb, u, v, uinit, vinit; istage has
+// room for the two skip arrays.
+struct UploadFields {
+  const double *in[12] = {}, *stress[12] = {};
+  const double *u = nullptr, *v = nullptr, *uinit = nullptr, *vinit = nullptr;
+  const double *strintx = nullptr, *strinty = nullptr, *Cb = nullptr;
+  const int32_t *skT = nullptr, *skU = nullptr;
+  bool mask = false;       // skT, skU are ice masks (nonzero: not skipped)
+  bool zero_halo = false;  // halo velocities are 0, not read
+  size_t n_f = 0, n_uv = 0;
+  const int32_t *map_f = nullptr, *map_uv = nullptr;  // device
+  double *stage = nullptr;
+  size_t stage_step = 0;
+  int32_t *istage = nullptr;
+};
+// Where one call's results go (null: not wanted); u and v: n_u elements where
+// the array is staged (the list points come first there), str: n_str.
+struct DownloadFields {
+  double *stress[12] = {}, *u = nullptr, *v = nullptr, *strintx = nullptr, *strinty = nullptr;
+  double *Cb = nullptr, *str[8] = {};
+  size_t n_f = 0, n_u = 0, n_str = 0;
+  const int32_t *map_f = nullptr, *map_uv = nullptr;
+  double *stage = nullptr;
+  size_t stage_step = 0;
+};
+// Page-locked memory shared by the handles of the process, allocated on first
+// use (a page-locking call takes 2.5 ms, however small) and freed with the
+// last handle: a page of words, one per handle, and one staging buffer of
+// kPinnedStage bytes that a call borrows.  All are safe from several threads.
+void pinned_hold(DeviceProblem *d);     // takes a reference and a word
+void pinned_release(DeviceProblem *d);
+// Whether the GPU can address the `bytes` bytes of host memory at p
+// (page-locked or managed, the whole range, `align`ed); *dev: at which address.
+bool device_view(const void *p, size_t bytes, size_t align, void **dev);
+// Fields host -> device: state in both sets, slot-ordered inputs, drag factor
+// (aiu*rhow)*Cw, constant blocks; str zeroed; uvel_init/vvel_init default to
+// the velocities; cur = 0.  With `wait` the arrays may be changed afterwards.
+int problem_upload(DeviceProblem *d, const UploadFields &f, double rhow, bool wait);
+// Results device -> host; waits for the stream.  *code: the error word of the
+// bounded waits, cleared; if it is set, no result has been written.
+int problem_download(DeviceProblem *d, const DownloadFields &f, int *code);
 // Rebuild the per-tile constant blocks from the slot arrays (after the
 // per-call fields or the drag factor changed), with the field checks in
 // cflags.
 int problem_fill_const(DeviceProblem *d);
-// Results device -> host; waits for the stream.
-int problem_download(DeviceProblem *d, const evp1d_fields *io);
 
 // Views for the kernels.
 DevState problem_inplace_view(const DeviceProblem &d);

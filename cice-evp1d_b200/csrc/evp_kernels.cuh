@@ -232,11 +232,9 @@ void launch_scatter(const PermBatch &b, int nslots, const int32_t *point_of_slot
 // dst[f][p] = src[f][slot_of_point[p]], p < na.
 void launch_gather(const PermBatch &b, int na, const int32_t *slot_of_point,
                    cudaStream_t st);
-// flags[s] from int32 skipT/skipU in reference order (padding: both bits);
-// meta[s] = lnb[s] | flags[s] << 30.
-void launch_flags(int nslots, const int32_t *point_of_slot,
-                  const int32_t *skipT, const int32_t *skipU, uint8_t *flags,
-                  const uint32_t *lnb, uint32_t *meta, cudaStream_t st);
+// flags[s] = both bits, meta[s] = lnb[s] | flags[s] << 30.
+void launch_skip_all(int nslots, uint8_t *flags, const uint32_t *lnb, uint32_t *meta,
+                     cudaStream_t st);
 // cblk[(t*kConstFields + f)*256 + l] for l < tile_cnt[t] and slot
 // s = tile_off[t] + l: src[f][s] for f < 7, meta[s] | lcor[s] << 32 with the
 // sign bits of uinit (src[18]) and vinit (src[19]) in bits 62 and 63 for

@@ -147,16 +147,11 @@ __global__ void k_gather(PermBatch b, int na, const int32_t *sop) {
   }
 }
 
-__global__ void k_flags(int nslots, const int32_t *pos, const int32_t *skipT,
-                        const int32_t *skipU, uint8_t *flags,
-                        const uint32_t *lnb, uint32_t *meta) {
+__global__ void k_skip_all(int nslots, uint8_t *flags, const uint32_t *lnb, uint32_t *meta) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nslots;
        s += gridDim.x * blockDim.x) {
-    const int p = pos[s];
-    const uint8_t f = p < 0 ? (uint8_t)(kSkipT | kSkipU)
-                            : (uint8_t)((skipT[p] ? kSkipT : 0) | (skipU[p] ? kSkipU : 0));
-    flags[s] = f;
-    meta[s] = lnb[s] | ((uint32_t)f << 30);
+    flags[s] = kSkipT | kSkipU;
+    meta[s] = lnb[s] | ((uint32_t)(kSkipT | kSkipU) << 30);
   }
 }
 
@@ -195,11 +190,10 @@ void launch_gather(const PermBatch &b, int na, const int32_t *sop,
   k_gather<<<blocks_for(na), 256, 0, st>>>(b, na, sop);
 }
 
-void launch_flags(int nslots, const int32_t *pos, const int32_t *skipT,
-                  const int32_t *skipU, uint8_t *flags, const uint32_t *lnb,
-                  uint32_t *meta, cudaStream_t st) {
+void launch_skip_all(int nslots, uint8_t *flags, const uint32_t *lnb, uint32_t *meta,
+                     cudaStream_t st) {
   if (nslots <= 0) return;
-  k_flags<<<blocks_for(nslots), 256, 0, st>>>(nslots, pos, skipT, skipU, flags, lnb, meta);
+  k_skip_all<<<blocks_for(nslots), 256, 0, st>>>(nslots, flags, lnb, meta);
 }
 
 void launch_drag_factor(int n, const double *aiu, const double *Cw,

@@ -1,6 +1,4 @@
-// evp_problem.cu -- device arena of one 1D problem and its movement between
-// the caller's reference-order host arrays and the slot-ordered device state.
-#include <cstring>
+// evp_problem.cu -- device arena of one 1D problem and the kernels' views of it.
 #include <vector>
 
 #include "evp_internal.h"
@@ -44,12 +42,6 @@ int h2d(void *dst, const void *src, size_t bytes, cudaStream_t st) {
   return EVP1D_OK;
 }
 
-int d2h(void *dst, const void *src, size_t bytes, cudaStream_t st) {
-  if (bytes == 0) return EVP1D_OK;
-  CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
-  return EVP1D_OK;
-}
-
 void layout(DeviceProblem *d, Carve &c, size_t nhalo_total, size_t nuvx_total,
             size_t ndep_total) {
   const size_t R = (size_t)d->res_blocks * (size_t)d->res_threads;
@@ -77,6 +69,7 @@ void layout(DeviceProblem *d, Carve &c, size_t nhalo_total, size_t nuvx_total,
   c.take(&d->halo_idx, nhalo_total);
   c.take(&d->slot_of_point, (size_t)d->na);
   c.take(&d->point_of_slot, S);
+  c.take(&d->tile_of_quad, S / kSlotAlign);
   for (int k = 0; k < 6; k++) c.take(&d->nb[k], S);
   c.take(&d->lnb, S);
   c.take(&d->flags, S);
@@ -124,6 +117,7 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
     d->res_threads = res.threads;
     d->res_cls = res.cls;
   }
+  pinned_hold(d);
   Carve sizing;
   layout(d, sizing, plan.halo_idx.size(), plan.uvx_idx.size(), plan.dep_idx.size());
   CUDA_TRY(device_alloc(&d->arena, sizing.off));
@@ -149,6 +143,11 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
   TRY(h2d(d->halo_idx, plan.halo_idx.data(), plan.halo_idx.size() * sizeof(int32_t), st));
   TRY(h2d(d->slot_of_point, plan.slot_of_point.data(), (size_t)d->na * sizeof(int32_t), st));
   TRY(h2d(d->point_of_slot, plan.point_of_slot.data(), S4, st));
+  std::vector<int32_t> quad((size_t)d->nslots / kSlotAlign);
+  for (int t = 0; t < d->ntiles; t++)
+    for (int s = plan.tile_off[t]; s < plan.tile_off[t] + plan.tile_cnt[t]; s += kSlotAlign)
+      quad[s / kSlotAlign] = t;
+  TRY(h2d(d->tile_of_quad, quad.data(), quad.size() * sizeof(int32_t), st));
   const std::vector<int32_t> *nbv[6] = {&plan.ee, &plan.ne, &plan.se,
                                         &plan.nw, &plan.sw, &plan.sse};
   for (int k = 0; k < 6; k++) TRY(h2d(d->nb[k], nbv[k]->data(), S4, st));
@@ -204,6 +203,10 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
     b.n++;
   }
   launch_scatter(b, d->nslots, d->point_of_slot, st);
+  // every slot skipped until an upload (padding slots stay so), and the
+  // constant blocks' geometry and padding
+  launch_skip_all(d->nslots, d->flags, d->lnb, d->meta, st);
+  TRY(problem_fill_const(d));
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(st));
   return EVP1D_OK;
@@ -215,107 +218,12 @@ void problem_destroy(DeviceProblem *d) {
     cudaStreamSynchronize(d->stream);
   }
   if (d->arena) cudaFree(d->arena);
+  if (d->uv_pos) cudaFree(d->uv_pos);
+  pinned_release(d);
+  d->uv_pos = nullptr;
   if (d->stream) cudaStreamDestroy(d->stream);
   d->arena = nullptr;
   d->stream = nullptr;
-}
-
-int problem_upload(DeviceProblem *d, const evp1d_fields *io, double rhow) {
-  const int na = d->na, navel = d->navel;
-  if (na == 0) return EVP1D_OK;
-  const double *in[12] = {io->strength, io->Cw, io->aiu, io->uocn,
-                          io->vocn, io->waterx, io->watery, io->forcex,
-                          io->forcey, io->umassdti, io->fm, io->Tbu};
-  static const char *inname[12] = {"strength", "Cw", "aiu", "uocn",
-                                   "vocn", "waterx", "watery", "forcex",
-                                   "forcey", "umassdti", "fm", "Tbu"};
-  for (int k = 0; k < 12; k++)
-    if (!in[k]) return error(EVP1D_ERR_INVALID_ARG, "field %s is NULL", inname[k]);
-  for (int k = 0; k < 12; k++)
-    if (!io->stress[k]) return error(EVP1D_ERR_INVALID_ARG, "stress[%d] is NULL", k);
-  if (!io->skipT || !io->skipU || !io->uvel || !io->vvel || !io->strintx ||
-      !io->strinty || !io->Cb)
-    return error(EVP1D_ERR_INVALID_ARG,
-                 "skipT/skipU/uvel/vvel/strintx/strinty/Cb must not be NULL");
-  cudaStream_t st = d->stream;
-  const size_t bd = (size_t)na * sizeof(double);
-  const size_t bv = (size_t)navel * sizeof(double);
-  auto slot = [&](int k) { return d->stage + (size_t)k * navel; };
-  // staging slots: 0..11 per-call inputs, 12..23 stresses, 24 u, 25 v,
-  // 26 uinit, 27 vinit, 28 strintx, 29 strinty, 30 Cb, 31 skipT|skipU (int32)
-  for (int k = 0; k < 12; k++) TRY(h2d(slot(k), in[k], bd, st));
-  for (int k = 0; k < 12; k++) TRY(h2d(slot(12 + k), io->stress[k], bd, st));
-  TRY(h2d(slot(24), io->uvel, bv, st));
-  TRY(h2d(slot(25), io->vvel, bv, st));
-  if (io->uvel_init) TRY(h2d(slot(26), io->uvel_init, bd, st));
-  if (io->vvel_init) TRY(h2d(slot(27), io->vvel_init, bd, st));
-  TRY(h2d(slot(28), io->strintx, bd, st));
-  TRY(h2d(slot(29), io->strinty, bd, st));
-  TRY(h2d(slot(30), io->Cb, bd, st));
-  int32_t *skT = (int32_t *)slot(31);
-  int32_t *skU = skT + navel;  // 2 x navel int32 fit in navel doubles
-  TRY(h2d(skT, io->skipT, (size_t)na * sizeof(int32_t), st));
-  TRY(h2d(skU, io->skipU, (size_t)na * sizeof(int32_t), st));
-  return problem_upload_staged(d, io->uvel_init != nullptr, io->vvel_init != nullptr, rhow);
-}
-
-int problem_upload_staged(DeviceProblem *d, bool uinit_given, bool vinit_given, double rhow) {
-  const int na = d->na, navel = d->navel;
-  if (na == 0) return EVP1D_OK;
-  cudaStream_t st = d->stream;
-  auto slot = [&](int k) { return d->stage + (size_t)k * navel; };
-  const double *uinit_src = uinit_given ? slot(26) : slot(24);
-  const double *vinit_src = vinit_given ? slot(27) : slot(25);
-  int32_t *skT = (int32_t *)slot(31);
-  int32_t *skU = skT + navel;
-  launch_flags(d->nslots, d->point_of_slot, skT, skU, d->flags, d->lnb, d->meta, st);
-  PermBatch a;  // single-copy fields
-  for (int k = 0; k < 12; k++) {
-    a.src[a.n] = slot(k);
-    a.dst[a.n++] = d->dyn[k];
-  }
-  a.src[a.n] = uinit_src;
-  a.dst[a.n++] = d->dyn[kUinit];
-  a.src[a.n] = vinit_src;
-  a.dst[a.n++] = d->dyn[kVinit];
-  a.src[a.n] = slot(28);
-  a.dst[a.n++] = d->strintx;
-  a.src[a.n] = slot(29);
-  a.dst[a.n++] = d->strinty;
-  a.src[a.n] = slot(30);
-  a.dst[a.n++] = d->Cb;
-  launch_scatter(a, d->nslots, d->point_of_slot, st);
-  PermBatch b;  // state: both ping-pong buffers
-  for (int k = 0; k < 12; k++) {
-    b.src[b.n] = slot(12 + k);
-    b.dst[b.n] = d->stress[0][k];
-    b.dst2[b.n++] = d->stress[1][k];
-  }
-  b.src[b.n] = slot(24);
-  b.dst[b.n] = d->u[0];
-  b.dst2[b.n++] = d->u[1];
-  b.src[b.n] = slot(25);
-  b.dst[b.n] = d->v[0];
-  b.dst2[b.n++] = d->v[1];
-  launch_scatter(b, d->nslots, d->point_of_slot, st);
-  CUDA_TRY(cudaGetLastError());
-  if (d->nhs > 0) {
-    const size_t bh = (size_t)d->nhs * sizeof(double);
-    for (int k = 0; k < 2; k++) {
-      CUDA_TRY(cudaMemcpyAsync(d->u[k] + d->nslots, slot(24) + na, bh,
-                               cudaMemcpyDeviceToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(d->v[k] + d->nslots, slot(25) + na, bh,
-                               cudaMemcpyDeviceToDevice, st));
-    }
-  }
-  launch_drag_factor(d->nslots, d->dyn[kAiu], d->dyn[kCw], rhow, d->dyn[kKvrel], st);
-  TRY(problem_fill_const(d));
-  for (int k = 0; k < 8; k++)
-    CUDA_TRY(cudaMemsetAsync(d->str[k], 0, (size_t)d->nuv * sizeof(double), st));
-  CUDA_TRY(cudaGetLastError());
-  CUDA_TRY(cudaStreamSynchronize(st));
-  d->cur = 0;
-  return EVP1D_OK;
 }
 
 int problem_fill_const(DeviceProblem *d) {
@@ -328,64 +236,6 @@ int problem_fill_const(DeviceProblem *d) {
   CUDA_TRY(cudaMemsetAsync(d->cflags, 0, sizeof(int), d->stream));
   launch_const_blocks(d->ntiles, d->tile_off, d->tile_cnt, src, d->meta, d->lcor, d->cblk,
                       d->cflags, d->stream);
-  CUDA_TRY(cudaGetLastError());
-  return EVP1D_OK;
-}
-
-int problem_download(DeviceProblem *d, const evp1d_fields *io) {
-  const int na = d->na, navel = d->navel;
-  if (na == 0) return EVP1D_OK;
-  cudaStream_t st = d->stream;
-  auto slot = [&](int k) { return d->stage + (size_t)k * navel; };
-  bool want_str[8];
-  for (int k = 0; k < 8; k++) want_str[k] = io->str[k] != nullptr;
-  TRY(problem_download_staged(d, want_str));
-  const size_t bd = (size_t)na * sizeof(double);
-  for (int k = 0; k < 12; k++)
-    if (io->stress[k]) TRY(d2h(io->stress[k], slot(k), bd, st));
-  if (io->uvel) TRY(d2h(io->uvel, slot(12), bd, st));
-  if (io->vvel) TRY(d2h(io->vvel, slot(13), bd, st));
-  if (io->strintx) TRY(d2h(io->strintx, slot(14), bd, st));
-  if (io->strinty) TRY(d2h(io->strinty, slot(15), bd, st));
-  if (io->Cb) TRY(d2h(io->Cb, slot(16), bd, st));
-  for (int k = 0; k < 8; k++)
-    if (io->str[k]) {
-      TRY(d2h(io->str[k], slot(17 + k), bd, st));
-      if (d->nhs > 0)
-        TRY(d2h(io->str[k] + na, d->str[k] + d->nslots,
-                (size_t)d->nhs * sizeof(double), st));
-    }
-  CUDA_TRY(cudaStreamSynchronize(st));
-  return EVP1D_OK;
-}
-
-int problem_download_staged(DeviceProblem *d, const bool want_str[8]) {
-  const int na = d->na, navel = d->navel;
-  if (na == 0) return EVP1D_OK;
-  cudaStream_t st = d->stream;
-  auto slot = [&](int k) { return d->stage + (size_t)k * navel; };
-  PermBatch g;
-  const int c = d->cur;
-  for (int k = 0; k < 12; k++) {
-    g.src[g.n] = d->stress[c][k];
-    g.dst[g.n++] = slot(k);
-  }
-  g.src[g.n] = d->u[c];
-  g.dst[g.n++] = slot(12);
-  g.src[g.n] = d->v[c];
-  g.dst[g.n++] = slot(13);
-  g.src[g.n] = d->strintx;
-  g.dst[g.n++] = slot(14);
-  g.src[g.n] = d->strinty;
-  g.dst[g.n++] = slot(15);
-  g.src[g.n] = d->Cb;
-  g.dst[g.n++] = slot(16);
-  for (int k = 0; k < 8; k++)
-    if (want_str[k]) {
-      g.src[g.n] = d->str[k];
-      g.dst[g.n++] = slot(17 + k);
-    }
-  launch_gather(g, na, d->slot_of_point, st);
   CUDA_TRY(cudaGetLastError());
   return EVP1D_OK;
 }
@@ -572,8 +422,10 @@ cudaError_t problem_launch_resident(DeviceProblem *d, const Params &p, int nsub,
 
 int problem_take_error(DeviceProblem *d, int *code) {
   int v = 0;
-  CUDA_TRY(cudaMemcpyAsync(&v, d->err, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
+  int *to = d->err_host ? d->err_host : &v;
+  CUDA_TRY(cudaMemcpyAsync(to, d->err, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
   CUDA_TRY(cudaStreamSynchronize(d->stream));
+  v = *to;
   if (v) CUDA_TRY(cudaMemsetAsync(d->err, 0, sizeof(int), d->stream));
   *code = v;
   return EVP1D_OK;

@@ -1,0 +1,473 @@
+// evp_transfer.cu -- a call's fields between the caller's host arrays and the
+// slot-ordered device state.
+//
+// Arrays that the GPU can address (page-locked or managed memory, the whole
+// range checked) are read and written by the kernels themselves, each field
+// once, in the caller's order: k_upload takes a point's 29 values, skip flags
+// included, and writes every place they go to (both state sets, the
+// slot-ordered inputs, the constant blocks); k_download gathers the results.
+// Other arrays pass through page-locked staging of the handle when they are
+// small (one copy by the host, then the same kernels), else through device
+// staging with cudaMemcpyAsync.
+//
+// What bounds it: the host link for large calls; for small ones it was the
+// number of copies (31 up, 17 down, about 2 us each, and a dozen kernels
+// and fills): 2.0k points took 190 us up and 90 us down.
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+#include "evp_internal.h"
+
+namespace evp {
+
+namespace {
+
+#define CUDA_TRY(x)                                                        \
+  do {                                                                     \
+    cudaError_t e_ = (x);                                                  \
+    if (e_ != cudaSuccess)                                                 \
+      return error(e_ == cudaErrorMemoryAllocation ? EVP1D_ERR_NOMEM       \
+                                                   : EVP1D_ERR_CUDA,       \
+                   "%s: %s", #x, cudaGetErrorString(e_));                  \
+  } while (0)
+
+// Staged bytes of one call up to which they go through page-locked staging
+// (the host copies them at about 10 GB/s, one array after another); above,
+// cudaMemcpyAsync's own pipelining of pageable memory wins.
+constexpr size_t kPinnedStage = 8u << 20;
+
+// Bytes of one call up to which the kernels go to addressable host arrays
+// themselves.  They move about 40 GB/s over the host link where
+// cudaMemcpyAsync's copy engine moves 55, which pays for its 31 (17) copies of
+// 3 us each only in larger calls, us up and down by the kernels and by copies:
+// 74k points 406, 240 and 537, 268; 124k 675, 370 and 731, 398; 296k 1765,
+// 1085 and 1629, 829.  Calls with an index map (2D arrays: only the list's
+// cells travel) always go direct.
+constexpr size_t kDirectUp = 40u << 20, kDirectDown = 20u << 20;
+
+constexpr int kThreads = 128;
+
+struct UploadArgs {
+  int na, navel, nslots, nuv;
+  const int32_t *slot_of_point, *tile_of_quad, *tile_off;
+  const int32_t *map_f, *map_uv;  // null: the point itself
+  bool mask, zero_halo;
+  double rhow;
+  const double *in[12], *stress[12];
+  const double *u, *v, *uinit, *vinit, *strintx, *strinty, *Cb;
+  const int32_t *skT, *skU;
+  // destinations, by slot
+  double *dyn[kNumDyn];
+  double *s0[12], *s1[12], *u0, *u1, *v0, *v1, *o_strintx, *o_strinty, *o_Cb, *str[8];
+  const uint32_t *lnb, *lcor;
+  uint8_t *flags;
+  uint32_t *meta;
+  double *cblk;
+  int *cflags;
+};
+
+__global__ void __launch_bounds__(kThreads) k_upload(UploadArgs a) {
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (i < a.nuv) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) a.str[k][i] = 0.0;
+  }
+  if (i >= a.navel) return;
+  if (i >= a.na) {  // the reference's halo slots
+    const int s = a.nslots + (i - a.na);
+    double u = 0.0, v = 0.0;
+    if (!a.zero_halo) {
+      const int c = a.map_uv ? a.map_uv[i] : i;
+      u = a.u[c];
+      v = a.v[c];
+    }
+    a.u0[s] = a.u1[s] = u;
+    a.v0[s] = a.v1[s] = v;
+    return;
+  }
+  const int s = a.slot_of_point[i];
+  const int c = a.map_f ? a.map_f[i] : i;
+  const int cu = a.map_uv ? a.map_uv[i] : c;
+  double in[12], st[12];
+#pragma unroll
+  for (int k = 0; k < 12; k++) in[k] = a.in[k][c];
+#pragma unroll
+  for (int k = 0; k < 12; k++) st[k] = a.stress[k][c];
+  const double u = a.u[cu], v = a.v[cu];
+  const double ui = a.uinit ? a.uinit[c] : u, vi = a.vinit ? a.vinit[c] : v;
+  const double sx = a.strintx[c], sy = a.strinty[c], cb = a.Cb[c];
+  const int32_t mt = a.skT[c], mu = a.skU[c];
+  const uint32_t fl = ((mt != 0) != a.mask ? kSkipT : 0u) | ((mu != 0) != a.mask ? kSkipU : 0u);
+  const uint32_t meta = a.lnb[s] | fl << 30;
+  a.flags[s] = (uint8_t)fl;
+  a.meta[s] = meta;
+  const double kv = drag_factor(in[kAiu], a.rhow, in[kCw]);
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    a.dyn[k][s] = in[k];
+    a.s0[k][s] = st[k];
+    a.s1[k][s] = st[k];
+  }
+  a.dyn[kUinit][s] = ui;
+  a.dyn[kVinit][s] = vi;
+  a.dyn[kKvrel][s] = kv;
+  a.u0[s] = a.u1[s] = u;
+  a.v0[s] = a.v1[s] = v;
+  a.o_strintx[s] = sx;
+  a.o_strinty[s] = sy;
+  a.o_Cb[s] = cb;
+  // the tile's constant block (launch_const_blocks), without the geometry
+  const int t = a.tile_of_quad[s >> 2];
+  double *blk = a.cblk + (size_t)t * kConstFields * kConstTileSlots + (s - a.tile_off[t]);
+  const unsigned long long su = (unsigned long long)__double_as_longlong(ui) >> 63;
+  const unsigned long long sv = (unsigned long long)__double_as_longlong(vi) >> 63;
+  auto put = [&](int f, double x) { blk[(size_t)f * kConstTileSlots] = x; };
+  put(6, in[kStrength]);
+  put(7, __longlong_as_double((long long)((unsigned long long)meta |
+                                          ((unsigned long long)a.lcor[s] << 32) | su << 62 |
+                                          sv << 63)));
+  put(8, kv);
+#pragma unroll
+  for (int k = kUocn; k <= kFm; k++) put(9 + (k - kUocn), in[k]);
+  put(18, in[kTbu]);
+  put(19, ui);
+  put(20, vi);
+  const int bad = (__double_as_longlong(in[kTbu]) != 0 ? 1 : 0) |
+                  (!isfinite(ui) || !isfinite(vi) ? 2 : 0);
+  if (bad) atomicOr(a.cflags, bad);
+}
+static_assert(kConstStressFields == 8 && kConstFields == 21 && kFm - kUocn == 7,
+              "constant block layout");
+
+struct DownloadArgs {
+  int na, navel, nslots;
+  const int32_t *slot_of_point;
+  const int32_t *map_f, *map_uv;
+  const double *s[12], *u, *v, *strintx, *strinty, *Cb, *str[8];
+  double *o_s[12], *o_u, *o_v, *o_strintx, *o_strinty, *o_Cb, *o_str[8];  // null: not wanted
+  const int *err;
+};
+
+__global__ void __launch_bounds__(kThreads) k_download(DownloadArgs a) {
+  // a wait that ran out: the results are not valid, the caller's arrays stay
+  if (*a.err) return;
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= a.navel) return;
+  const int s = i < a.na ? a.slot_of_point[i] : a.nslots + (i - a.na);
+  const int cu = a.map_uv ? a.map_uv[i] : i;
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (a.o_str[k]) a.o_str[k][cu] = a.str[k][s];
+  if (i >= a.na) return;  // halo velocities are never written
+  const int c = a.map_f ? a.map_f[i] : i;
+  const int cv = a.map_uv ? cu : c;
+#pragma unroll
+  for (int k = 0; k < 12; k++)
+    if (a.o_s[k]) a.o_s[k][c] = a.s[k][s];
+  if (a.o_u) a.o_u[cv] = a.u[s];
+  if (a.o_v) a.o_v[cv] = a.v[s];
+  if (a.o_strintx) a.o_strintx[c] = a.strintx[s];
+  if (a.o_strinty) a.o_strinty[c] = a.strinty[s];
+  if (a.o_Cb) a.o_Cb[c] = a.Cb[s];
+}
+
+// The driver's range query: where an address is page-locked, managed or device
+// memory, the allocation around it.
+using PtrAttrs = int (*)(unsigned, int *, void **, unsigned long long);
+
+PtrAttrs ptr_attrs() {
+  static const PtrAttrs f = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) !=
+            cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return reinterpret_cast<PtrAttrs>(p);
+  }();
+  return f;
+}
+
+struct PinnedPool {
+  static constexpr int kWords = 1024;
+  std::mutex m;
+  int refs = 0;
+  int *words = nullptr;
+  bool used[kWords] = {};
+  void *stage = nullptr;
+  bool lent = false;
+};
+PinnedPool &pool() {
+  static PinnedPool p;
+  return p;
+}
+
+// The staging buffer, or null while another call has it (the caller then
+// takes device staging).
+void *borrow_stage() {
+  PinnedPool &p = pool();
+  std::lock_guard<std::mutex> lock(p.m);
+  if (p.lent) return nullptr;
+  if (!p.stage && cudaHostAlloc(&p.stage, kPinnedStage, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    p.stage = nullptr;
+    return nullptr;
+  }
+  p.lent = true;
+  return p.stage;
+}
+
+void return_stage() {
+  PinnedPool &p = pool();
+  std::lock_guard<std::mutex> lock(p.m);
+  p.lent = false;
+}
+
+}  // namespace
+
+void pinned_hold(DeviceProblem *d) {
+  PinnedPool &p = pool();
+  std::lock_guard<std::mutex> lock(p.m);
+  p.refs++;
+  d->pins = true;
+  if (!p.words && cudaHostAlloc((void **)&p.words, sizeof(int) * PinnedPool::kWords,
+                                cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    p.words = nullptr;
+    return;
+  }
+  for (int k = 0; k < PinnedPool::kWords; k++)
+    if (!p.used[k]) {
+      p.used[k] = true;
+      d->err_host = p.words + k;
+      return;
+    }
+}
+
+void pinned_release(DeviceProblem *d) {
+  if (!d->pins) return;
+  PinnedPool &p = pool();
+  std::lock_guard<std::mutex> lock(p.m);
+  d->pins = false;
+  if (d->err_host) p.used[d->err_host - p.words] = false;
+  d->err_host = nullptr;
+  if (--p.refs > 0) return;
+  if (p.words) cudaFreeHost(p.words);
+  if (p.stage && !p.lent) {
+    cudaFreeHost(p.stage);
+    p.stage = nullptr;
+  }
+  p.words = nullptr;
+}
+
+bool device_view(const void *p, size_t bytes, size_t align, void **dev) {
+  PtrAttrs query = ptr_attrs();
+  if (!query || !p || bytes == 0) return false;
+  // CUpointer_attribute: MEMORY_TYPE 2, DEVICE_POINTER 3, IS_MANAGED 8,
+  // RANGE_START_ADDR 11, RANGE_SIZE 12
+  int what[5] = {2, 3, 8, 11, 12};
+  unsigned type = 0, managed = 0;
+  unsigned long long dptr = 0, start = 0;
+  size_t size = 0;
+  void *out[5] = {&type, &dptr, &managed, &start, &size};
+  const unsigned long long at = (unsigned long long)(uintptr_t)p;
+  if (query(5, what, out, at) != 0) return false;
+  constexpr unsigned kHost = 1;  // CU_MEMORYTYPE_HOST
+  if (!(type == kHost || managed) || dptr == 0 || start == 0) return false;
+  // the range query gives the allocation in the address space it is asked in
+  // (host addresses of page-locked memory equal its device addresses); an
+  // array that only begins in registered memory is not addressable
+  const unsigned long long base = at >= start && at < start + size ? at : dptr;
+  if (base < start || bytes > size || base - start > size - bytes) return false;
+  if (dptr % align) return false;
+  *dev = reinterpret_cast<void *>((uintptr_t)dptr);
+  return true;
+}
+
+namespace {
+
+// Where each array of a call is for the kernels.
+struct Placer {
+  size_t direct_limit;
+  explicit Placer(size_t limit) : direct_limit(limit) {}
+  ~Placer() {
+    if (pinned) return_stage();
+  }
+  Placer(const Placer &) = delete;
+  Placer &operator=(const Placer &) = delete;
+  struct Item {
+    const void *host;
+    void *stage;  // device staging of the array
+    size_t bytes;
+    void **dev;   // the pointer the kernels get
+    size_t off = 0;
+  };
+  std::vector<Item> staged, direct;
+  size_t total = 0, direct_total = 0;
+  bool pinned = false;
+
+  // dev: device address for the kernels, at once where the GPU can address the
+  // array, else set by place().  `fixed`: an array its map makes direct.
+  void add(const void *host, size_t bytes, size_t align, void *stage, void **dev,
+           bool fixed = false) {
+    if (device_view(host, bytes, align, dev)) {
+      if (!fixed) {
+        direct.push_back({host, stage, bytes, dev});
+        direct_total += bytes;
+      }
+    } else {
+      stage_it({host, stage, bytes, dev});
+    }
+  }
+  void stage_it(Item it) {
+    *it.dev = it.stage;
+    it.off = total;
+    total += (it.bytes + 255) & ~size_t(255);
+    staged.push_back(it);
+  }
+  // Page-locked staging for the staged arrays, where they are small; the copy
+  // engine for addressable ones, where they are many.
+  void place() {
+    if (direct_total > direct_limit) {
+      for (const Item &it : direct) stage_it(it);
+      return;
+    }
+    if (staged.empty() || total > kPinnedStage) return;
+    char *base = static_cast<char *>(borrow_stage());
+    if (!base) return;
+    pinned = true;
+    for (Item &it : staged) *it.dev = base + it.off;
+  }
+};
+
+}  // namespace
+
+int problem_upload(DeviceProblem *d, const UploadFields &f, double rhow, bool wait) {
+  if (d->na == 0) return EVP1D_OK;
+  cudaStream_t st = d->stream;
+  UploadArgs a;
+  a.na = d->na;
+  a.navel = d->navel;
+  a.nslots = d->nslots;
+  a.nuv = d->nuv;
+  a.slot_of_point = d->slot_of_point;
+  a.tile_of_quad = d->tile_of_quad;
+  a.tile_off = d->tile_off;
+  a.map_f = f.map_f;
+  a.map_uv = f.map_uv;
+  a.mask = f.mask;
+  a.zero_halo = f.zero_halo;
+  a.rhow = rhow;
+  Placer P(kDirectUp);
+  const size_t bf = f.n_f * sizeof(double), bu = f.n_uv * sizeof(double);
+  int slot = 0;
+  auto take = [&](const double *host, size_t bytes, const double **dev, bool fixed = false) {
+    double *stage = f.stage + (size_t)(slot++) * f.stage_step;
+    P.add(host, bytes, sizeof(double), stage, (void **)dev, fixed);
+  };
+  for (int k = 0; k < 12; k++) take(f.in[k], bf, &a.in[k]);
+  for (int k = 0; k < 12; k++) take(f.stress[k], bf, &a.stress[k]);
+  take(f.strintx, bf, &a.strintx);
+  take(f.strinty, bf, &a.strinty);
+  take(f.Cb, bf, &a.Cb);
+  take(f.u, bu, &a.u, f.map_uv != nullptr);
+  take(f.v, bu, &a.v, f.map_uv != nullptr);
+  a.uinit = a.vinit = nullptr;
+  if (f.uinit) take(f.uinit, bf, &a.uinit);
+  if (f.vinit) take(f.vinit, bf, &a.vinit);
+  const size_t bi = f.n_f * sizeof(int32_t);
+  P.add(f.skT, bi, sizeof(int32_t), f.istage, (void **)&a.skT);
+  P.add(f.skU, bi, sizeof(int32_t), f.istage + f.n_f, (void **)&a.skU);
+  // (2D arrays: the device staging keeps the cells outside the list for the
+  // way back)
+  if (!f.map_f) P.place();
+  for (const Placer::Item &it : P.staged) {
+    if (P.pinned)
+      memcpy(*it.dev, it.host, it.bytes);
+    else
+      CUDA_TRY(cudaMemcpyAsync(it.stage, it.host, it.bytes, cudaMemcpyHostToDevice, st));
+  }
+  for (int k = 0; k < kNumDyn; k++) a.dyn[k] = d->dyn[k];
+  for (int k = 0; k < 12; k++) {
+    a.s0[k] = d->stress[0][k];
+    a.s1[k] = d->stress[1][k];
+  }
+  a.u0 = d->u[0];
+  a.u1 = d->u[1];
+  a.v0 = d->v[0];
+  a.v1 = d->v[1];
+  a.o_strintx = d->strintx;
+  a.o_strinty = d->strinty;
+  a.o_Cb = d->Cb;
+  for (int k = 0; k < 8; k++) a.str[k] = d->str[k];
+  a.lnb = d->lnb;
+  a.lcor = d->lcor;
+  a.flags = d->flags;
+  a.meta = d->meta;
+  a.cblk = d->cblk;
+  a.cflags = d->cflags;
+  CUDA_TRY(cudaMemsetAsync(d->cflags, 0, sizeof(int), st));
+  const int n = d->nuv > d->navel ? d->nuv : d->navel;
+  k_upload<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(a);
+  CUDA_TRY(cudaGetLastError());
+  // (the borrowed staging goes back when this returns)
+  if (wait || P.pinned) CUDA_TRY(cudaStreamSynchronize(st));
+  d->cur = 0;
+  return EVP1D_OK;
+}
+
+int problem_download(DeviceProblem *d, const DownloadFields &f, int *code) {
+  *code = 0;
+  if (d->na == 0) return EVP1D_OK;
+  cudaStream_t st = d->stream;
+  DownloadArgs a;
+  a.na = d->na;
+  a.navel = d->navel;
+  a.nslots = d->nslots;
+  a.slot_of_point = d->slot_of_point;
+  a.map_f = f.map_f;
+  a.map_uv = f.map_uv;
+  a.err = d->err;
+  const int c = d->cur;
+  Placer P(kDirectDown);
+  auto give = [&](const double *src, double *host, size_t elems, const double **from, double **to,
+                  int at, bool fixed = false) {
+    *from = src;
+    *to = nullptr;
+    double *stage = f.stage + (size_t)at * f.stage_step;
+    if (host) P.add(host, elems * sizeof(double), sizeof(double), stage, (void **)to, fixed);
+  };
+  const bool fixed = f.map_uv != nullptr;
+  for (int k = 0; k < 12; k++) give(d->stress[c][k], f.stress[k], f.n_f, &a.s[k], &a.o_s[k], 12 + k);
+  give(d->strintx, f.strintx, f.n_f, &a.strintx, &a.o_strintx, 24);
+  give(d->strinty, f.strinty, f.n_f, &a.strinty, &a.o_strinty, 25);
+  give(d->Cb, f.Cb, f.n_f, &a.Cb, &a.o_Cb, 26);
+  give(d->u[c], f.u, f.n_u, &a.u, &a.o_u, 27, fixed);
+  give(d->v[c], f.v, f.n_u, &a.v, &a.o_v, 28, fixed);
+  for (int k = 0; k < 8; k++)
+    give(d->str[k], f.str[k], f.n_str, &a.str[k], &a.o_str[k], k, fixed);
+  // Staged arrays of a 2D call hold the caller's values of the other cells in
+  // the device staging since the upload: they stay there.
+  if (!f.map_f) P.place();
+  if (!P.staged.empty() && !P.pinned) {
+    // nothing of the caller's is overwritten after a wait that ran out
+    const int rc = problem_take_error(d, code);
+    if (rc != EVP1D_OK || *code) return rc;
+  }
+  k_download<<<(d->navel + kThreads - 1) / kThreads, kThreads, 0, st>>>(a);
+  CUDA_TRY(cudaGetLastError());
+  if (!P.pinned)
+    for (const Placer::Item &it : P.staged)
+      CUDA_TRY(cudaMemcpyAsync(const_cast<void *>(it.host), it.stage, it.bytes,
+                               cudaMemcpyDeviceToHost, st));
+  const int rc = problem_take_error(d, code);  // waits for the stream
+  if (rc != EVP1D_OK || *code) return rc;
+  if (P.pinned)
+    for (const Placer::Item &it : P.staged) memcpy(const_cast<void *>(it.host), *it.dev, it.bytes);
+  return EVP1D_OK;
+}
+
+}  // namespace evp

@@ -126,11 +126,6 @@ cudaError_t launch_sub(evp1d_t *h, int from, bool last, bool after_sub) {
   return cudaGetLastError();
 }
 
-// Subcycles from which a call takes the resident launch: a single subcycle
-// costs as much in either form (about 11 us with its launch), and its results
-// would land in the set that other blocks still read.
-constexpr int kResidentMin = 2;
-
 // A bounded device-side wait that ran out leaves a code in the error word.
 int check_device_error(evp1d_t *h) {
   int code = 0;

@@ -167,7 +167,9 @@ k_adj_stepu(AdjArgs a, Params p, const double *__restrict__ u0, const double *__
     const double gfx = a.g[kGForcex][x], gfy = a.g[kGForcey][x], gcw = a.g[kGCw][x];
     // a skipped point (u(n+1) = u(n) there) passes lam on unchanged and
     // takes no gradient; selects, not branches, keep the loads above
-    const StepuAdjOut o = stepu_adjoint(in, p);
+    bool ok = true;
+    StepuAdjOut o = stepu_adjoint_t<true>(in, p, &ok);
+    if (!ok) o = stepu_adjoint(in, p);
     a.Pu[x] = skip ? lu : o.luold;
     a.Pv[x] = skip ? lv : o.lvold;
     a.Lx[x] = skip ? 0.0 : ar * o.lcc1;
@@ -239,6 +241,8 @@ k_adj_stress(AdjArgs a, Params p, const double *__restrict__ u, const double *__
     const Geom g = make_geom_fw(a.dxT[w], a.dyT[w], a.HTE[w], a.HTN[w], a.HTEm1[w],
                              a.HTNm1[w], p.deltaminEVP);
     double lc[8], lstr;
+    // (the straight-line form spills at 16 warps an SM and measured slower
+    // here, 47.1 against 41.8 us a subcycle for both kernels on 294k points)
     stress_adjoint(c, g, a.strength[w], p, lo, ls, lc, lstr);
 #pragma unroll
     for (int k = 0; k < 12; k++) a.LS[k][w] = ls[k];
@@ -318,6 +322,9 @@ struct AdjointState {
   int32_t *tr_off[kNumTr] = {}, *tr_idx[kNumTr] = {};
   int32_t *tr_one[kNumTr] = {};
   bool one = false;  // every transposed list has at most one entry
+  // the neighbour relations are each other's inverse, and the resident plan's
+  // blocks can run the reverse sweep (launch_resident_adjoint)
+  bool resident = false;
   double *Pu = nullptr, *Pv = nullptr, *Lx = nullptr, *Ly = nullptr;
   double *C8[8] = {}, *LS[12] = {}, *g[kNumGrad] = {};
   double *spp[2][12] = {};  // stress ping-pong of the segment recompute
@@ -414,6 +421,19 @@ int ensure_static(evp1d_t *h) {
         if (off[t][w + 1] > off[t][w]) direct[(size_t)t * S + w] = idx[t][off[t][w]];
   }
   A.one = one;
+  // nw of ee, sw of ne, sse of se and back, wherever both ends are list points
+  bool inverse = one;
+  for (int s = 0; s < S && inverse; s++) {
+    if (pos[s] < 0) continue;
+    const int pair[3][2] = {{0, 3}, {1, 4}, {2, 5}};
+    for (const auto &q : pair)
+      for (int r = 0; r < 2; r++) {
+        const int o = nbk(q[r], s);
+        if (o < S && nbk(q[1 - r], o) != s) inverse = false;
+      }
+  }
+  A.resident = inverse && h->resident && d.res_blocks > 0 && d.res_cls <= kResAdjointMax &&
+               resident_adjoint_prepare(d.device, d.res_cls, d.res_blocks) != 0;
   // carve
   const size_t SD = pad256((size_t)S);
   size_t ints = one ? (size_t)kNumTr * pad_ints((size_t)S) : 0;
@@ -817,11 +837,56 @@ int evp1d_adjoint_sweep(evp1d_t *h) {
     }
     launches += 2;
   };
+  // subcycles of `len` tape entries from e0 on, last first
+  auto reverse_range = [&](int e0, int len) {
+    // one form for every segment of a sweep, however short
+    if (A.resident && h->p.revp == 0.0 && use_resident(h, kResidentMin)) {
+      ResidentAdjArgs r;
+      r.nslots = d.nslots;
+      r.slot = d.res_slot;
+      r.cnt = d.res_cnt;
+      r.corner = d.res_corner;
+      r.str_idx = d.res_str;
+      r.flags = d.flags;
+      const int geo_order[6] = {kDxT, kDyT, kHTE, kHTN, kHTEm1, kHTNm1};
+      for (int k = 0; k < 6; k++) r.sg[k] = d.geo[geo_order[k]];
+      r.sg[6] = d.dyn[kStrength];
+      r.kvrel = a.kvrel;
+      r.aiu = a.aiu;
+      r.uocn = a.uocn;
+      r.vocn = a.vocn;
+      r.waterx = a.waterx;
+      r.watery = a.watery;
+      r.umassdti = a.umassdti;
+      r.fm = a.fm;
+      r.Tbu = a.Tbu;
+      r.uarear = a.uarear;
+      r.Pu = A.Pu;
+      r.Pv = A.Pv;
+      for (int k = 0; k < 8; k++) r.C8[k] = A.C8[k];
+      for (int k = 0; k < 12; k++) r.LS[k] = A.LS[k];
+      r.gs = A.g[kGStrength];
+      r.gC = A.g[kGCw];
+      r.gx = A.g[kGForcex];
+      r.gy = A.g[kGForcey];
+      r.tu = tape_u(A, e0);
+      r.tv = tape_v(A, e0);
+      r.step = 2 * A.stride;
+      r.nsub = len;
+      r.mail = d.res_mail;
+      r.seq = d.res_seq;
+      r.err = d.err;
+      d.res_seq += (unsigned)len;
+      keep(launch_resident_adjoint(r, h->p, d.res_cls, d.res_threads, d.res_blocks, st));
+      launches++;
+      return;
+    }
+    for (int i = len - 1; i >= 0; i--)
+      reverse_step(tape_u(A, e0 + i), tape_v(A, e0 + i), tape_u(A, e0 + i + 1),
+                   tape_v(A, e0 + i + 1));
+  };
   // taped tail
-  for (int n = A.ndte - 1; n >= A.n_cp; n--) {
-    const int e = n - A.n_cp;
-    reverse_step(tape_u(A, e), tape_v(A, e), tape_u(A, e + 1), tape_v(A, e + 1));
-  }
+  if (A.n_cp < A.ndte) reverse_range(0, A.ndte - A.n_cp);
   // checkpointed head, one segment at a time from the last
   const int k = A.interval;
   for (int j = A.nck - 1; j >= 0; j--) {
@@ -857,9 +922,7 @@ int evp1d_adjoint_sweep(evp1d_t *h) {
       ADJ_TRY(cudaMemcpyAsync(tape_v(A, e0 + len), ev, sizeof(double) * d.nuv,
                               cudaMemcpyDeviceToDevice, st));
     }
-    for (int i = len - 1; i >= 0; i--)
-      reverse_step(tape_u(A, e0 + i), tape_v(A, e0 + i), tape_u(A, e0 + i + 1),
-                   tape_v(A, e0 + i + 1));
+    reverse_range(e0, len);
   }
   if (one)
     k_adj_final<true><<<grid, kThreads, 0, st>>>(a, A.uinit_explicit ? 0 : 1);

@@ -20,6 +20,10 @@ void adjoint_invalidate(AdjointState *a);
 int upload_fields(evp1d_handle *h, const evp1d_fields *io, bool wait);
 // rc; if it is an error, after the handle's stream has ended.
 int settle(evp1d_handle *h, int rc);
+// Subcycles from which a call takes the resident launch: a single subcycle
+// costs as much in either form (about 11 us with its launch), and its results
+// would land in the set that other blocks still read.
+constexpr int kResidentMin = 2;
 // Whether a call of n subcycles, queued now on the handle's stream, takes the
 // resident launch.  Not under stream capture: its mailbox numbers are launch
 // arguments, and a replay would find the previous replay's messages.

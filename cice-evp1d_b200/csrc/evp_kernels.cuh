@@ -218,6 +218,36 @@ int resident_prepare(int device, int cls, int nblocks);
 cudaError_t launch_resident(const ResidentArgs &a, const Params &p, int cls, int threads,
                             int nblocks, cudaStream_t st);
 
+// The reverse sweep's subcycles in one launch on the same plan
+// (evp_adjoint_resident.cu), for lists whose neighbour relations are each
+// other's inverse (nw of ee, sw of ne, sse of se).  Widths up to
+// kResAdjointMax.
+struct ResidentAdjArgs {
+  int nslots = 0;
+  const int32_t *slot = nullptr, *cnt = nullptr, *corner = nullptr;
+  const uint32_t *str_idx = nullptr;
+  const uint8_t *flags = nullptr;
+  const double *sg[7] = {};  // dxT, dyT, HTE, HTN, HTEm1, HTNm1, strength by slot
+  const double *kvrel = nullptr, *aiu = nullptr, *uocn = nullptr, *vocn = nullptr;
+  const double *waterx = nullptr, *watery = nullptr, *umassdti = nullptr, *fm = nullptr;
+  const double *Tbu = nullptr, *uarear = nullptr;
+  // the sweep's state by slot (AdjArgs): read at the start, written at the end
+  double *Pu = nullptr, *Pv = nullptr, *C8[8] = {}, *LS[12] = {};
+  double *gs = nullptr, *gC = nullptr, *gx = nullptr, *gy = nullptr;
+  // velocities: subcycle k of the launch's nsub, reversed from nsub - 1 down,
+  // took entry k to entry k + 1; entries `step` doubles apart
+  const double *tu = nullptr, *tv = nullptr;
+  size_t step = 0;
+  int nsub = 0;
+  double4 *mail = nullptr;
+  unsigned seq = 0;
+  int *err = nullptr;
+};
+constexpr int kResAdjointMax = 512;
+int resident_adjoint_prepare(int device, int cls, int nblocks);
+cudaError_t launch_resident_adjoint(const ResidentAdjArgs &a, const Params &p, int cls,
+                                    int threads, int nblocks, cudaStream_t st);
+
 // ---- layout conversion between the reference 1D order and slots ----------
 constexpr int kMaxBatch = 32;
 struct PermBatch {

@@ -40,14 +40,13 @@
 
 #include "evp_kernels.cuh"
 #include "evp_resident.h"
+#include "evp_resident_mail.cuh"
 
 namespace evp {
 
 namespace {
 
 constexpr int kResGeo = 10;  // dxT dyT cxp cyp cxm cym DminTarea dxhy dyhx strength
-constexpr unsigned long long kResWaitNs = 2000000000ull;  // 2 s
-constexpr int kResCode = 15;
 
 template <int NT, bool kSmemStress>
 struct ResSmem {
@@ -57,53 +56,6 @@ struct ResSmem {
   double cst[kTmaStepuFields][NT];
   double s[kSmemStress ? 12 : 1][kSmemStress ? NT : 1];
 };
-
-__device__ __forceinline__ void mail_put(double4 *box, double u, double v, unsigned seq) {
-  const unsigned long long a = (unsigned long long)__double_as_longlong(u);
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const unsigned long long n = (unsigned long long)seq << 32;
-  const unsigned long long m = 0xffffffffull;
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(box), "l"((a & m) | n),
-               "l"((a >> 32) | n)
-               : "memory");
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0+16], {%1, %2};" ::"l"(box), "l"((b & m) | n),
-               "l"((b >> 32) | n)
-               : "memory");
-}
-
-struct Mail {
-  unsigned long long a0, a1, b0, b1;
-};
-
-__device__ __forceinline__ Mail mail_get(const double4 *box) {
-  Mail w;
-  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
-               : "=l"(w.a0), "=l"(w.a1)
-               : "l"(box)
-               : "memory");
-  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2+16];"
-               : "=l"(w.b0), "=l"(w.b1)
-               : "l"(box)
-               : "memory");
-  return w;
-}
-
-__device__ __forceinline__ bool mail_is(const Mail &w, unsigned seq) {
-  return (unsigned)(w.a0 >> 32) == seq && (unsigned)(w.a1 >> 32) == seq &&
-         (unsigned)(w.b0 >> 32) == seq && (unsigned)(w.b1 >> 32) == seq;
-}
-
-__device__ __forceinline__ double2 mail_value(const Mail &w) {
-  const unsigned long long m = 0xffffffffull;
-  return make_double2(__longlong_as_double((long long)((w.a0 & m) | (w.a1 << 32))),
-                      __longlong_as_double((long long)((w.b0 & m) | (w.b1 << 32))));
-}
-
-__device__ __forceinline__ unsigned long long res_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 
 // Keeps the compiler from moving shared-memory accesses across: the lean
 // stress below is written so that few values are live at once.
@@ -288,33 +240,10 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResidentArgs a, Params p) {
     // ---- stress ------------------------------------------------------------
     if (actT) {
       double2 w[4];
-      // Velocities other blocks own: the corners are polled together, so that a
-      // round of reads costs one trip to L2; the words stay as they came until
-      // every corner has its own (fewer registers than the values beside them).
-      Mail m[4];
-      if (sub > 0 && polled) {
-        const unsigned seq = a.seq + (unsigned)sub;
-        const double4 *box = a.mail + (size_t)(sub & 1) * (size_t)a.nslots;
-        unsigned left = polled;
-        unsigned long long t0 = 0;
-        for (unsigned tries = 1;; tries++) {
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            if (left >> k & 1) m[k] = mail_get(box + ~ref[k]);
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            if ((left >> k & 1) && mail_is(m[k], seq)) left &= ~(1u << k);
-          if (!left) break;
-          if ((tries & 63u) == 0) {
-            const unsigned long long t = res_ns();
-            if (t0 == 0) t0 = t;
-            if (t - t0 > kResWaitNs) {
-              fail = true;
-              break;
-            }
-          }
-        }
-      }
+      Mail m[4];  // velocities other blocks own
+      if (sub > 0 && polled)
+        fail |= !mail_wait(m, a.mail + (size_t)(sub & 1) * (size_t)a.nslots, ref, polled,
+                           a.seq + (unsigned)sub);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         if (ref[k] >= 0)

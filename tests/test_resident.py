@@ -117,3 +117,35 @@ def test_same_as_one_launch_per_subcycle(monkeypatch, n):
     for k in ("stress", "uvel", "vvel", "strintx", "strinty", "Cb", "str"):
         a, b = (np.asarray(getattr(f, k)).view(np.int64) for f in got)
         assert np.array_equal(a, b), k
+
+
+# widths 128, 256, 384, 512 of the reverse kernel; segments of 1, 2 and more subcycles
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,ndte,interval", [(3, 2, 3, 0), (64, 48, 11, 0), (64, 48, 11, 5),
+                                                 (64, 48, 7, 1), (203, 151, 6, 4), (330, 250, 4, 0),
+                                                 (370, 280, 4, 3)])
+def test_reverse_launch_bitwise(monkeypatch, nx, ny, ndte, interval):
+    """The reverse sweep in one launch against its two kernels per subcycle:
+    the same gradients bit for bit (both add products by the same explicit
+    fused multiply-adds), with stress seeds, twice on one recording."""
+    g = synth.make_grid(nx, ny, seed=17, ndte=ndte, curvilinear=True)
+    rng = np.random.default_rng(8)
+    g.f["Tbu"] = np.asfortranarray(rng.uniform(0.0, 5.0, g.f["Tbu"].shape) *
+                                   (rng.random(g.f["Tbu"].shape) < 0.3))
+    pr = synth.to_1d(g)
+    lu, lv = rng.normal(size=pr.na), rng.normal(size=pr.na)
+    ls = rng.normal(size=(12, pr.na)) * 1e-6
+    got = []
+    for resident in ("1", "0"):
+        monkeypatch.setenv("EVP1D_RESIDENT", resident)
+        with evp1d.EVP1D.from_problem(pr, ndte=ndte) as s:
+            s.run_checkpointed(ndte, evp1d.FieldSet.from_problem(pr), interval)
+            first = s.adjoint(lu, lv, ls, stress=True)
+            again = s.adjoint(lu, lv, ls, stress=True)
+            launches = s.adjoint_info()["sweep_launches"]
+        for k in first:
+            assert np.array_equal(first[k].view(np.int64), again[k].view(np.int64)), k
+        got.append(first)
+    assert launches > 2 * ndte  # the second handle ran the two kernels
+    for k in got[0]:
+        assert np.array_equal(got[0][k].view(np.int64), got[1][k].view(np.int64)), k

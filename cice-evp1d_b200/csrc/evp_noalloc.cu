@@ -3,9 +3,11 @@
 // device memory (a host code whose device memory is owned by another runtime
 // or memory pool, or that runs where a cudaMalloc would synchronise or fail).
 //
-// It runs the reference-order pair of grid-stride kernels (stress then stepu,
-// src/bench_v2b.F90:62-312, 444-549; the loop of
-// integration/ice_dyn_evp1d.F90:188-207) in place on the caller's arrays.
+// It runs the reference-order stress and stepu (src/bench_v2b.F90:62-312,
+// 444-549; the loop of integration/ice_dyn_evp1d.F90:188-207) in place on the
+// caller's arrays: all subcycles in one cooperative launch with a barrier over
+// the grid after each phase (k_na_run), or, where the device cannot hold that
+// launch, as a pair of grid-stride kernels per subcycle.
 // The only scratch -- str1..str8 and the velocities at call start -- lives in
 // one file-scope device array of fixed size, so the call allocates nothing.
 #include <cstdint>
@@ -28,7 +30,8 @@ constexpr int kStatusNone = 0x7f7f7f7f;
 
 static __device__ __align__(256) double g_scratch[kScratchArrays * (size_t)kNoAllocMaxNavel];
 // Index-check result of the current call (0 = every neighbour in range).
-static __device__ __align__(256) int g_status[1];
+// [1]: a grid barrier of k_na_run ran out; [2]: its arrivals (zeroed per call).
+static __device__ __align__(256) int g_status[3];
 
 struct NaArgs {
   int na, navel;
@@ -124,6 +127,260 @@ __global__ void __launch_bounds__(kThreads) k_na_stepu(NaArgs a, Params p) {
     a.u[w] = o.u;
     a.v[w] = o.v;
   }
+}
+
+// ---- all subcycles in one launch -------------------------------------------
+constexpr int kRunThreads = 512;  // 16 warps an SM at 128 registers
+constexpr unsigned long long kRunWaitNs = 2000000000ull;  // 2 s
+
+// Constants of the block's points, one per thread.
+struct NaSmem {
+  double geo[10][kRunThreads];  // dxT dyT cxp cyp cxm cym DminTarea dxhy dyhx strength
+  double cst[13][kRunThreads];  // the stepu inputs
+};
+
+__device__ __forceinline__ unsigned long long na_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Every block of the (cooperative) grid has reached its barrier number `k`
+// (1, 2, ...) and what its threads wrote before is visible at L2.  Bounded:
+// false, for the whole block, when the wait ran out.
+__device__ __forceinline__ bool grid_barrier(int *status, unsigned k) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned *count = reinterpret_cast<unsigned *>(status) + 2;
+    const unsigned need = k * gridDim.x;
+    __threadfence();
+    atomicAdd(count, 1u);
+    int good = 1;
+    unsigned long long t0 = 0;
+    for (unsigned tries = 1;; tries++) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+      if (v >= need) break;
+      if ((tries & 63u) == 0) {
+        const unsigned long long t = na_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kRunWaitNs) {
+          status[1] = 1;
+          good = 0;
+          break;
+        }
+      }
+    }
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// Velocities and str of other points are read past L1 (__ldcg): other blocks
+// write them during the launch.
+__device__ __forceinline__ Corners na_corners(const NaArgs &a, int w, int iee, int ine, int ise) {
+  Corners c;
+  c.ucc = __ldcg(a.u + w);
+  c.vcc = __ldcg(a.v + w);
+  c.uee = __ldcg(a.u + iee);
+  c.vee = __ldcg(a.v + iee);
+  c.une = __ldcg(a.u + ine);
+  c.vne = __ldcg(a.v + ine);
+  c.use = __ldcg(a.u + ise);
+  c.vse = __ldcg(a.v + ise);
+  return c;
+}
+
+// kOne: one point per thread, whose stresses stay in registers and whose
+// constants stay in shared memory for the whole call; otherwise every phase
+// walks the points with a grid stride and reads them from L2.
+template <bool kOne>
+__global__ void __launch_bounds__(kRunThreads, 1)
+k_na_run(NaArgs a, Params p, int ndte, int *status) {
+  extern __shared__ __align__(16) unsigned char na_raw[];
+  NaSmem &S = *reinterpret_cast<NaSmem *>(na_raw);
+  const int c = threadIdx.x;
+  const int w0 = blockIdx.x * kRunThreads + c;
+  unsigned bar = 0;
+  if (kOne) {
+    const bool have = w0 < a.na;
+    const int w = have ? w0 : 0;
+    const bool actT = have && !a.skipT[w], actU = have && !a.skipU[w];
+    const int iee = a.ee[w] - 1, ine = a.ne[w] - 1, ise = a.se[w] - 1;
+    const int inw = a.nw[w] - 1, isw = a.sw[w] - 1, isse = a.sse[w] - 1;
+    double st[12];
+    double own1 = 0.0, own5 = 0.0;  // str1, str5 of the point
+#pragma unroll
+    for (int k = 0; k < 12; k++) st[k] = a.stress[k][w];
+    {
+      const Geom g = make_geom(a.dxT[w], a.dyT[w], a.HTE[w], a.HTN[w], a.HTEm1[w], a.HTNm1[w],
+                               p.deltaminEVP);
+      const double gg[10] = {g.dxT, g.dyT, g.cxp, g.cyp, g.cxm, g.cym,
+                             g.DminTarea, g.dxhy, g.dyhx, a.strength[w]};
+#pragma unroll
+      for (int k = 0; k < 10; k++) S.geo[k][c] = gg[k];
+      const double cc[13] = {drag_factor(a.aiu[w], p.rhow, a.Cw[w]),
+                             a.uocn[w], a.vocn[w], a.waterx[w], a.watery[w],
+                             a.forcex[w], a.forcey[w], a.umassdti[w], a.fm[w],
+                             a.uarear[w], a.Tbu[w], a.uinit[w], a.vinit[w]};
+#pragma unroll
+      for (int k = 0; k < 13; k++) S.cst[k][c] = cc[k];
+    }
+    for (int n = 0; n < ndte; n++) {
+      const bool last = n == ndte - 1;
+      if (actT) {
+        Geom g;
+        g.dxT = S.geo[0][c];
+        g.dyT = S.geo[1][c];
+        g.cxp = S.geo[2][c];
+        g.cyp = S.geo[3][c];
+        g.cxm = S.geo[4][c];
+        g.cym = S.geo[5][c];
+        g.DminTarea = S.geo[6][c];
+        g.dxhy = S.geo[7][c];
+        g.dyhx = S.geo[8][c];
+        double out[8];
+        stress_point<false>(na_corners(a, w, iee, ine, ise), g, S.geo[9][c], st, out, p);
+        own1 = out[0];
+        own5 = out[4];
+#pragma unroll
+        for (int k = 1; k < 8; k++)
+          if (k != 4) a.str[k][w] = out[k];
+        if (last) {
+          a.str[0][w] = own1;
+          a.str[4][w] = own5;
+        }
+      }
+      if (!grid_barrier(status, ++bar)) return;
+      if (actU) {
+        StepuIn in;
+        in.uold = __ldcg(a.u + w);
+        in.vold = __ldcg(a.v + w);
+        in.s1 = own1;
+        in.s5 = own5;
+        in.s2nw = __ldcg(a.str[1] + inw);
+        in.s7nw = __ldcg(a.str[6] + inw);
+        in.s3sse = __ldcg(a.str[2] + isse);
+        in.s6sse = __ldcg(a.str[5] + isse);
+        in.s4sw = __ldcg(a.str[3] + isw);
+        in.s8sw = __ldcg(a.str[7] + isw);
+        in.kvrel = S.cst[0][c];
+        in.uocn = S.cst[1][c];
+        in.vocn = S.cst[2][c];
+        in.waterx = S.cst[3][c];
+        in.watery = S.cst[4][c];
+        in.forcex = S.cst[5][c];
+        in.forcey = S.cst[6][c];
+        in.umassdti = S.cst[7][c];
+        in.fm = S.cst[8][c];
+        in.uarear = S.cst[9][c];
+        in.Tbu = S.cst[10][c];
+        in.uinit = S.cst[11][c];
+        in.vinit = S.cst[12][c];
+        const StepuOut o = stepu_point(in, p);
+        a.u[w] = o.u;
+        a.v[w] = o.v;
+        if (last) {
+          a.Cb[w] = o.Cb;
+          a.strintx[w] = o.strintx;
+          a.strinty[w] = o.strinty;
+        }
+      }
+      if (!last && !grid_barrier(status, ++bar)) return;
+    }
+    if (actT) {
+#pragma unroll
+      for (int k = 0; k < 12; k++) a.stress[k][w] = st[k];
+    }
+    return;
+  }
+  const int stride = gridDim.x * kRunThreads;
+  for (int n = 0; n < ndte; n++) {
+    const bool last = n == ndte - 1;
+    for (int w = w0; w < a.na; w += stride) {
+      if (a.skipT[w]) continue;
+      const Geom g = make_geom(a.dxT[w], a.dyT[w], a.HTE[w], a.HTN[w], a.HTEm1[w], a.HTNm1[w],
+                               p.deltaminEVP);
+      double st[12], out[8];
+#pragma unroll
+      for (int k = 0; k < 12; k++) st[k] = a.stress[k][w];
+      stress_point<false>(na_corners(a, w, a.ee[w] - 1, a.ne[w] - 1, a.se[w] - 1), g,
+                          a.strength[w], st, out, p);
+#pragma unroll
+      for (int k = 0; k < 12; k++) a.stress[k][w] = st[k];
+#pragma unroll
+      for (int k = 0; k < 8; k++) a.str[k][w] = out[k];
+    }
+    if (!grid_barrier(status, ++bar)) return;
+    for (int w = w0; w < a.na; w += stride) {
+      if (a.skipU[w]) continue;
+      const int inw = a.nw[w] - 1, isw = a.sw[w] - 1, isse = a.sse[w] - 1;
+      StepuIn in;
+      in.uold = __ldcg(a.u + w);
+      in.vold = __ldcg(a.v + w);
+      in.s1 = __ldcg(a.str[0] + w);
+      in.s5 = __ldcg(a.str[4] + w);
+      in.s2nw = __ldcg(a.str[1] + inw);
+      in.s7nw = __ldcg(a.str[6] + inw);
+      in.s3sse = __ldcg(a.str[2] + isse);
+      in.s6sse = __ldcg(a.str[5] + isse);
+      in.s4sw = __ldcg(a.str[3] + isw);
+      in.s8sw = __ldcg(a.str[7] + isw);
+      in.kvrel = drag_factor(a.aiu[w], p.rhow, a.Cw[w]);
+      in.uocn = a.uocn[w];
+      in.vocn = a.vocn[w];
+      in.waterx = a.waterx[w];
+      in.watery = a.watery[w];
+      in.forcex = a.forcex[w];
+      in.forcey = a.forcey[w];
+      in.umassdti = a.umassdti[w];
+      in.fm = a.fm[w];
+      in.uarear = a.uarear[w];
+      in.Tbu = a.Tbu[w];
+      in.uinit = a.uinit[w];
+      in.vinit = a.vinit[w];
+      const StepuOut o = stepu_point(in, p);
+      a.u[w] = o.u;
+      a.v[w] = o.v;
+      if (last) {
+        a.Cb[w] = o.Cb;
+        a.strintx[w] = o.strintx;
+        a.strinty[w] = o.strinty;
+      }
+    }
+    if (!last && !grid_barrier(status, ++bar)) return;
+  }
+}
+
+// One launch for all subcycles; false where the device cannot hold it (or a
+// launch is refused: less of the device is free to this context).
+bool launch_na_run(const NaArgs &given, const Params &given_p, int ndte, int *status, int dev,
+                   cudaStream_t st) {
+  int sms = 0, coop = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) {
+    cudaGetLastError();
+    return false;
+  }
+  // One point per thread up to 512 a SM.  uvel_init given as uvel itself follows
+  // it from subcycle to subcycle, so it cannot be kept.
+  const int blocks = (given.na + kRunThreads - 1) / kRunThreads;
+  const bool one = blocks <= sms && given.uinit != given.u && given.vinit != given.v;
+  const void *k = one ? (const void *)k_na_run<true> : (const void *)k_na_run<false>;
+  const size_t smem = one ? sizeof(NaSmem) : 0;
+  NaArgs a = given;
+  Params p = given_p;
+  void *args[] = {&a, &p, &ndte, &status};
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess ||
+      cudaLaunchCooperativeKernel(k, dim3(one ? blocks : (blocks < sms ? blocks : sms)), dim3(kRunThreads), args, smem,
+                                  st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
 }
 
 #define NA_TRY(x)                                                          \
@@ -294,6 +551,7 @@ extern "C" int evp1d_run_device_noalloc(int na, int navel, const int32_t *ee,
   // neighbour check before any state is touched
   int host_status = kStatusNone;
   NA_TRY(cudaMemsetAsync(status, 0x7f, sizeof(int), st));
+  NA_TRY(cudaMemsetAsync(status + 1, 0, 2 * sizeof(int), st));
   k_na_check<<<grid_for(na), kThreads, 0, st>>>(a, status);
   NA_TRY(cudaGetLastError());
   NA_TRY(cudaMemcpyAsync(&host_status, status, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -309,7 +567,8 @@ extern "C" int evp1d_run_device_noalloc(int na, int navel, const int32_t *ee,
     NA_TRY(cudaMemsetAsync(a.str[k], 0, sizeof(double) * navel, st));
   const int grid = grid_for(na);
   const Params p = kernel_params(*params);
-  for (int s = 0; s < ndte; s++) {
+  const bool run = launch_na_run(a, p, ndte, status, dev, st);
+  for (int s = 0; s < ndte && !run; s++) {
     k_na_stress<<<grid, kThreads, 0, st>>>(a, p);
     k_na_stepu<<<grid, kThreads, 0, st>>>(a, p);
   }
@@ -318,6 +577,12 @@ extern "C" int evp1d_run_device_noalloc(int na, int navel, const int32_t *ee,
     if (io->str[k])
       NA_TRY(cudaMemcpyAsync(io->str[k], a.str[k], sizeof(double) * navel,
                              cudaMemcpyDeviceToDevice, st));
+  int ran_out = 0;
+  if (run)
+    NA_TRY(cudaMemcpyAsync(&ran_out, status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
   NA_TRY(cudaStreamSynchronize(st));
+  if (ran_out)
+    return error(EVP1D_ERR_TIMEOUT, "a bounded device-side wait ran out (a barrier over the "
+                 "grid); the results of this call are not valid");
   return EVP1D_OK;
 }

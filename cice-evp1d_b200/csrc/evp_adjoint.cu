@@ -777,17 +777,12 @@ int evp1d_adjoint_seed(evp1d_t *h, const double *lam_uvel, const double *lam_vve
   };
   ADJ_CHECK(add(lam_uvel, A.Pu));
   ADJ_CHECK(add(lam_vvel, A.Pv));
-  for (int k = 0; k < 12; k++) {
-    if (lam_stress && lam_stress[k])
-      ADJ_CHECK(add(lam_stress[k], A.LS[k]));
-    else
-      ADJ_TRY(cudaMemsetAsync(A.LS[k], 0, sizeof(double) * d.nslots, st));
-  }
+  for (int k = 0; k < 12; k++)
+    if (lam_stress && lam_stress[k]) ADJ_CHECK(add(lam_stress[k], A.LS[k]));
+  // the shares, stress adjoints and gradients lie together (ensure_static)
+  ADJ_TRY(cudaMemsetAsync(A.C8[0], 0, sizeof(double) * (size_t)(A.g[kNumGrad - 1] + d.nslots - A.C8[0]),
+                          st));
   launch_scatter(b, d.nslots, d.point_of_slot, st);
-  for (int k = 0; k < 8; k++)
-    ADJ_TRY(cudaMemsetAsync(A.C8[k], 0, sizeof(double) * d.nslots, st));
-  for (int k = 0; k < kNumGrad; k++)
-    ADJ_TRY(cudaMemsetAsync(A.g[k], 0, sizeof(double) * d.nslots, st));
   ADJ_TRY(cudaGetLastError());
   A.seeded = true;
   return EVP1D_OK;
@@ -952,7 +947,6 @@ int evp1d_adjoint_gradients(evp1d_t *h, const evp1d_grads *g) {
     return error(EVP1D_ERR_TIMEOUT,
                  "a bounded device-side wait ran out (code %d: %s); the gradients are not valid",
                  code, tma_wait_name(code));
-  const size_t nv = (size_t)(d.navel > 0 ? d.navel : 1);
   const size_t bn = sizeof(double) * (size_t)d.na;
   struct Out {
     const double *src;
@@ -976,20 +970,13 @@ int evp1d_adjoint_gradients(evp1d_t *h, const evp1d_grads *g) {
     if (g->uvel_init) memset(g->uvel_init, 0, bn);
     if (g->vvel_init) memset(g->vvel_init, 0, bn);
   }
-  for (size_t o = 0; o < outs.size(); o += kMaxBatch) {
-    PermBatch b;
-    for (size_t q = o; q < outs.size() && b.n < kMaxBatch; q++) {
-      b.src[b.n] = outs[q].src;
-      b.dst[b.n] = d.stage + (size_t)b.n * nv;
-      b.n++;
-    }
-    launch_gather(b, d.na, d.slot_of_point, st);
-    for (int q = 0; q < b.n; q++)
-      ADJ_TRY(cudaMemcpyAsync(outs[o + q].host, b.dst[q], bn, cudaMemcpyDeviceToHost, st));
-    ADJ_TRY(cudaStreamSynchronize(st));
+  std::vector<const double *> src;
+  std::vector<double *> host;
+  for (const Out &o : outs) {
+    src.push_back(o.src);
+    host.push_back(o.host);
   }
-  ADJ_TRY(cudaGetLastError());
-  return EVP1D_OK;
+  return problem_gather_to_host(&d, (int)outs.size(), src.data(), host.data());
 }
 
 int evp1d_adjoint(evp1d_t *h, const double *lam_uvel, const double *lam_vvel,

@@ -135,6 +135,10 @@ struct DownloadFields {
   double *stage = nullptr;
   size_t stage_step = 0;
 };
+// n slot-ordered arrays to the caller's host arrays (na points each, reference
+// order); waits for the stream.
+int problem_gather_to_host(DeviceProblem *d, int n, const double *const *src,
+                           double *const *host);
 // Page-locked memory shared by the handles of the process, allocated on first
 // use (a page-locking call takes 2.5 ms, however small) and freed with the
 // last handle: a page of words, one per handle, and one staging buffer of

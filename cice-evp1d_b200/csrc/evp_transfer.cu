@@ -6,15 +6,18 @@
 // once, in the caller's order: k_upload takes a point's 29 values, skip flags
 // included, and writes every place they go to (both state sets, the
 // slot-ordered inputs, the constant blocks); k_download gathers the results.
-// Other arrays pass through page-locked staging of the handle when they are
-// small (one copy by the host, then the same kernels), else through device
-// staging with cudaMemcpyAsync.
+// Other arrays pass through page-locked staging: a small call's by one copy by
+// the host and the same kernels; a large call's in chunks that several host
+// threads copy while the copy engine moves others to or from device staging.
 //
 // What bounds it: the host link for large calls; for small ones it was the
 // number of copies (31 up, 17 down, about 2 us each, and a dozen kernels
 // and fills): 2.0k points took 190 us up and 90 us down.
+#include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
+#include <thread>
 #include <vector>
 
 #include "evp_internal.h"
@@ -32,10 +35,17 @@ namespace {
                    "%s: %s", #x, cudaGetErrorString(e_));                  \
   } while (0)
 
-// Staged bytes of one call up to which they go through page-locked staging
-// (the host copies them at about 10 GB/s, one array after another); above,
-// cudaMemcpyAsync's own pipelining of pageable memory wins.
-constexpr size_t kPinnedStage = 8u << 20;
+// The page-locked staging buffer, and the staged bytes of one call up to which
+// the kernels go to it: one host thread fills it at about 10 GB/s, which
+// overlaps with nothing; larger calls take chunks of it in turn.
+constexpr size_t kPinnedStage = 8u << 20, kStagedDirect = 3u << 20;
+static_assert(kStagedDirect <= kPinnedStage, "one call's staging");
+// Host threads of a chunked copy: one per kThreadBytes, up to kMaxThreads (a
+// thread takes 30 us to start and copies about 10 GB/s; 42 MB into fresh pages
+// took 3.0, 2.5, 1.4 and 0.9 ms on 1, 2, 4 and 8 threads, and 5.9 through
+// cudaMemcpyAsync's own staging).
+constexpr size_t kThreadBytes = 2u << 20;
+constexpr int kMaxThreads = 8;
 
 // Bytes of one call up to which the kernels go to addressable host arrays
 // themselves.  They move about 40 GB/s over the host link where
@@ -263,9 +273,16 @@ void pinned_release(DeviceProblem *d) {
   p.words = nullptr;
 }
 
-bool device_view(const void *p, size_t bytes, size_t align, void **dev) {
+namespace {
+
+// Whose memory a caller's array is: the host's own (pageable, or not wholly
+// registered), the GPU's to address as well, or a device's alone, which no host
+// code may touch (cudaMemcpyAsync copies it).
+enum HostKind { kPageable, kAddressable, kDeviceOnly };
+
+HostKind host_kind(const void *p, size_t bytes, size_t align, void **dev) {
   PtrAttrs query = ptr_attrs();
-  if (!query || !p || bytes == 0) return false;
+  if (!query || !p || bytes == 0) return kPageable;
   // CUpointer_attribute: MEMORY_TYPE 2, DEVICE_POINTER 3, IS_MANAGED 8,
   // RANGE_START_ADDR 11, RANGE_SIZE 12
   int what[5] = {2, 3, 8, 11, 12};
@@ -274,17 +291,136 @@ bool device_view(const void *p, size_t bytes, size_t align, void **dev) {
   size_t size = 0;
   void *out[5] = {&type, &dptr, &managed, &start, &size};
   const unsigned long long at = (unsigned long long)(uintptr_t)p;
-  if (query(5, what, out, at) != 0) return false;
-  constexpr unsigned kHost = 1;  // CU_MEMORYTYPE_HOST
-  if (!(type == kHost || managed) || dptr == 0 || start == 0) return false;
+  if (query(5, what, out, at) != 0) return kPageable;
+  constexpr unsigned kHost = 1, kDevice = 2, kArray = 3;  // CUmemorytype
+  if ((type == kDevice || type == kArray) && !managed) return kDeviceOnly;
+  if (!(type == kHost || managed) || dptr == 0 || start == 0) return kPageable;
   // the range query gives the allocation in the address space it is asked in
   // (host addresses of page-locked memory equal its device addresses); an
   // array that only begins in registered memory is not addressable
   const unsigned long long base = at >= start && at < start + size ? at : dptr;
-  if (base < start || bytes > size || base - start > size - bytes) return false;
-  if (dptr % align) return false;
+  if (base < start || bytes > size || base - start > size - bytes) return kPageable;
+  if (dptr % align) return kPageable;
   *dev = reinterpret_cast<void *>((uintptr_t)dptr);
-  return true;
+  return kAddressable;
+}
+
+// One array between host memory and device staging.
+struct CopyItem {
+  char *host, *dev;
+  size_t bytes;
+  HostKind kind;
+};
+
+// Pageable items through `stage` (kPinnedStage bytes) in chunks, each host
+// thread with two halves of its own share of it.  Up: the copies are queued on
+// the stream, and complete, on return; down: the results are in host memory.
+cudaError_t copy_chunked(const std::vector<CopyItem> &items, bool up, char *stage, int device,
+                         cudaStream_t st) {
+  size_t total = 0;
+  for (const CopyItem &it : items) total += it.bytes;
+  const unsigned hw = std::thread::hardware_concurrency();
+  int nt = (int)std::min<size_t>(kMaxThreads, total / kThreadBytes);
+  if (hw > 0 && nt > (int)hw) nt = (int)hw;
+  if (nt < 1) nt = 1;
+  const size_t half = (kPinnedStage / nt / 2) & ~size_t(4095);
+  std::vector<CopyItem> chunks;
+  for (const CopyItem &it : items)
+    for (size_t o = 0; o < it.bytes; o += half)
+      chunks.push_back({it.host + o, it.dev + o, std::min(half, it.bytes - o), it.kind});
+  std::atomic<size_t> next{0};
+  std::atomic<int> failed{(int)cudaSuccess};
+  auto work = [&](int w) {
+    auto check = [&](cudaError_t e) {
+      int none = (int)cudaSuccess;
+      if (e != cudaSuccess) failed.compare_exchange_strong(none, (int)e);
+      return e == cudaSuccess;
+    };
+    char *buf[2] = {stage + (size_t)w * 2 * half, stage + ((size_t)w * 2 + 1) * half};
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    const CopyItem *busy[2] = {nullptr, nullptr};
+    bool ok = check(cudaSetDevice(device)) &&
+              check(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming)) &&
+              check(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
+    // the copy queued on half b has ended; down: its chunk goes to the caller
+    auto drain = [&](int b) {
+      if (!busy[b]) return true;
+      const CopyItem *c = busy[b];
+      busy[b] = nullptr;
+      if (!check(cudaEventSynchronize(ev[b]))) return false;
+      if (!up) memcpy(c->host, buf[b], c->bytes);
+      return true;
+    };
+    int b = 0;
+    while (ok && failed.load() == (int)cudaSuccess) {
+      const size_t k = next.fetch_add(1);
+      if (k >= chunks.size()) break;
+      const CopyItem &c = chunks[k];
+      ok = drain(b);
+      if (!ok) break;
+      if (up) memcpy(buf[b], c.host, c.bytes);
+      ok = check(up ? cudaMemcpyAsync(c.dev, buf[b], c.bytes, cudaMemcpyHostToDevice, st)
+                    : cudaMemcpyAsync(buf[b], c.dev, c.bytes, cudaMemcpyDeviceToHost, st)) &&
+           check(cudaEventRecord(ev[b], st));
+      if (!ok) break;
+      busy[b] = &c;
+      b ^= 1;
+    }
+    if (ok) ok = drain(b) && drain(b ^ 1);
+    if (!ok) cudaStreamSynchronize(st);  // nothing may still be reading the halves
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+  };
+  std::vector<std::thread> threads;
+  try {
+    threads.reserve((size_t)nt);
+    for (int w = 1; w < nt; w++) threads.emplace_back(work, w);
+  } catch (...) {
+    // fewer threads than wanted: the chunks are taken by those there are
+  }
+  work(0);
+  for (std::thread &t : threads) t.join();
+  return (cudaError_t)failed.load();
+}
+
+// Every item: pageable ones in chunks where the staging buffer is free and
+// they are large, the others by the copy engine's own call.  Up: queued on
+// return, and pageable memory is no longer read; down: queued (pageable:
+// complete).
+cudaError_t copy_items(const std::vector<CopyItem> &items, bool up, int device, cudaStream_t st) {
+  std::vector<CopyItem> own;
+  size_t total = 0;
+  for (const CopyItem &it : items) {
+    if (it.kind == kPageable) {
+      own.push_back(it);
+      total += it.bytes;
+      continue;
+    }
+    const cudaError_t e =
+        up ? cudaMemcpyAsync(it.dev, it.host, it.bytes, cudaMemcpyHostToDevice, st)
+           : cudaMemcpyAsync(it.host, it.dev, it.bytes, cudaMemcpyDeviceToHost, st);
+    if (e != cudaSuccess) return e;
+  }
+  if (own.empty()) return cudaSuccess;
+  char *stage = total >= kThreadBytes ? static_cast<char *>(borrow_stage()) : nullptr;
+  if (stage) {
+    const cudaError_t e = copy_chunked(own, up, stage, device, st);
+    return_stage();
+    return e;
+  }
+  for (const CopyItem &it : own) {
+    const cudaError_t e =
+        up ? cudaMemcpyAsync(it.dev, it.host, it.bytes, cudaMemcpyHostToDevice, st)
+           : cudaMemcpyAsync(it.host, it.dev, it.bytes, cudaMemcpyDeviceToHost, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace
+
+bool device_view(const void *p, size_t bytes, size_t align, void **dev) {
+  return host_kind(p, bytes, align, dev) == kAddressable;
 }
 
 namespace {
@@ -303,23 +439,27 @@ struct Placer {
     void *stage;  // device staging of the array
     size_t bytes;
     void **dev;   // the pointer the kernels get
+    HostKind kind;
     size_t off = 0;
   };
   std::vector<Item> staged, direct;
   size_t total = 0, direct_total = 0;
   bool pinned = false;
+  bool foreign = false;  // a device's own memory among the arrays
 
   // dev: device address for the kernels, at once where the GPU can address the
   // array, else set by place().  `fixed`: an array its map makes direct.
   void add(const void *host, size_t bytes, size_t align, void *stage, void **dev,
            bool fixed = false) {
-    if (device_view(host, bytes, align, dev)) {
+    const HostKind kind = host_kind(host, bytes, align, dev);
+    if (kind == kAddressable) {
       if (!fixed) {
-        direct.push_back({host, stage, bytes, dev});
+        direct.push_back({host, stage, bytes, dev, kind});
         direct_total += bytes;
       }
     } else {
-      stage_it({host, stage, bytes, dev});
+      foreign = foreign || kind == kDeviceOnly;
+      stage_it({host, stage, bytes, dev, kind});
     }
   }
   void stage_it(Item it) {
@@ -335,11 +475,17 @@ struct Placer {
       for (const Item &it : direct) stage_it(it);
       return;
     }
-    if (staged.empty() || total > kPinnedStage) return;
+    if (staged.empty() || foreign || total > kStagedDirect) return;
     char *base = static_cast<char *>(borrow_stage());
     if (!base) return;
     pinned = true;
     for (Item &it : staged) *it.dev = base + it.off;
+  }
+  std::vector<CopyItem> copies() const {
+    std::vector<CopyItem> c;
+    for (const Item &it : staged)
+      c.push_back({(char *)it.host, (char *)it.stage, it.bytes, it.kind});
+    return c;
   }
 };
 
@@ -384,12 +530,10 @@ int problem_upload(DeviceProblem *d, const UploadFields &f, double rhow, bool wa
   // (2D arrays: the device staging keeps the cells outside the list for the
   // way back)
   if (!f.map_f) P.place();
-  for (const Placer::Item &it : P.staged) {
-    if (P.pinned)
-      memcpy(*it.dev, it.host, it.bytes);
-    else
-      CUDA_TRY(cudaMemcpyAsync(it.stage, it.host, it.bytes, cudaMemcpyHostToDevice, st));
-  }
+  if (P.pinned)
+    for (const Placer::Item &it : P.staged) memcpy(*it.dev, it.host, it.bytes);
+  else
+    CUDA_TRY(copy_items(P.copies(), true, d->device, st));
   for (int k = 0; k < kNumDyn; k++) a.dyn[k] = d->dyn[k];
   for (int k = 0; k < 12; k++) {
     a.s0[k] = d->stress[0][k];
@@ -459,14 +603,39 @@ int problem_download(DeviceProblem *d, const DownloadFields &f, int *code) {
   }
   k_download<<<(d->navel + kThreads - 1) / kThreads, kThreads, 0, st>>>(a);
   CUDA_TRY(cudaGetLastError());
-  if (!P.pinned)
-    for (const Placer::Item &it : P.staged)
-      CUDA_TRY(cudaMemcpyAsync(const_cast<void *>(it.host), it.stage, it.bytes,
-                               cudaMemcpyDeviceToHost, st));
+  if (!P.pinned) CUDA_TRY(copy_items(P.copies(), false, d->device, st));
   const int rc = problem_take_error(d, code);  // waits for the stream
   if (rc != EVP1D_OK || *code) return rc;
   if (P.pinned)
     for (const Placer::Item &it : P.staged) memcpy(const_cast<void *>(it.host), *it.dev, it.bytes);
+  return EVP1D_OK;
+}
+
+int problem_gather_to_host(DeviceProblem *d, int n, const double *const *src,
+                           double *const *host) {
+  const size_t bytes = (size_t)d->na * sizeof(double);
+  cudaStream_t st = d->stream;
+  for (int at = 0; at < n; at += kMaxBatch) {
+    const int m = std::min(kMaxBatch, n - at);
+    Placer P(kDirectDown);
+    PermBatch b;
+    b.n = m;
+    void *to[kMaxBatch];
+    for (int k = 0; k < m; k++) {
+      b.src[k] = src[at + k];
+      P.add(host[at + k], bytes, sizeof(double),
+            d->stage + (size_t)k * (size_t)(d->navel > 0 ? d->navel : 1), &to[k]);
+    }
+    P.place();
+    for (int k = 0; k < m; k++) b.dst[k] = static_cast<double *>(to[k]);
+    launch_gather(b, d->na, d->slot_of_point, st);
+    CUDA_TRY(cudaGetLastError());
+    if (!P.pinned) CUDA_TRY(copy_items(P.copies(), false, d->device, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    if (P.pinned)
+      for (const Placer::Item &it : P.staged)
+        memcpy(const_cast<void *>(it.host), *it.dev, it.bytes);
+  }
   return EVP1D_OK;
 }
 

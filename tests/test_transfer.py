@@ -103,3 +103,84 @@ def test_batched_positions(pinned):
             s.run(3, one)
         assert np.array_equal(u[m].view(np.int64), one.uvel.view(np.int64))
         assert np.array_equal(np.ascontiguousarray(st[m]).view(np.int64), one.str.view(np.int64))
+
+
+@pytest.mark.parametrize("nx,ny", [(97, 61), (330, 250), (640, 480)])
+def test_gradients_into_any_memory(nx, ny):
+    """Gradients gathered by the kernel (page-locked), through page-locked
+    staging and in chunks by several host threads: the same bits."""
+    from evp1d import _lib
+    pr = problem(nx, ny)
+    rng = np.random.default_rng(4)
+    lu, lv = rng.normal(size=pr.na), rng.normal(size=pr.na)
+    names = ("strength", "Cw", "forcex", "forcey", "uvel", "vvel")
+    with evp1d.EVP1D.from_problem(pr, ndte=3) as s:
+        s.run_checkpointed(3, evp1d.FieldSet.from_problem(pr), 0)
+        want = s.adjoint(lu, lv, stress=True)
+        g = _lib.Grads()
+        out = {k: evp1d.pinned_empty(pr.na) for k in names}
+        st = evp1d.pinned_empty((12, pr.na))
+        for k in names:
+            setattr(g, k, out[k].ctypes.data_as(_D))
+        for k in range(12):
+            g.stress[k] = st[k].ctypes.data_as(_D)
+        s.adjoint_seed(lu, lv)
+        s.adjoint_sweep()
+        _lib.check(s._L.evp1d_adjoint_gradients(s.h, C.byref(g)), "gradients")
+    for k in names:
+        assert np.array_equal(out[k].view(np.int64), want[k].view(np.int64)), k
+    assert np.array_equal(np.ascontiguousarray(st).view(np.int64), want["stress"].view(np.int64))
+
+
+def test_pageable_calls_from_two_threads():
+    """Two handles' large pageable calls at once: one has the staging buffer,
+    the other goes without; both give the serial call's bits."""
+    import threading
+    pr = problem(400, 300)
+    ref = evp1d.FieldSet.from_problem(pr, want_str=True)
+    with evp1d.EVP1D.from_problem(pr, ndte=3) as s:
+        s.run(3, ref)
+    sets = [evp1d.FieldSet.from_problem(pr, want_str=True) for _ in range(2)]
+    solvers = [evp1d.EVP1D.from_problem(pr, ndte=3) for _ in range(2)]
+    errors = []
+
+    def call(k):
+        try:
+            for _ in range(3):
+                sets[k].refill(pr)
+                solvers[k].run(3, sets[k])
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+    threads = [threading.Thread(target=call, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for s in solvers:
+        s.finalize()
+    assert not errors
+    for fs in sets:
+        for k in FIELDS:
+            assert np.array_equal(bits(fs)[k], bits(ref)[k]), k
+
+
+def test_device_memory_among_the_arrays():
+    """Device memory in the place of a host array is copied, never touched by
+    host code: the same bits."""
+    import torch
+    pr = problem(97, 61)
+    ref = evp1d.FieldSet.from_problem(pr, want_str=True)
+    fs = evp1d.FieldSet.from_problem(pr, want_str=True)
+    t = {k: torch.from_numpy(fs.dyn[k]).cuda() for k in ("strength", "uocn")}
+    cb = torch.from_numpy(fs.Cb).cuda()
+    for k in t:
+        setattr(fs.c, k, C.cast(C.c_void_p(t[k].data_ptr()), _D))
+    fs.c.Cb = C.cast(C.c_void_p(cb.data_ptr()), _D)
+    torch.cuda.synchronize()
+    with evp1d.EVP1D.from_problem(pr, ndte=3) as s:
+        s.run(3, ref)
+        s.run(3, fs)
+    fs.Cb[:] = cb.cpu().numpy()
+    a, b = bits(ref), bits(fs)
+    for k in FIELDS:
+        assert np.array_equal(a[k], b[k]), k

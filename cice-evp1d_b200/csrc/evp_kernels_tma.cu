@@ -22,7 +22,10 @@
 // the new stresses and velocities to the other ping-pong buffer.  Stepu reads
 // str from the tile's own table and from the previous tile's, which stays
 // alive: three str tables rotate, so that one tile's stress can start while
-// stepu still reads the two before it.  The 13 stepu inputs of a tile (the
+// stepu still reads the two before it (six of the eight str, in pairs read
+// together; str1 and str5 are read by their own point alone and stay in its
+// registers: 26.3 -> 25.9 us a subcycle at 296k points against tables of
+// eight).  The 13 stepu inputs of a tile (the
 // second part of its constant block) arrive by one more bulk copy into a
 // stepu slot, which the consumers release as soon as each has its point's
 // inputs in registers.  Where every Tbu of the call is +0, every uinit and
@@ -79,7 +82,9 @@ struct USlot {
 struct Smem {
   SSlot ss[kSSlots];
   USlot us;
-  double str[3][8][kStrRow];  // rotating str tables; position kZeroSlot holds 0
+  // rotating str tables of what other points read: (str2, str7), (str3, str6),
+  // (str4, str8); position kZeroSlot holds 0
+  double2 str[3][3][kStrRow];
   int32_t rec[kRecRing][kRecInts];
   unsigned long long sfull[kSSlots];
   unsigned long long sempty[kSSlots];
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     S.abort_flag = 0;
     mbar_fence_init();
   }
-  if (tid < 24) S.str[tid >> 3][tid & 7][kZeroSlot] = 0.0;
+  if (tid < 9) S.str[tid / 3][tid % 3][kZeroSlot] = make_double2(0.0, 0.0);
   __syncthreads();
   // A launch of one subcycle may be followed by the next subcycle's, launched
   // as a programmatic dependent (a.pdl there): it can start as soon as every
@@ -648,6 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     uint32_t m = 0;
     uint32_t sg = 0;  // sign bits of uinit (bit 0) and vinit (bit 1)
     double uold = 0.0, vold = 0.0;
+    double s1 = 0.0, s5 = 0.0;  // str1, str5: read by the point itself only
     int off = 0, cnt = 0;
   };
 
@@ -715,8 +721,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
             for (int k = 0; k < 12; k++) a.s[to][k][cy.off + c] = s12[k];
           }
         }
-#pragma unroll
-        for (int k = 0; k < 8; k++) S.str[b][k][c] = out[k];
+        S.str[b][0][c] = make_double2(out[1], out[6]);
+        S.str[b][1][c] = make_double2(out[2], out[5]);
+        S.str[b][2][c] = make_double2(out[3], out[7]);
+        cy.s1 = out[0];
+        cy.s5 = out[4];
         if (wlast && own) {
 #pragma unroll
           for (int k = 0; k < 8; k++) a.str_out[k][cy.off + c] = out[k];
@@ -772,25 +781,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     }
     if (act) {
       const uint32_t m = cy.m;
-      const double(&str)[8][kStrRow] = S.str[b];
       // a neighbour's str: own table, or the previous tile's (kStrPrev)
       const uint32_t vnw = m & kLnbMask, vsw = (m >> kLnbBits) & kLnbMask;
       const uint32_t vsse = (m >> (2 * kLnbBits)) & kLnbMask;
-      const double(&tnw)[8][kStrRow] = (vnw & kStrPrev) ? S.str[bp] : S.str[b];
-      const double(&tsw)[8][kStrRow] = (vsw & kStrPrev) ? S.str[bp] : S.str[b];
-      const double(&tsse)[8][kStrRow] = (vsse & kStrPrev) ? S.str[bp] : S.str[b];
-      const int lnw = vnw & (kStrPrev - 1), lsw = vsw & (kStrPrev - 1);
-      const int lsse = vsse & (kStrPrev - 1);
+      const double2 nw = S.str[(vnw & kStrPrev) ? bp : b][0][vnw & (kStrPrev - 1)];
+      const double2 sse = S.str[(vsse & kStrPrev) ? bp : b][1][vsse & (kStrPrev - 1)];
+      const double2 sw = S.str[(vsw & kStrPrev) ? bp : b][2][vsw & (kStrPrev - 1)];
       in.uold = cy.uold;
       in.vold = cy.vold;
-      in.s1 = str[0][c];
-      in.s2nw = tnw[1][lnw];
-      in.s3sse = tsse[2][lsse];
-      in.s4sw = tsw[3][lsw];
-      in.s5 = str[4][c];
-      in.s6sse = tsse[5][lsse];
-      in.s7nw = tnw[6][lnw];
-      in.s8sw = tsw[7][lsw];
+      in.s1 = cy.s1;
+      in.s5 = cy.s5;
+      in.s2nw = nw.x;
+      in.s7nw = nw.y;
+      in.s3sse = sse.x;
+      in.s6sse = sse.y;
+      in.s4sw = sw.x;
+      in.s8sw = sw.y;
       const StepuOut o = stepu_point(in, p);
       double *u_out = kMulti && a.uv_step ? a.u[0] + (size_t)(sub + 1) * a.uv_step : a.u[to];
       double *v_out = kMulti && a.uv_step ? a.v[0] + (size_t)(sub + 1) * a.uv_step : a.v[to];

@@ -285,14 +285,17 @@ int init_common(evp1d_t **handle, int na, int navel, const int32_t *const idx[6]
   }
 
   // The resident plan, unless a setting of the subcycle kernel asks for that
-  // kernel (EVP1D_RESIDENT=0: never)
+  // kernel (EVP1D_RESIDENT=0: never; 2: one thread per point at every size)
   evp::ResidentPlan res;
-  bool resident = g_tile_points.load() == evp::kTileCompute;
+  bool resident = g_tile_points.load() == evp::kTileCompute, quad = true;
   for (const char *name : {"EVP1D_PATH", "EVP1D_PERSIST", "EVP1D_PDL", "EVP1D_COMPACT", "EVP1D_RUNS",
                            "EVP1D_STRIP_W", "EVP1D_PREFETCH", "EVP1D_TRACE"})
     resident = resident && !getenv(name);
-  if (const char *e = getenv("EVP1D_RESIDENT")) resident = resident && atoi(e) != 0;
-  if (resident && evp::build_resident_plan(na, nbp, plan, sms, &res) &&
+  if (const char *e = getenv("EVP1D_RESIDENT")) {
+    resident = resident && atoi(e) != 0;
+    quad = atoi(e) != 2;
+  }
+  if (resident && evp::build_resident_plan(na, nbp, plan, sms, &res, quad) &&
       getenv("EVP1D_CHECK_PLAN")) {
     std::string first;
     const long long bad = evp::verify_resident_plan(res, na, nbp, plan, &first);

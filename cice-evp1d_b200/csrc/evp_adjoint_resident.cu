@@ -172,13 +172,13 @@ __global__ void __launch_bounds__(NT, 1) k_resident_adj(ResidentAdjArgs a, Param
     }
     __syncthreads();
     // ---- stress reversed -----------------------------------------------------
+    Mail m[4];
+    fail |= !mail_wait(m, box, ref, actT ? polled : 0u, a.seq + (unsigned)it);
     if (actT) {
       double2 w[4];  // velocities of cc, ee, ne, se
 #pragma unroll
       for (int k = 0; k < 4; k++)
         w[k] = ref[k] >= 0 ? S.uv[ref[k]] : make_double2(tu[~ref[k]], tv[~ref[k]]);
-      Mail m[4];
-      if (polled) fail |= !mail_wait(m, box, ref, polled, a.seq + (unsigned)it);
       double2 l[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {

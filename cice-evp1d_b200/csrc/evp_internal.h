@@ -94,6 +94,7 @@ struct DeviceProblem {
   int cur = 0;              // buffer holding the current state
   // resident plan (evp_resident.h), res_blocks == 0: none
   int res_blocks = 0, res_threads = 0, res_cls = 0;
+  bool res_quad = false;
   int32_t *res_slot = nullptr, *res_cnt = nullptr, *res_corner = nullptr;
   uint32_t *res_str = nullptr;
   double4 *res_mail = nullptr;  // 2 x nslots velocity mailboxes

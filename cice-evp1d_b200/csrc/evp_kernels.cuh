@@ -212,10 +212,11 @@ struct ResidentArgs {
   unsigned seq = 0;           // number of the launch's first subcycle
   int *err = nullptr;
 };
-// Enable the variant of width class `cls` and tell whether `nblocks` of its
-// CTAs are resident at once (1) or the plan cannot run here (0).
-int resident_prepare(int device, int cls, int nblocks);
-cudaError_t launch_resident(const ResidentArgs &a, const Params &p, int cls, int threads,
+// Enable the variant of width class `cls` (quad: four lanes per point) and tell
+// whether `nblocks` of its CTAs are resident at once (1) or the plan cannot run
+// here (0).  `threads`: the plan's, compute positions per block.
+int resident_prepare(int device, bool quad, int cls, int nblocks);
+cudaError_t launch_resident(const ResidentArgs &a, const Params &p, bool quad, int cls, int threads,
                             int nblocks, cudaStream_t st);
 
 // The reverse sweep's subcycles in one launch on the same plan

@@ -33,9 +33,9 @@
 // What bounds it: the FP64 pipe (about 535 operations a point, two issue
 // cycles each, 64 lanes an SM) for full blocks, the dependent chain through
 // stress, stepu and the exchange for small ones; no HBM traffic per subcycle.
-// Measured, us per subcycle, against the one-launch-per-subcycle kernel:
-// 2.0k points 3.0 / 4.8, 18k 3.5 / 5.0, 51k 3.6 / 7.8, 64k 4.2 / 8.0,
-// 74k 6.4 / 10.4.
+// Measured, us per subcycle, against the one-launch-per-subcycle kernel (before
+// the straight-line divisions of evp_fp64.cuh): 18k points 2.6 / 5.0, 51k 3.2 /
+// 7.8, 64k 3.9 / 8.0, 74k 6.1 / 10.4; smaller problems: k_resident_quad.
 #include <cstdint>
 
 #include "evp_kernels.cuh"
@@ -238,12 +238,12 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResidentArgs a, Params p) {
   for (int sub = 0; sub < a.nsub; sub++) {
     const bool wlast = a.last && sub == a.nsub - 1;
     // ---- stress ------------------------------------------------------------
+    Mail m[4];  // velocities other blocks own
+    if (sub > 0)
+      fail |= !mail_wait(m, a.mail + (size_t)(sub & 1) * (size_t)a.nslots, ref,
+                         actT ? polled : 0u, a.seq + (unsigned)sub);
     if (actT) {
       double2 w[4];
-      Mail m[4];  // velocities other blocks own
-      if (sub > 0 && polled)
-        fail |= !mail_wait(m, a.mail + (size_t)(sub & 1) * (size_t)a.nslots, ref, polled,
-                           a.seq + (unsigned)sub);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         if (ref[k] >= 0)
@@ -356,6 +356,229 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResidentArgs a, Params p) {
   }
 }
 
+// ---- four lanes per point ---------------------------------------------------
+// Lane k of a point's quad has corner k (0 ne, 1 nw, 2 sw, 3 se): its velocity
+// (cc, ee, ne, se: one mailbox at most to poll), its strain rates, its
+// viscosity and its three stresses.  The sums of str_combine
+// (src/bench_v2b.F90:217-310) are symmetric in the corners: with s the own
+// corner's stress and s1, s2, s3 those of lanes k^1, k^2, k^3,
+//   sides        N = s + s1, N' = s2 + s3 (north/south), E = s + s3,
+//                E' = s1 + s2 (east/west)
+//   csig         P111*s + P055*(s1 + s3) + P027*s2
+//   strp, str12  c * (P333*N + P166*N'), or with E, E'
+// and lane k writes the two str of its corner, str1/5, 2/7, 4/8, 3/6, which
+// differ in signs only.  Addition commutes and negation is exact, so these are
+// the reference's values bit for bit.  stepu runs one thread per point, on the
+// block's first warps.  A lane has 130 of stress's 440 FP64 operations, so a
+// warp's chain is a third as long; all in all 17 % more operations, on SMs that
+// one thread per point leaves four fifths idle.  us per subcycle against one
+// thread per point: 2.0k points 1.65 / 2.55, 6.2k 1.70 / 2.53, 13.6k 1.78 / 2.64
+// (above 128 points a block the lanes fill the SM, and one thread per point is
+// as fast).
+struct QuadSmem {
+  double2 uv[kQuadMaxWidth];         // velocities of the owned points
+  double2 str[4][kQuadMaxWidth + 1];  // by corner: (str1, str5), (2, 7), (4, 8), (3, 6)
+  double cst[kTmaStepuFields][kQuadMaxWidth];
+};
+
+__device__ __forceinline__ double quad_xor(double x, int mask) {
+  return __shfl_xor_sync(0xffffffffu, x, mask);
+}
+
+__device__ __forceinline__ double quad_sign(double x, bool negative) {
+  return negative ? -x : x;
+}
+
+template <int NT, bool kStd>
+__global__ void __launch_bounds__(NT, 1) k_resident_quad(ResidentArgs a, Params p) {
+  extern __shared__ __align__(16) unsigned char res_raw[];
+  QuadSmem &S = *reinterpret_cast<QuadSmem *>(res_raw);
+  const int tid = threadIdx.x;
+  const int M = blockDim.x >> 2;
+  const int c = tid >> 2, k = tid & 3;  // the stress point and corner
+  const int cnt = a.cnt[blockIdx.x];
+  const size_t at = (size_t)blockIdx.x * M + c;
+  const int slot = a.slot[at];
+  const bool actT = slot >= 0 && !(a.flags[slot] & kSkipT);
+  // the stepu point of this thread
+  const bool own = tid < cnt;
+  const size_t uat = (size_t)blockIdx.x * M + (own ? tid : 0);
+  const int uslot = a.slot[uat];
+  const uint32_t nbr = a.str_idx[uat];
+  const bool actU = own && !(a.flags[uslot] & kSkipU);
+  const bool exported = own && (nbr & kResExport);
+
+  // ---- constants and state --------------------------------------------------
+  int ref = 0;  // where the corner's velocity is (ResidentPlan::corner)
+  Geom g = {};
+  double strength = 0.0, sp = 0.0, sm = 0.0, st = 0.0;
+  if (slot >= 0) {
+    ref = a.corner[4 * at + k];
+    g = make_geom(a.sg[0][slot], a.sg[1][slot], a.sg[2][slot], a.sg[3][slot], a.sg[4][slot],
+                  a.sg[5][slot], p.deltaminEVP);
+    strength = a.sg[6][slot];
+    sp = a.s_in[k][slot];
+    sm = a.s_in[4 + k][slot];
+    st = a.s_in[8 + k][slot];
+  }
+  const bool polled = slot >= 0 && ref < 0 && ~ref < a.nslots;
+  const bool ew = (k == 0) | (k == 3), ns = k < 2;
+  if (own) {
+#pragma unroll
+    for (int f = 0; f < kTmaStepuFields; f++) S.cst[f][tid] = a.uf[f][uslot];
+    S.uv[tid] = make_double2(a.u_in[uslot], a.v_in[uslot]);
+  }
+  if (c < M) S.str[k][c] = make_double2(0.0, 0.0);  // skipped T points keep str = 0
+  if (tid < 4) S.str[tid][kQuadMaxWidth] = make_double2(0.0, 0.0);
+  __syncthreads();
+
+  bool fail = false;
+  for (int sub = 0; sub < a.nsub; sub++) {
+    const bool wlast = a.last && sub == a.nsub - 1;
+    // ---- stress: whole warps (the shuffles), results of active points only ---
+    double2 w = make_double2(0.0, 0.0);
+    const bool wait = actT && polled && sub > 0;
+    if (actT && !wait) w = ref >= 0 ? S.uv[ref] : make_double2(a.u_in[~ref], a.v_in[~ref]);
+    // The warp polls together and stays converged (lanes that left a loop of
+    // their own one by one went through the rest of the stress one after the
+    // other: 4.7 us a subcycle instead of 1.65).
+    if (__any_sync(0xffffffffu, wait)) {
+      const unsigned seq = a.seq + (unsigned)sub;
+      const double4 *box =
+          a.mail + (size_t)(sub & 1) * (size_t)a.nslots + (wait ? ~ref : 0);
+      bool left = wait;
+      unsigned long long t0 = 0;
+      for (unsigned tries = 1;; tries++) {
+        if (left) {
+          const Mail m = mail_get(box);
+          if (mail_is(m, seq)) {
+            w = mail_value(m);
+            left = false;
+          }
+        }
+        if (!__any_sync(0xffffffffu, left)) break;
+        if ((tries & 63u) == 0) {
+          const unsigned long long t = res_ns();
+          if (t0 == 0) t0 = t;
+          if (__any_sync(0xffffffffu, t - t0 > kResWaitNs)) {
+            fail = left;
+            break;
+          }
+        }
+      }
+    }
+    const double u2 = quad_xor(w.x, 1), v2 = quad_xor(w.y, 1);
+    const double u4 = quad_xor(w.x, 3), v4 = quad_xor(w.y, 3);
+    double div, ten, shr, sq;
+    corner_strain_sq(k, w.x, w.y, u2, v2, u4, v4, g, p.e_factor, div, ten, shr, sq);
+    double Delta = 0.0;
+    const bool fast = fp64_dividend(strength) & fp64_mid(g.DminTarea) & fp64_radicand(sq) &
+                      (kStd | (p.capping == kC1) | (p.capping == 0.0));
+    Delta = fp64_sqrt(sq);
+    const bool capped = kStd || p.capping == kC1;
+    const double den = capped ? fmax_ref(Delta, g.DminTarea) : Delta + g.DminTarea;
+    const double visc = fp64_quot(strength, den, fp64_recip(den));
+    if (actT) {
+      if (fast)
+        corner_relax<kStd>(sp, sm, st, div, ten, shr, Delta, visc, p);
+      else
+        corner_update(sp, sm, st, div, ten, shr, sqrt(sq), strength, g.DminTarea, p);
+    }
+    __syncwarp();
+    const double p1 = quad_xor(sp, 1), p2 = quad_xor(sp, 2), p3 = quad_xor(sp, 3);
+    const double m1 = quad_xor(sm, 1), m2 = quad_xor(sm, 2), m3 = quad_xor(sm, 3);
+    const double t1 = quad_xor(st, 1), t2 = quad_xor(st, 2), t3 = quad_xor(st, 3);
+    if (actT) {
+      const double pN = sp + p1, pS = p2 + p3, pE = sp + p3, pW = p1 + p2;
+      const double mN = sm + m1, mS = m2 + m3, mE = sm + m3, mW = m1 + m2;
+      const double tN = st + t1, tS = t2 + t3, tE = st + t3, tW = t1 + t2;
+      const double cp = kP111 * sp + (p1 + p3) * kP055 + kP027 * p2;
+      const double cm = kP111 * sm + (m1 + m3) * kP055 + kP027 * m2;
+      const double ct = kP222 * st + (t1 + t3) * kP111 + kP055 * t2;
+      const double dx = g.dxT, dy = g.dyT;
+      const double tx = kP5 * dx * (kP333 * tE + kP166 * tW);
+      const double ty = kP5 * dy * (kP333 * tN + kP166 * tS);
+      const double px = kP25 * dy * (kP333 * pN + kP166 * pS);
+      const double mx = kP25 * dy * (kP333 * mN + kP166 * mS);
+      const double py = kP25 * dx * (kP333 * pE + kP166 * pW);
+      const double my = kP25 * dx * (kP333 * mE + kP166 * mW);
+      // ne, se: -strp - strm; nw, sw: +strp + strm; north: -str12, south: +
+      const double ox = quad_sign(px, ew) + quad_sign(mx, ew) + quad_sign(tx, ns) +
+                        g.dxhy * (-cp + cm) + g.dyhx * ct;
+      // north: -strp + strm; south: +strp - strm; east: -str12, west: +
+      const double oy = quad_sign(py, ns) + quad_sign(my, !ns) + quad_sign(ty, ew) -
+                        g.dyhx * (cp + cm) + g.dxhy * ct;
+      S.str[k][c] = make_double2(ox, oy);
+      if (wlast && c < cnt) {
+        // str1/5, str2/7, str4/8, str3/6
+        const int ix = ns ? k : 5 - k, iy = k == 0 ? 4 : k == 1 ? 6 : k == 2 ? 7 : 5;
+        a.str_out[ix][slot] = ox;
+        a.str_out[iy][slot] = oy;
+      }
+    }
+    if (fail) atomicMax(a.err, kResCode);
+    if (__syncthreads_or(fail)) return;
+    // ---- stepu ---------------------------------------------------------------
+    if (own) {
+      double2 z = S.uv[tid];
+      if (actU) {
+        StepuIn in;
+        in.uold = z.x;
+        in.vold = z.y;
+        in.kvrel = S.cst[0][tid];
+        in.uocn = S.cst[1][tid];
+        in.vocn = S.cst[2][tid];
+        in.waterx = S.cst[3][tid];
+        in.watery = S.cst[4][tid];
+        in.forcex = S.cst[5][tid];
+        in.forcey = S.cst[6][tid];
+        in.umassdti = S.cst[7][tid];
+        in.fm = S.cst[8][tid];
+        in.uarear = S.cst[9][tid];
+        in.Tbu = S.cst[10][tid];
+        in.uinit = S.cst[11][tid];
+        in.vinit = S.cst[12][tid];
+        const double2 s0 = S.str[0][tid], nw = S.str[1][nbr & 1023];
+        const double2 sw = S.str[2][(nbr >> 10) & 1023], sse = S.str[3][(nbr >> 20) & 1023];
+        in.s1 = s0.x;
+        in.s5 = s0.y;
+        in.s2nw = nw.x;
+        in.s7nw = nw.y;
+        in.s3sse = sse.x;
+        in.s6sse = sse.y;
+        in.s4sw = sw.x;
+        in.s8sw = sw.y;
+        const StepuOut o = stepu_point(in, p);
+        z = make_double2(o.u, o.v);
+        S.uv[tid] = z;
+        if (wlast) {
+          a.strintx[uslot] = o.strintx;
+          a.strinty[uslot] = o.strinty;
+          a.Cb[uslot] = o.Cb;
+        }
+      }
+      if (sub + 1 < a.nsub) {
+        if (exported)
+          mail_put(a.mail + (size_t)((sub + 1) & 1) * (size_t)a.nslots + uslot, z.x, z.y,
+                   a.seq + (unsigned)sub + 1u);
+        if (actU && a.uv_step) {
+          a.u_out[(size_t)(sub + 1) * a.uv_step + uslot] = z.x;
+          a.v_out[(size_t)(sub + 1) * a.uv_step + uslot] = z.y;
+        }
+      } else if (actU) {
+        a.u_out[(size_t)a.nsub * a.uv_step + uslot] = z.x;
+        a.v_out[(size_t)a.nsub * a.uv_step + uslot] = z.y;
+      }
+    }
+    __syncthreads();
+  }
+  if (c < cnt && actT) {  // (see k_resident)
+    a.s_out[k][slot] = sp;
+    a.s_out[4 + k][slot] = sm;
+    a.s_out[8 + k][slot] = st;
+  }
+}
+
 using ResKernel = void (*)(ResidentArgs, Params);
 struct ResVariant {
   int width;
@@ -376,7 +599,14 @@ const ResVariant kVariants[] = {variant<128, false>(), variant<256, false>(),
                                 variant<640, true>()};
 static_assert(sizeof(ResSmem<640, true>) <= 227 * 1024, "shared memory per block");
 
-const ResVariant *find_variant(int cls) {
+// The class of a quad plan is kQuadMaxWidth, of four threads a point.
+const ResVariant kQuad = {4 * kQuadMaxWidth,
+                          {k_resident_quad<4 * kQuadMaxWidth, false>,
+                           k_resident_quad<4 * kQuadMaxWidth, true>},
+                          sizeof(QuadSmem)};
+
+const ResVariant *find_variant(bool quad, int cls) {
+  if (quad) return cls == kQuadMaxWidth ? &kQuad : nullptr;
   for (const ResVariant &v : kVariants)
     if (v.width == cls) return &v;
   return nullptr;
@@ -384,8 +614,8 @@ const ResVariant *find_variant(int cls) {
 
 }  // namespace
 
-int resident_prepare(int device, int cls, int nblocks) {
-  const ResVariant *v = find_variant(cls);
+int resident_prepare(int device, bool quad, int cls, int nblocks) {
+  const ResVariant *v = find_variant(quad, cls);
   if (!v) return 0;
   int coop = 0, sms = 0, per_sm = 0;
   cudaError_t e = cudaSuccess;
@@ -403,15 +633,15 @@ int resident_prepare(int device, int cls, int nblocks) {
   return coop && nblocks <= sms * per_sm ? 1 : 0;
 }
 
-cudaError_t launch_resident(const ResidentArgs &given, const Params &p, int cls, int threads,
-                            int nblocks, cudaStream_t st) {
-  const ResVariant *v = find_variant(cls);
+cudaError_t launch_resident(const ResidentArgs &given, const Params &p, bool quad, int cls,
+                            int threads, int nblocks, cudaStream_t st) {
+  const ResVariant *v = find_variant(quad, cls);
   if (!v || nblocks <= 0 || given.nsub <= 0) return cudaErrorInvalidValue;
   ResidentArgs a = given;
   Params pp = p;
   void *args[] = {&a, &pp};
   return cudaLaunchCooperativeKernel((const void *)v->k[std_params(p) ? 1 : 0], dim3(nblocks),
-                                     dim3(threads), args, v->smem, st);
+                                     dim3(quad ? 4 * threads : threads), args, v->smem, st);
 }
 
 }  // namespace evp

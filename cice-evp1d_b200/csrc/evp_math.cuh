@@ -171,7 +171,7 @@ __host__ __device__ __forceinline__ void corner_update(
   s12 = (s12 * (kC1 - arlx1i * revp) + arlx1i * kP5 * e * shr) * denom1;
 }
 
-// Strain rates and Delta of corner k (0 ne, 1 nw, 2 sw, 3 se) in one
+// Strain rates and the square of Delta of corner k (0 ne, 1 nw, 2 sw, 3 se) in one
 // branch-free form, so that the four corners of a point can run on four lanes
 // of a warp.  With P1 = (cc, ee, ne, se)[k], P2 = (ee, cc, se, ne)[k] and
 // P4 = (se, ne, ee, cc)[k], the reference's twelve expressions
@@ -183,10 +183,10 @@ __host__ __device__ __forceinline__ void corner_update(
 // C3 = (cxm,cxm,cxp,cxp), B2 = (-dyT,dyT,dyT,-dyT), B4 = (-dxT,-dxT,dxT,dxT).
 // Every product and sum is the reference's own: a - b is a + (-b) and
 // (-a)*b is -(a*b) exactly in IEEE arithmetic.
-__host__ __device__ __forceinline__ void corner_strain(
+__host__ __device__ __forceinline__ void corner_strain_sq(
     int k, double u1, double v1, double u2, double v2, double u4, double v4,
     const Geom &g, double e_factor, double &div, double &ten, double &shr,
-    double &Delta) {
+    double &sq) {
   const bool a = (k == 0) | (k == 3);
   const bool b = k < 2;
   const double A1 = a ? g.cyp : g.cym;
@@ -198,7 +198,7 @@ __host__ __device__ __forceinline__ void corner_strain(
   div = A1 * u1 + B2 * u2 + A3 * v1 + B4 * v4;
   ten = -(C1 * u1) + B2 * u2 + C3 * v1 + (-B4) * v4;
   shr = -(C1 * v1) + B2 * v2 + (-C3) * u1 + B4 * u4;
-  Delta = sqrt(div * div + e_factor * (ten * ten + shr * shr));
+  sq = div * div + e_factor * (ten * ten + shr * shr);
 }
 
 // The 8 str combinations of the updated stresses (src/bench_v2b.F90:217-310).

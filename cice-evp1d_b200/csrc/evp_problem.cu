@@ -112,7 +112,8 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
   CUDA_TRY(cudaDeviceGetAttribute(&d->nctas, cudaDevAttrMultiProcessorCount, device));
   if (tma_prepare(device) != 0)
     return error(EVP1D_ERR_CUDA, "cannot enable %d bytes of shared memory", 0);
-  if (res.nblocks > 0 && resident_prepare(device, res.cls, res.nblocks)) {
+  if (res.nblocks > 0 && resident_prepare(device, res.quad, res.cls, res.nblocks)) {
+    d->res_quad = res.quad;
     d->res_blocks = res.nblocks;
     d->res_threads = res.threads;
     d->res_cls = res.cls;
@@ -417,7 +418,7 @@ cudaError_t problem_launch_resident(DeviceProblem *d, const Params &p, int nsub,
   a.seq = d->res_seq;
   a.err = d->err;
   d->res_seq += (unsigned)nsub;
-  return launch_resident(a, p, d->res_cls, d->res_threads, d->res_blocks, d->stream);
+  return launch_resident(a, p, d->res_quad, d->res_cls, d->res_threads, d->res_blocks, d->stream);
 }
 
 int problem_take_error(DeviceProblem *d, int *code) {

@@ -64,18 +64,24 @@ bool cut_blocks(int na, const int32_t *const nb0[6], const TilePlan &T, int thre
 }  // namespace
 
 bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T, int max_blocks,
-                         ResidentPlan *plan) {
+                         ResidentPlan *plan, bool quad) {
   ResidentPlan &R = *plan;
   R = ResidentPlan();
   // 17 bits of strip, row and piece in the sort key
   if (na <= 0 || !T.from_coords || max_blocks < 1 || na > (1 << 17)) return false;
   const double o = std::ceil((double)na / max_blocks);
-  const int least = (int)std::ceil((o + 1.8 * std::sqrt(o)) / 32.0) * 32;
+  const double least = o + 1.8 * std::sqrt(o);
   Cut cut;
-  int threads = std::max(least, kResMinWidth);
-  for (;; threads += 32) {
-    if (threads > kResMaxWidth) return false;
+  int threads = std::max((int)std::ceil(least / 8.0) * 8, kQuadMinWidth);
+  for (; quad && threads <= kQuadMaxWidth; threads += 8)
     if (cut_blocks(na, nb0, T, threads, max_blocks, &cut)) break;
+  R.quad = quad && threads <= kQuadMaxWidth;
+  if (!R.quad) {
+    threads = std::max((int)std::ceil(least / 32.0) * 32, kResMinWidth);
+    for (;; threads += 32) {
+      if (threads > kResMaxWidth) return false;
+      if (cut_blocks(na, nb0, T, threads, max_blocks, &cut)) break;
+    }
   }
   const int nb = (int)cut.off.size() - 1;
   R.nblocks = nb;
@@ -175,7 +181,7 @@ long long verify_resident_plan(const ResidentPlan &R, int na, const int32_t *con
   };
   const int M = R.threads;
   const size_t N = (size_t)R.nblocks * M;
-  if (M % 32 || M > R.cls || R.cls > kResMaxWidth || R.slot.size() != N || R.str.size() != N ||
+  if (M % (R.quad ? 8 : 32) || (R.quad && M > kQuadMaxWidth) || M > R.cls || R.cls > kResMaxWidth || R.slot.size() != N || R.str.size() != N ||
       R.corner.size() != 4 * N || R.cnt.size() != (size_t)R.nblocks) {
     wrong("sizes", -1, -1);
     return bad;

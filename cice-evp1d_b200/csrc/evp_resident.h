@@ -22,12 +22,17 @@ namespace evp {
 constexpr int kResWidths[] = {128, 256, 384, 512, 640};
 constexpr int kResMaxWidth = 640;
 constexpr int kResMinWidth = 128;  // four warps, one per scheduler
+// Small problems take four lanes per point (k_resident_quad), in blocks of up to
+// kQuadMaxWidth points: below that one thread per point leaves an SM's
+// schedulers a warp each, whose 2300 cycles of stress are instruction latency.
+constexpr int kQuadMinWidth = 32, kQuadMaxWidth = 128;
 // ResidentPlan::str bits
 constexpr uint32_t kResExport = 1u << 30;
 
 struct ResidentPlan {
   int nblocks = 0;
-  int threads = 0;  // per block: compute positions, a multiple of 32
+  int threads = 0;  // per block: compute positions (a multiple of 32; quad: of 8)
+  bool quad = false;  // four lanes per compute position
   int cls = 0;      // the kResWidths entry the kernel runs at
   std::vector<int32_t> cnt;   // [nblocks] owned points; positions below cnt are owned
   // [nblocks * threads]: device slot of each position, -1 for none
@@ -47,8 +52,9 @@ struct ResidentPlan {
 // problem does not fit one point per thread, has no grid layout, or where a
 // block would read from a block that does not read from it (the kernel's
 // two-deep mailboxes need the symmetry; grids have it).
+// `quad`: blocks for four lanes per point where the problem is small enough.
 bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &tiles,
-                         int max_blocks, ResidentPlan *plan);
+                         int max_blocks, ResidentPlan *plan, bool quad = true);
 
 // Decode every index of `plan` and compare it with the neighbour vectors.
 // Returns the number of violations; *first (if not null) describes the first.

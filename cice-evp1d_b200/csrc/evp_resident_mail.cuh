@@ -57,29 +57,31 @@ __device__ __forceinline__ unsigned long long res_ns() {
   return t;
 }
 
-// Wait (bounded) for message `seq` of the corners in `polled` (bit k: corner
-// k, whose point's slot is ~ref[k]).  The corners are polled together, so that
-// a round of reads costs one trip to L2; the words stay as they came until
-// every corner has its own (fewer registers than the values beside them).
-// Returns false when the wait ran out.
+// The whole warp waits (bounded) for message `seq` of the corners in each
+// lane's `polled` (bit k: corner k, whose point's slot is ~ref[k]; 0: none).
+// The corners are polled together, so that a round of reads costs one trip to
+// L2; the words stay as they came until every corner has its own (fewer
+// registers than the values beside them).  The lanes leave the loop together:
+// a warp whose lanes left one by one would go through what follows in as many
+// parts.  Returns false in every lane when the wait ran out.
 __device__ __forceinline__ bool mail_wait(Mail (&m)[4], const double4 *box, const int (&ref)[4],
                                           unsigned polled, unsigned seq) {
   unsigned left = polled;
   unsigned long long t0 = 0;
-  for (unsigned tries = 1;; tries++) {
+  for (unsigned tries = 1; __any_sync(0xffffffffu, left != 0); tries++) {
 #pragma unroll
     for (int k = 0; k < 4; k++)
       if (left >> k & 1) m[k] = mail_get(box + ~ref[k]);
 #pragma unroll
     for (int k = 0; k < 4; k++)
       if ((left >> k & 1) && mail_is(m[k], seq)) left &= ~(1u << k);
-    if (!left) return true;
     if ((tries & 63u) == 0) {
       const unsigned long long t = res_ns();
       if (t0 == 0) t0 = t;
-      if (t - t0 > kResWaitNs) return false;
+      if (__any_sync(0xffffffffu, t - t0 > kResWaitNs)) return false;
     }
   }
+  return true;
 }
 
 }  // namespace evp

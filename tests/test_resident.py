@@ -76,13 +76,16 @@ def _params(ndte, general):
     return p
 
 
-# widths 128, 256, 384, 512, 640 of the kernel
+# four lanes per point (mode 1, the smaller sizes; 180 x 140 is near its end), one
+# thread per point (mode 2): widths 128, 256, 384, 512, 640 of the kernel
 @pytest.mark.gpu
 @pytest.mark.parametrize("general", [False, True])
-@pytest.mark.parametrize("nx,ny,ndte", [(3, 2, 5), (64, 48, 24), (200, 150, 5), (300, 200, 5),
-                                        (330, 250, 4), (400, 300, 4)])
-def test_launch_bitwise(oracle_mod, nx, ny, ndte, general):
+@pytest.mark.parametrize("nx,ny,ndte,mode", [
+    (3, 2, 5, 1), (64, 48, 24, 1), (131, 77, 6, 1), (180, 140, 5, 1), (3, 2, 5, 2), (64, 48, 24, 2),
+    (200, 150, 5, 1), (300, 200, 5, 1), (330, 250, 4, 1), (400, 300, 4, 1)])
+def test_launch_bitwise(oracle_mod, monkeypatch, nx, ny, ndte, mode, general):
     from test_gpu_parity import assert_same, gpu_run, oracle_run
+    monkeypatch.setenv("EVP1D_RESIDENT", str(mode))
     g = synth.make_grid(nx, ny, seed=13, ndte=ndte, curvilinear=True)
     if general:
         rng = np.random.default_rng(5)
@@ -95,11 +98,12 @@ def test_launch_bitwise(oracle_mod, nx, ny, ndte, general):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 2, 3, 7, 101])
-def test_same_as_one_launch_per_subcycle(monkeypatch, n):
+@pytest.mark.parametrize("nx,ny", [(64, 48), (203, 151)])
+def test_same_as_one_launch_per_subcycle(monkeypatch, nx, ny, n):
     """The same bits as the subcycle kernel in every output, over three calls
     on one handle (mailbox numbers go on, both buffer sets are used), and the
     call that does not end (evp1d_subcycles_inner) between them."""
-    pr = synth.to_1d(synth.make_grid(203, 151, seed=5, ndte=n, curvilinear=True))
+    pr = synth.to_1d(synth.make_grid(nx, ny, seed=5, ndte=n, curvilinear=True))
     got = []
     for resident in ("1", "0"):
         monkeypatch.setenv("EVP1D_RESIDENT", resident)

@@ -191,6 +191,7 @@ bool tma_can_persist(int device, int nruns);
 struct ResidentArgs {
   int nslots = 0;
   // the resident plan (evp_resident.h)
+  int width = 0;  // positions per block (set by launch_resident)
   const int32_t *slot = nullptr, *cnt = nullptr, *corner = nullptr;
   const uint32_t *str_idx = nullptr;
   const uint8_t *flags = nullptr;

@@ -17,30 +17,34 @@ namespace evp {
 namespace {
 
 struct Cut {
+  int w = 0;                   // strip width of `order`
   std::vector<int32_t> order;  // list points, block after block
   std::vector<int32_t> off;    // [nblocks + 1]
 };
 
-// Blocks of at most `threads` compute positions, or nothing once more than
-// `max_blocks` are needed.
-bool cut_blocks(int na, const int32_t *const nb0[6], const TilePlan &T, int threads,
+// Blocks of at most `threads` compute positions and `owned` owned points, or
+// nothing once more than `max_blocks` are needed.
+bool cut_blocks(int na, const int32_t *const nb0[6], const TilePlan &T, int threads, int owned,
                 int max_blocks, Cut *cut) {
   const int w = std::max(4, std::min(63, (int)std::lround(std::sqrt((double)threads))));
-  std::vector<std::pair<uint64_t, int32_t>> key((size_t)na);
-  for (int p = 0; p < na; p++) {
-    const uint64_t i = (uint64_t)T.ci[p], j = (uint64_t)T.cj[p];
-    key[p] = {((uint64_t)T.piece[p] << 40) | ((i / w) << 23) | (j << 6) | (i % w), p};
+  if (cut->w != w) {
+    cut->w = w;
+    std::vector<std::pair<uint64_t, int32_t>> key((size_t)na);
+    for (int p = 0; p < na; p++) {
+      const uint64_t i = (uint64_t)T.ci[p], j = (uint64_t)T.cj[p];
+      key[p] = {((uint64_t)T.piece[p] << 40) | ((i / w) << 23) | (j << 6) | (i % w), p};
+    }
+    std::sort(key.begin(), key.end());
+    cut->order.resize((size_t)na);
+    for (int p = 0; p < na; p++) cut->order[p] = key[p].second;
   }
-  std::sort(key.begin(), key.end());
-  cut->order.resize((size_t)na);
-  for (int p = 0; p < na; p++) cut->order[p] = key[p].second;
   cut->off.assign(1, 0);
   std::vector<int32_t> own((size_t)na, -1), halo((size_t)na, -1);
   for (int k = 0; k < na;) {
     const int b = (int)cut->off.size() - 1;
     if (b == max_blocks) return false;
     int nh = 0, best = 1, len = 0;
-    while (k + len < na && len < threads && len + nh <= threads + 32) {
+    while (k + len < na && len < owned && len + nh <= threads + 32) {
       const int p = cut->order[k + len++];
       own[p] = b;
       if (halo[p] == b) nh--;
@@ -74,13 +78,17 @@ bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T,
   Cut cut;
   int threads = std::max((int)std::ceil(least / 8.0) * 8, kQuadMinWidth);
   for (; quad && threads <= kQuadMaxWidth; threads += 8)
-    if (cut_blocks(na, nb0, T, threads, max_blocks, &cut)) break;
+    if (cut_blocks(na, nb0, T, threads, threads, max_blocks, &cut)) break;
   R.quad = quad && threads <= kQuadMaxWidth;
   if (!R.quad) {
     threads = std::max((int)std::ceil(least / 32.0) * 32, kResMinWidth);
     for (;; threads += 32) {
       if (threads > kResMaxWidth) return false;
-      if (cut_blocks(na, nb0, T, threads, max_blocks, &cut)) break;
+      // wider than a CTA: a second stepu pass only where it cannot be avoided
+      if (threads > kResMaxThreads &&
+          cut_blocks(na, nb0, T, threads, kResMaxThreads, max_blocks, &cut))
+        break;
+      if (cut_blocks(na, nb0, T, threads, threads, max_blocks, &cut)) break;
     }
   }
   const int nb = (int)cut.off.size() - 1;
@@ -181,7 +189,8 @@ long long verify_resident_plan(const ResidentPlan &R, int na, const int32_t *con
   };
   const int M = R.threads;
   const size_t N = (size_t)R.nblocks * M;
-  if (M % (R.quad ? 8 : 32) || (R.quad && M > kQuadMaxWidth) || M > R.cls || R.cls > kResMaxWidth || R.slot.size() != N || R.str.size() != N ||
+  if (M % (R.quad ? 8 : 32) || (R.quad && M > kQuadMaxWidth) || M > R.cls ||
+      R.cls > kResMaxWidth || R.slot.size() != N || R.str.size() != N ||
       R.corner.size() != 4 * N || R.cnt.size() != (size_t)R.nblocks) {
     wrong("sizes", -1, -1);
     return bad;

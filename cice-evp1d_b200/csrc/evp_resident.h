@@ -17,10 +17,13 @@
 
 namespace evp {
 
-// Launch widths the kernel is compiled for; a block's compute set (owned
-// points, then forward halo) has at most that many points, one thread each.
-constexpr int kResWidths[] = {128, 256, 384, 512, 640};
-constexpr int kResMaxWidth = 640;
+// Widths the kernel is compiled for: a block's compute set (owned points, then
+// forward halo) has at most that many positions.  Up to kResMaxThreads a thread
+// each; of a wider block the positions beyond take four lanes each
+// (k_resident), as far as shared memory holds their constants.
+constexpr int kResMaxThreads = 512;
+constexpr int kResWidths[] = {128, 256, 384, kResMaxThreads, 736};
+constexpr int kResMaxWidth = 736;
 constexpr int kResMinWidth = 128;  // four warps, one per scheduler
 // Small problems take four lanes per point (k_resident_quad), in blocks of up to
 // kQuadMaxWidth points: below that one thread per point leaves an SM's

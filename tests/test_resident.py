@@ -77,7 +77,7 @@ def _params(ndte, general):
 
 
 # four lanes per point (mode 1, the smaller sizes; 180 x 140 is near its end), one
-# thread per point (mode 2): widths 128, 256, 384, 512, 640 of the kernel
+# thread per point (mode 2): widths 128, 256, 384, 512 of the kernel and beyond
 @pytest.mark.gpu
 @pytest.mark.parametrize("general", [False, True])
 @pytest.mark.parametrize("nx,ny,ndte,mode", [
@@ -153,3 +153,46 @@ def test_reverse_launch_bitwise(monkeypatch, nx, ny, ndte, interval):
     assert launches > 2 * ndte  # the second handle ran the two kernels
     for k in got[0]:
         assert np.array_equal(got[0][k].view(np.int64), got[1][k].view(np.int64)), k
+
+
+# blocks wider than a CTA: the positions beyond its 512 threads take four lanes
+# each, in one pass (400 x 300) or two (440 x 330, 460 x 345: the kernel's end);
+# more than 512 owned points a block (410 x 310 on) take two passes of stepu
+WIDE = [(400, 300), (410, 310), (440, 330), (460, 345)]
+
+
+@pytest.mark.parametrize("nx,ny", WIDE)
+def test_wide_plan_indices(shim, nx, ny):
+    pr = synth.to_1d(synth.make_grid(nx, ny, seed=3, ndte=2))
+    bad, (nb, threads, cls, most, halo, exported) = plan(shim, pr)
+    assert bad == 0
+    assert 512 < most <= threads <= cls
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("general", [False, True])
+@pytest.mark.parametrize("nx,ny", WIDE)
+def test_wide_launch_bitwise(oracle_mod, nx, ny, general):
+    """Against the oracle over calls that keep the resident launch's state
+    (stresses of the extra positions included), bit for bit."""
+    from test_gpu_parity import assert_same, gpu_run, oracle_run
+    ndte = 3
+    pr = synth.to_1d(synth.make_grid(nx, ny, seed=3, ndte=ndte, curvilinear=True))
+    p = _params(ndte, general)
+    fs = gpu_run(pr, ndte, params=p, explicit_init=general)
+    assert_same(fs, oracle_run(oracle_mod, pr, ndte, params=p), pr)
+    got = []
+    for resident in (True, False):
+        f = evp1d.FieldSet.from_problem(pr, want_str=True)
+        with evp1d.EVP1D.from_problem(pr, ndte=7, params=p) as s:
+            s.upload(f)
+            s.launch_count(reset=True)
+            for n in ((7, 6) if resident else (1,) * 13):
+                s.subcycles_inner(n)
+            assert s.launch_count() == (2 if resident else 13)
+            s.subcycles(2)
+            s.download(f)
+        got.append(f)
+    for k in ("stress", "uvel", "vvel", "strintx", "strinty", "Cb", "str"):
+        a, b = (np.asarray(getattr(f, k)).view(np.int64) for f in got)
+        assert np.array_equal(a, b), k

@@ -51,10 +51,21 @@ namespace {
 
 constexpr int kSSlots = 2;                          // stress-part ring
 constexpr int kRecRing = 4;                         // producer records in flight
-constexpr int kConsumers = kTileCompute;            // 256 = 8 warps, two per scheduler
-constexpr int kGatherWarps = 2;                     // producer warps issuing cp.async gathers
-constexpr int kStageWarps = 1 + kGatherWarps;       // bulk warp + gather warps
-constexpr int kThreads = kConsumers + 32 * kStageWarps;
+constexpr int kStressThreads = kTileCompute;        // 256 = 8 warps, two per scheduler
+constexpr int kStepuThreads = kTileCompute;         // 8 more
+constexpr int kGatherWarps = 3;                     // producer warps issuing cp.async gathers
+constexpr int kStageWarps = 1 + kGatherWarps;       // bulk warp + gather warps: a warpgroup
+constexpr int kThreads = kStressThreads + kStepuThreads + 32 * kStageWarps;
+// Registers: the launch gives each of 640 threads kLaunchRegs; the roles share
+// the same sum out again (setmaxnreg; its inc would wait for ever for more than
+// the launch's sum, which tma_prepare checks against the compiled kernels).
+constexpr int kLaunchRegs = 96;
+constexpr int kStressRegs = 144, kStepuRegs = 72, kStageRegs = 48;
+static_assert(kStressThreads * kStressRegs + kStepuThreads * kStepuRegs +
+                      32 * kStageWarps * kStageRegs <=
+                  kThreads * kLaunchRegs,
+              "the roles' registers are the launch's");
+static_assert(kStageWarps == 4, "setmaxnreg goes by warpgroups of four warps");
 constexpr int kUV = kTileOwned + kTileUvx;
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
 
@@ -85,13 +96,15 @@ struct Smem {
   // rotating str tables of what other points read: (str2, str7), (str3, str6),
   // (str4, str8); position kZeroSlot holds 0
   double2 str[3][3][kStrRow];
+  double2 own_str[2][kTileOwned];  // (str1, str5), read by their own point only
   int32_t rec[kRecRing][kRecInts];
   unsigned long long sfull[kSSlots];
   unsigned long long sempty[kSSlots];
-  unsigned long long rec_full[kRecRing];
+  unsigned long long rec_full[kRecRing], rec_empty[kRecRing];
   unsigned long long ufull, uempty;
-  int abort_flag;
-  int prod_ok;  // the bulk warp's waits succeeded for the current tile
+  unsigned long long strfull[2];  // stress of a step is in the str tables (even, odd steps)
+  unsigned long long strread[2];  // stepu of a step has read them
+  volatile int prod_ok;  // several subcycles: no producer warp's wait has run out
 };
 
 static_assert(sizeof(SSlot) % 16 == 0, "slots must keep 16-byte alignment");
@@ -207,18 +220,14 @@ __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Barrier of the consumer warps that also ORs a predicate over them.
-__device__ __forceinline__ bool consumer_sync_or(bool pred) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, 1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)pred), "r"(kConsumers)
-      : "memory");
-  return r != 0;
+// This warpgroup's registers per thread from here on.
+template <int kRegs>
+__device__ __forceinline__ void reg_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void reg_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
 
 // The bulk warp and the gather warps.
@@ -293,12 +302,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
   if (tid == 0) {
     for (int s = 0; s < kSSlots; s++) {
       mbar_init(&S.sfull[s], 1 + 32 * kGatherWarps);  // expect_tx arrival + cp.async lanes
-      mbar_init(&S.sempty[s], 1);                     // one consumer arrival per use
+      mbar_init(&S.sempty[s], kStressThreads / 32 + kStepuThreads / 32);
+      mbar_init(&S.strfull[s], kStressThreads / 32);
+      mbar_init(&S.strread[s], kStepuThreads / 32);
     }
-    for (int r = 0; r < kRecRing; r++) mbar_init(&S.rec_full[r], 1);
+    for (int r = 0; r < kRecRing; r++) {
+      mbar_init(&S.rec_full[r], 1);
+      mbar_init(&S.rec_empty[r], kStageWarps);
+    }
     mbar_init(&S.ufull, 1);
-    mbar_init(&S.uempty, kConsumers / 32);  // one arrival per consumer warp
-    S.abort_flag = 0;
+    mbar_init(&S.uempty, kStepuThreads / 32);
+    S.prod_ok = 1;
     mbar_fence_init();
   }
   if (tid < 9) S.str[tid / 3][tid % 3][kZeroSlot] = make_double2(0.0, 0.0);
@@ -321,7 +335,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
   constexpr size_t kBlk = (size_t)kConstFields * kTileOwned;  // doubles per constant block
   if (n <= 0) return;
 
-  if (tid >= kConsumers) {
+  if (tid >= kStressThreads + kStepuThreads) {
+    reg_dec<kStageRegs>();
     // ======================= producers ===================================
     // The bulk warp (pw 0) waits for the tile record and the free slot,
     // writes the slot header, arms the slot's full barrier and issues the
@@ -349,10 +364,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     // for the next slot absorbs the fence.  Every step's stepu part is out
     // before a round can wait on counters, so consumers finish every earlier
     // step without this round: no wait can depend on itself.
-    const int pw = (tid - kConsumers) >> 5;
+    const int pw = (tid - kStressThreads - kStepuThreads) >> 5;
     const int lane = tid & 31;
     constexpr uint32_t kRecBytes = kRecInts * 4u;
     const uint32_t ubytes = (cpt ? kTmaStepuCompact : kTmaStepuFields) * kTileOwned * 8u;
+    int nu = 0;   // stepu parts issued (the bulk warp's lane 0 counts)
     auto issue_stepu = [&](int q) {  // lane 0 of the bulk warp
       mbar_arrive_expect_tx(&S.ufull, ubytes);
       bulk_g2s(S.us.cu,
@@ -360,8 +376,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
                             kTileOwned,
                ubytes, &S.ufull);
     };
+    // issue the next one if its slot is free (stepu of the step before has its
+    // inputs)
+    auto pump_stepu = [&]() {
+      if (nu > 0 && nu < nq && mbar_test_wait(&S.uempty, (uint32_t)(nu - 1) & 1)) issue_stepu(nu++);
+    };
     int pub = 0;  // steps whose counters are raised (multi-subcycle launches)
-    int nu = 0;   // stepu parts issued (the bulk warp's lane 0 counts)
     // Lane 0: raise the counters of every step whose stepu has completed.
     // Stepu phases below nu - 1 are known complete (the bulk warp waited for
     // each before issuing a later stepu part); phase nu - 1, the last one
@@ -378,13 +398,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
         pub++;
       }
     };
-    if (pw == 0 && lane == 0) {
-      for (int r = 0; r < kRecRing && r < nq; r++) {
-        const int t = T0 + (kMulti ? r % n : r);
-        mbar_arrive_expect_tx(&S.rec_full[r], kRecBytes);
-        bulk_g2s(S.rec[r], a.tile_rec + (size_t)t * kRecInts, kRecBytes, &S.rec_full[r]);
-      }
-    }
+    int nrec = 0;  // records issued (the bulk warp's lane 0 counts)
+    auto issue_rec = [&]() {
+      const int r = nrec % kRecRing;
+      const int t = T0 + (kMulti ? nrec % n : nrec);
+      mbar_arrive_expect_tx(&S.rec_full[r], kRecBytes);
+      bulk_g2s(S.rec[r], a.tile_rec + (size_t)t * kRecInts, kRecBytes, &S.rec_full[r]);
+      nrec++;
+    };
+    if (pw == 0 && lane == 0)
+      while (nrec < kRecRing && nrec < nq) issue_rec();
     int issued = 0;
     bool ok = true;
     unsigned seen = 0u;  // per lane: the smallest counter polled for the next step
@@ -398,19 +421,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       const uint32_t use = (uint32_t)(issued / kSSlots);
       SSlot &st = S.ss[s];
       const int32_t *rec = S.rec[r];
-      if (pw == 0) {
-        int w = 1;
-        if (lane == 0) {
-          w = mbar_wait(&S.rec_full[r], (uint32_t)(issued / kRecRing) & 1, a.err, 6) ? 1 : 0;
-          trace_stamp(a, issued, 3);
-          if (w && issued >= kSSlots) {
-            // step q-1's stepu part; the slot frees after stepu of step q-2
-            w = mbar_wait(&S.uempty, (uint32_t)(nu - 1) & 1, a.err, 9) ? 1 : 0;
-            if (w) issue_stepu(nu++);
-            if (w) w = mbar_wait(&S.sempty[s], (use - 1) & 1, a.err, 2) ? 1 : 0;
+      int w = 1;
+      if (lane == 0) {
+        w = mbar_wait(&S.rec_full[r], (uint32_t)(issued / kRecRing) & 1, a.err, 6) ? 1 : 0;
+        if (pw == 0) trace_stamp(a, issued, 3);
+        if (w && issued >= kSSlots) {
+          if (pw == 0) {
+            // the bulk warp also issues stepu parts as their slot comes free
+            const unsigned long long t0 = global_ns();
+            while (!mbar_test_wait(&S.sempty[s], (use - 1) & 1)) {
+              pump_stepu();
+              if (global_ns() - t0 > kWaitNs) {
+                atomicMax(a.err, 2);
+                w = 0;
+                break;
+              }
+            }
+          } else {
+            w = mbar_wait(&S.sempty[s], (use - 1) & 1, a.err, 2) ? 1 : 0;
           }
         }
-        w = __shfl_sync(0xffffffffu, w, 0);
+      }
+      w = __shfl_sync(0xffffffffu, w, 0);
+      __syncwarp();
+      if (pw == 0) {
         if constexpr (kMulti) {
           if (w && sub > 0) {
             // the tiles step q depends on have finished subcycle sub - 1; the
@@ -426,7 +460,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
                 mine = ld_relaxed(a.epoch + a.dep_idx[d]) >= need;
               }
               if (__all_sync(0xffffffffu, mine)) break;
-              if (lane == 0) publish(q);
+              if (lane == 0) {
+                pump_stepu();  // (this CTA's own finished steps need theirs)
+                publish(q);
+              }
               // one decision for the whole warp (lane 0's clock)
               if (__shfl_sync(0xffffffffu, global_ns() - t0 > kWaitNs ? 1 : 0, 0)) {
                 if (lane == 0) atomicMax(a.err, 13);
@@ -460,10 +497,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
             mbar_arrive_expect_tx(&S.sfull[s], kCsBytes + 14 * b8);
           }
         }
-        if (lane == 0) S.prod_ok = w;
       }
-      stage_sync();  // handshake 1
-      if (!S.prod_ok) {
+      if constexpr (kMulti) {
+        // one decision for all four warps, which meet again below
+        if (!w && lane == 0) S.prod_ok = 0;
+        stage_sync();
+        w = S.prod_ok;
+        fence_proxy_async_global();
+      }
+      if (!w) {
         ok = false;
         break;
       }
@@ -478,13 +520,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
         }
         // the state the previous subcycle wrote
         if (issued == 0) griddep_wait();
-        if (lane >= 1 && lane <= 12)
-          bulk_g2s(st.s12[lane - 1], a.s[from][lane - 1] + off, b8, &S.sfull[s]);
-        else if (lane == 13)
-          bulk_g2s(st.u, u_in + off, b8, &S.sfull[s]);
-        else if (lane == 14)
-          bulk_g2s(st.v, v_in + off, b8, &S.sfull[s]);
         if (lane == 0) {
+          bulk_g2s(st.u, u_in + off, b8, &S.sfull[s]);
+          bulk_g2s(st.v, v_in + off, b8, &S.sfull[s]);
           if (issued == 0 && nu == 0) issue_stepu(nu++);
           trace_stamp(a, issued, 6);
         }
@@ -493,6 +531,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
         // every kGatherWarps-th halo field; the last one also the halo meta
         const int gw = pw - 1;
         if (issued == 0) griddep_wait();
+        if (lane < 12 / kGatherWarps) {
+          const int k = gw * (12 / kGatherWarps) + lane;
+          bulk_g2s(st.s12[k], a.s[from][k] + off, (uint32_t)((cnt + 3) & ~3) * 8u, &S.sfull[s]);
+        }
+        __syncwarp();
         if (!multi) {
           if (gw == 0)
             for (int x = lane; x < nx; x += 32)
@@ -559,14 +602,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       }
       // the record's generic reads come before its async-proxy refill
       fence_proxy_async();
-      stage_sync();  // handshake 2
+      if constexpr (kMulti) stage_sync();  // every warp is done with prod_ok
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.rec_empty[r]);
       if (pw == 0) {
-        if (lane == 0) trace_stamp(a, issued, 0);
-        const int qr = q + kRecRing;
-        if (lane == 0 && qr < nq) {
-          mbar_arrive_expect_tx(&S.rec_full[r], kRecBytes);
-          bulk_g2s(S.rec[r], a.tile_rec + (size_t)(T0 + (kMulti ? qr % n : qr)) * kRecInts, kRecBytes,
-                   &S.rec_full[r]);
+        if (lane == 0) {
+          trace_stamp(a, issued, 0);
+          pump_stepu();
+          // the record every warp has finished with by now
+          if (q >= 1 && nrec < nq) {
+            if (mbar_wait(&S.rec_empty[(q - 1) % kRecRing], (uint32_t)((q - 1) / kRecRing) & 1,
+                          a.err, 18))
+              issue_rec();
+          }
         }
         if (a.prefetch > 0 && !multi) {
           const int tp = t + a.prefetch;
@@ -598,9 +646,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     if (pw == 0) {
       if (ok && lane == 0) {
         // the stepu parts of the last steps
-        for (; nu < issued; nu++) {
+        while (nu < nq) {
           if (!mbar_wait(&S.uempty, (uint32_t)(nu - 1) & 1, a.err, 9)) break;
-          issue_stepu(nu);
+          issue_stepu(nu++);
         }
       }
       if (lane == 0 && nu > 0) mbar_wait(&S.ufull, (uint32_t)(nu - 1) & 1, a.err, 10);
@@ -619,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       }
       // records issued ahead and never consumed must land before exit too
       if (lane == 0) {
-        for (int k = issued; k < issued + kRecRing && k < nq; k++)
+        for (int k = issued; k < nrec; k++)
           mbar_wait(&S.rec_full[k % kRecRing], (uint32_t)(k / kRecRing) & 1, a.err, 7);
       }
     }
@@ -627,73 +675,161 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     return;
   }
 
-  // ========================= consumers ===================================
-  // Per step one block barrier: after stress, when the tile's str table is
-  // complete.  Stepu then runs warp by warp and each warp goes straight on to
-  // the next step's stress, so one warp's stepu overlaps the others' stress.
-  // Stepu of step q reads the tables of steps q and q-1 while stress of step
-  // q+1 writes the third; the table it writes last held step q-2, whose
-  // readers (stepu of q-2 and q-1) every warp has finished before any passes
-  // the barrier of step q.  (The first tile of a run never reads the previous
-  // table, so nothing crosses from one subcycle to the next there.)  The
-  // stepu slot is released by one arrival per warp.  A wait that ran out
-  // anywhere is OR-reduced at the barrier, so all consumers leave the loop
-  // together.
-  const int c = tid;  // compute-set index: owned c < cnt, halo cnt + h
   const int lane = tid & 31;
-  bool fail = false;
-  // Consumers write the ping-pong set the previous subcycle read: only after
-  // it has completed (their first tile cannot land before that anyway).
+  if (tid >= kStressThreads) {
+    // ======================= stepu of the owned points =====================
+    // Its inputs come to registers while stress of the same step runs: the
+    // packed word and the old velocities from the stress slot, the 13 fields
+    // from the stepu slot, which this frees for the next tile's.
+    reg_dec<kStepuRegs>();
+    const int c = tid - kStressThreads;
+    griddep_wait();
+    for (int q = 0; q < nq; q++) {
+      const int s = q % kSSlots;
+      const int b = q % 3;
+      const int bp = (q + 2) % 3;  // the previous tile's table
+      const int sub = kMulti ? q / n : 0;
+      const int to = (sub & 1) ^ 1;
+      const bool wlast = kMulti ? (a.last && sub == a.nsub - 1) : kLast;
+      StepuIn in;
+      uint32_t m = 0, sg = 0;  // sg: sign bits of uinit (bit 0) and vinit (bit 1)
+      int at = 0;
+      bool act = false;
+      bool ok = mbar_wait(&S.sfull[s], (uint32_t)(q / kSSlots) & 1, a.err, 1);
+      if (ok) {
+        const SSlot &st = S.ss[s];
+        at = st.hdr[0] + c;
+        if (c < st.hdr[1]) {
+          const unsigned long long ml = (unsigned long long)__double_as_longlong(st.cs[7][c]);
+          m = (uint32_t)ml;
+          sg = (uint32_t)(ml >> 62);
+          act = !((m >> 30) & kSkipU);
+          in.uold = st.u[c];
+          in.vold = st.v[c];
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.sempty[s]);
+      ok &= mbar_wait(&S.ufull, (uint32_t)q & 1, a.err, 11);
+      act &= ok;
+      if (act) {
+        const USlot &us = S.us;
+        in.kvrel = us.cu[0][c];
+        in.uocn = us.cu[1][c];
+        in.vocn = us.cu[2][c];
+        in.waterx = us.cu[3][c];
+        in.watery = us.cu[4][c];
+        in.forcex = us.cu[5][c];
+        in.forcey = us.cu[6][c];
+        in.umassdti = us.cu[7][c];
+        in.fm = us.cu[8][c];
+        in.uarear = us.cu[9][c];
+        if (cpt) {
+          // Tbu is +0; revp == 0, so revp*uinit is a zero with uinit's sign
+          in.Tbu = 0.0;
+          in.uinit = (sg & 1u) ? -1.0 : 1.0;
+          in.vinit = (sg & 2u) ? -1.0 : 1.0;
+        } else {
+          in.Tbu = us.cu[10][c];
+          in.uinit = us.cu[11][c];
+          in.vinit = us.cu[12][c];
+        }
+      }
+      // (In a launch of several subcycles the release also tells the bulk
+      // warp that the tile's velocities are stored, which it publishes to
+      // other CTAs: there it comes after the stores.)
+      if (!kMulti) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.uempty);
+      }
+      ok &= mbar_wait(&S.strfull[q & 1], (uint32_t)(q >> 1) & 1, a.err, 16);
+      act &= ok;
+      if (act) {
+        // a neighbour's str: own table, or the previous tile's (kStrPrev)
+        const uint32_t vnw = m & kLnbMask, vsw = (m >> kLnbBits) & kLnbMask;
+        const uint32_t vsse = (m >> (2 * kLnbBits)) & kLnbMask;
+        const double2 own = S.own_str[q & 1][c];
+        const double2 nw = S.str[(vnw & kStrPrev) ? bp : b][0][vnw & (kStrPrev - 1)];
+        const double2 sse = S.str[(vsse & kStrPrev) ? bp : b][1][vsse & (kStrPrev - 1)];
+        const double2 sw = S.str[(vsw & kStrPrev) ? bp : b][2][vsw & (kStrPrev - 1)];
+        in.s1 = own.x;
+        in.s5 = own.y;
+        in.s2nw = nw.x;
+        in.s7nw = nw.y;
+        in.s3sse = sse.x;
+        in.s6sse = sse.y;
+        in.s4sw = sw.x;
+        in.s8sw = sw.y;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.strread[q & 1]);
+      if (act) {
+        const StepuOut o = stepu_point(in, p);
+        double *u_out = kMulti && a.uv_step ? a.u[0] + (size_t)(sub + 1) * a.uv_step : a.u[to];
+        double *v_out = kMulti && a.uv_step ? a.v[0] + (size_t)(sub + 1) * a.uv_step : a.v[to];
+        u_out[at] = o.u;
+        v_out[at] = o.v;
+        if (wlast) {
+          a.strintx[at] = o.strintx;
+          a.strinty[at] = o.strinty;
+          a.Cb[at] = o.Cb;
+        }
+      }
+      if (kMulti) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.uempty);
+      }
+      if (c == 0) trace_stamp(a, q, 5);
+      if (__any_sync(0xffffffffu, !ok)) return;
+    }
+    return;
+  }
+
+  // ========================= stress ======================================
+  // A warp goes from tile to tile by itself: its inputs are all in registers
+  // before the arithmetic, so that the slot is free for the tile after next.
+  // The three str tables: stepu of step q reads those of q and q-1 while
+  // stress of q+1 writes the third; stress of q+2 writes over that of q-1, and
+  // over the even/odd own_str of q, and waits until stepu of q has read them.
+  // (The first tile of a run never reads the previous table, so nothing
+  // crosses from one subcycle to the next there.)  A warp whose wait ran out
+  // leaves; the waits for its arrivals run out in turn.
+  reg_inc<kStressRegs>();
+  const int c = tid;  // compute-set index: owned c < cnt, halo cnt + h
+  // Writes the ping-pong set the previous subcycle read: only after it has
+  // completed (the first tile cannot land before that anyway).
   griddep_wait();
-
-
-  // What stepu of a tile needs from its stress part, kept by the owned
-  // thread so that the slot can be released after stress.
-  struct Carry {
-    uint32_t m = 0;
-    uint32_t sg = 0;  // sign bits of uinit (bit 0) and vinit (bit 1)
-    double uold = 0.0, vold = 0.0;
-    double s1 = 0.0, s5 = 0.0;  // str1, str5: read by the point itself only
-    int off = 0, cnt = 0;
-  };
-
-  // ---------------- stress of step q ---------------------------------------
-  auto stress_tile = [&](int q) -> Carry {
-    Carry cy;
+  for (int q = 0; q < nq; q++) {
     const int s = q % kSSlots;
     const int b = q % 3;
     const int sub = kMulti ? q / n : 0;
     const int to = (sub & 1) ^ 1;
     const bool wlast = kMulti ? (a.last && sub == a.nsub - 1) : kLast;
-    const bool have = mbar_wait(&S.sfull[s], (uint32_t)(q / kSSlots) & 1, a.err, 1);
-    fail |= !have;
+    bool ok = mbar_wait(&S.sfull[s], (uint32_t)(q / kSSlots) & 1, a.err, 1);
     if (tid == 0) trace_stamp(a, q, 1);
-    const SSlot &st = S.ss[s];
-    if (have) {
-      cy.off = st.hdr[0];
-      cy.cnt = st.hdr[1];
-      const int nh = st.hdr[2];
-      const bool own = c < cy.cnt;
-      const int h = c - cy.cnt;
-      if (own || h < nh) {
+    bool own = false, in = false, act = false;
+    int at = 0;
+    double geo[7], s12[12];
+    Corners cr;
+    if (ok) {
+      const SSlot &st = S.ss[s];
+      const int cnt = st.hdr[1];
+      at = st.hdr[0] + c;
+      own = c < cnt;
+      const int h = c - cnt;
+      in = own || h < st.hdr[2];
+      if (in) {
         uint32_t m, lc;
         if (own) {
           const unsigned long long ml = (unsigned long long)__double_as_longlong(st.cs[7][c]);
           m = (uint32_t)ml;
           lc = (uint32_t)(ml >> 32);
-          cy.m = m;
-          cy.sg = lc >> 30;
-          cy.uold = st.u[c];
-          cy.vold = st.v[c];
         } else {
           m = st.hmeta[h];
           lc = st.hlcor[h];
         }
-        double out[8];
-        if ((m >> 30) & kSkipT) {
-#pragma unroll
-          for (int k = 0; k < 8; k++) out[k] = 0.0;
-        } else {
+        act = !((m >> 30) & kSkipT);
+        if (act) {
           // geometry and strength (fields 0..6), then the 12 stresses
           const double *F = own ? &st.cs[0][c] : &st.hf[0][h];
           const double *F12 = own ? &st.s12[0][c] : &st.hf[7][h];
@@ -701,7 +837,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
           const int cc = own ? c : (int)st.hlcc[h];
           const int iee = lc & kLnbMask, ine = (lc >> kLnbBits) & kLnbMask;
           const int ise = (lc >> (2 * kLnbBits)) & kLnbMask;
-          Corners cr;
           cr.ucc = st.u[cc];
           cr.vcc = st.v[cc];
           cr.uee = st.u[iee];
@@ -710,130 +845,41 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
           cr.vne = st.v[ine];
           cr.use = st.u[ise];
           cr.vse = st.v[ise];
-          const Geom gm = make_geom(F[0 * fs], F[1 * fs], F[2 * fs], F[3 * fs], F[4 * fs],
-                                    F[5 * fs], p.deltaminEVP);
-          double s12[12];
+#pragma unroll
+          for (int k = 0; k < 7; k++) geo[k] = F[k * fs];
 #pragma unroll
           for (int k = 0; k < 12; k++) s12[k] = F12[k * fs];
-          stress_point<kStd>(cr, gm, F[6 * fs], s12, out, p);
-          if (own) {
-#pragma unroll
-            for (int k = 0; k < 12; k++) a.s[to][k][cy.off + c] = s12[k];
-          }
-        }
-        S.str[b][0][c] = make_double2(out[1], out[6]);
-        S.str[b][1][c] = make_double2(out[2], out[5]);
-        S.str[b][2][c] = make_double2(out[3], out[7]);
-        cy.s1 = out[0];
-        cy.s5 = out[4];
-        if (wlast && own) {
-#pragma unroll
-          for (int k = 0; k < 8; k++) a.str_out[k][cy.off + c] = out[k];
         }
       }
     }
-    return cy;
-  };
-
-  // ---------------- stepu of step q, owned points ------------------------
-  auto stepu_tile = [&](int q, const Carry &cy) {
-    const int b = q % 3;
-    const int bp = (q + 2) % 3;  // the previous tile's table
-    const int sub = kMulti ? q / n : 0;
-    const int to = (sub & 1) ^ 1;
-    const bool wlast = kMulti ? (a.last && sub == a.nsub - 1) : kLast;
-    const bool hu = mbar_wait(&S.ufull, (uint32_t)q & 1, a.err, 11);
-    fail |= !hu;
-    const bool act = hu && c < cy.cnt && !((cy.m >> 30) & kSkipU);
-    // the 13 stepu inputs into registers first, so that the stepu slot is
-    // released before the arithmetic: the bulk warp then issues the next
-    // tile's stepu part and, behind it, the stress part after next a whole
-    // stepu earlier.  (In a launch of several subcycles the release also
-    // tells the bulk warp that the tile's velocities are stored, which it
-    // publishes to other CTAs: there it stays after the stores.)
-    StepuIn in;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&S.sempty[s]);
+    double out[8];
     if (act) {
-      const USlot &us = S.us;
-      in.kvrel = us.cu[0][c];
-      in.uocn = us.cu[1][c];
-      in.vocn = us.cu[2][c];
-      in.waterx = us.cu[3][c];
-      in.watery = us.cu[4][c];
-      in.forcex = us.cu[5][c];
-      in.forcey = us.cu[6][c];
-      in.umassdti = us.cu[7][c];
-      in.fm = us.cu[8][c];
-      in.uarear = us.cu[9][c];
-      if (cpt) {
-        // Tbu is +0; revp == 0, so revp*uinit is a zero with uinit's sign
-        in.Tbu = 0.0;
-        in.uinit = (cy.sg & 1u) ? -1.0 : 1.0;
-        in.vinit = (cy.sg & 2u) ? -1.0 : 1.0;
-      } else {
-        in.Tbu = us.cu[10][c];
-        in.uinit = us.cu[11][c];
-        in.vinit = us.cu[12][c];
+      const Geom gm = make_geom(geo[0], geo[1], geo[2], geo[3], geo[4], geo[5], p.deltaminEVP);
+      stress_point<kStd>(cr, gm, geo[6], s12, out, p);
+      if (own) {
+#pragma unroll
+        for (int k = 0; k < 12; k++) a.s[to][k][at] = s12[k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k++) out[k] = 0.0;
+    }
+    if (q >= 2) ok &= mbar_wait(&S.strread[q & 1], (uint32_t)((q >> 1) - 1) & 1, a.err, 17);
+    if (ok && in) {
+      S.str[b][0][c] = make_double2(out[1], out[6]);
+      S.str[b][1][c] = make_double2(out[2], out[5]);
+      S.str[b][2][c] = make_double2(out[3], out[7]);
+      if (own) S.own_str[q & 1][c] = make_double2(out[0], out[4]);
+      if (wlast && own) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) a.str_out[k][at] = out[k];
       }
     }
-    if (!kMulti) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.uempty);  // this warp is done with the stepu slot
-    }
-    if (act) {
-      const uint32_t m = cy.m;
-      // a neighbour's str: own table, or the previous tile's (kStrPrev)
-      const uint32_t vnw = m & kLnbMask, vsw = (m >> kLnbBits) & kLnbMask;
-      const uint32_t vsse = (m >> (2 * kLnbBits)) & kLnbMask;
-      const double2 nw = S.str[(vnw & kStrPrev) ? bp : b][0][vnw & (kStrPrev - 1)];
-      const double2 sse = S.str[(vsse & kStrPrev) ? bp : b][1][vsse & (kStrPrev - 1)];
-      const double2 sw = S.str[(vsw & kStrPrev) ? bp : b][2][vsw & (kStrPrev - 1)];
-      in.uold = cy.uold;
-      in.vold = cy.vold;
-      in.s1 = cy.s1;
-      in.s5 = cy.s5;
-      in.s2nw = nw.x;
-      in.s7nw = nw.y;
-      in.s3sse = sse.x;
-      in.s6sse = sse.y;
-      in.s4sw = sw.x;
-      in.s8sw = sw.y;
-      const StepuOut o = stepu_point(in, p);
-      double *u_out = kMulti && a.uv_step ? a.u[0] + (size_t)(sub + 1) * a.uv_step : a.u[to];
-      double *v_out = kMulti && a.uv_step ? a.v[0] + (size_t)(sub + 1) * a.uv_step : a.v[to];
-      u_out[cy.off + c] = o.u;
-      v_out[cy.off + c] = o.v;
-      if (wlast) {
-        a.strintx[cy.off + c] = o.strintx;
-        a.strinty[cy.off + c] = o.strinty;
-        a.Cb[cy.off + c] = o.Cb;
-      }
-    }
-    if (kMulti) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.uempty);
-    }
-    if (tid == 0) trace_stamp(a, q, 5);
-  };
-
-  // the barrier after stress of step q: its str table is complete and its
-  // stress slot free again
-  auto stress_done = [&](int q) -> bool {
-    const bool stop = consumer_sync_or(fail);
-    if (tid == 0) {
-      trace_stamp(a, q, 2);
-      mbar_arrive(&S.sempty[q % kSSlots]);
-    }
-    return stop;
-  };
-
-  Carry cur = stress_tile(0);
-  if (stress_done(0)) return;
-  for (int q = 0; q < nq; q++) {
-    stepu_tile(q, cur);
-    if (q + 1 >= nq) break;
-    const Carry nxt = stress_tile(q + 1);
-    if (stress_done(q + 1)) break;
-    cur = nxt;
+    if (__any_sync(0xffffffffu, !ok)) return;
+    if (lane == 0) mbar_arrive(&S.strfull[q & 1]);
+    if (tid == 0) trace_stamp(a, q, 2);
   }
 }
 
@@ -874,6 +920,9 @@ const char *tma_wait_name(int code) {
     case 9: return "the stepu-part warp waited for the stepu slot";
     case 10: return "the stepu-part warp waited for its last copy";
     case 11: return "a consumer waited for a tile's stepu inputs";
+    case 18: return "the producer waited for its warps to finish with a record";
+    case 16: return "stepu waited for a tile's stress";
+    case 17: return "stress waited for stepu to read the str tables";
     case 13: return "the producer waited for neighbouring tiles to finish a subcycle";
     case 15: return "a resident block waited for another block's velocities";
     case kProbeCode: return "the wait probe (evp1d_debug_wait_timeout)";
@@ -907,8 +956,13 @@ const TmaKernel kTmaAll[kTmaKernels] = {
 int tma_prepare(int device) {
   const int bytes = (int)smem_bytes();
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < kTmaKernels && e == cudaSuccess; i++)
-    e = cudaFuncSetAttribute(kTmaAll[i], cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  for (int i = 0; i < kTmaKernels && e == cudaSuccess; i++) {
+    cudaFuncAttributes at;
+    e = cudaFuncGetAttributes(&at, kTmaAll[i]);
+    if (e == cudaSuccess && at.numRegs < kLaunchRegs) e = cudaErrorInvalidKernelImage;
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kTmaAll[i], cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  }
   (void)device;
   return e == cudaSuccess ? 0 : (int)e;
 }

@@ -104,7 +104,7 @@ constexpr int kTmaStepuCompact = 10;
 // kTileOwned doubles per tile, fields [0..5] dxT dyT HTE HTN HTEm1 HTNm1,
 // [6] strength, [7] meta | lcor << 32 (the kConstStressFields that stress
 // reads), then [8..20] the 13 stepu inputs in the uf order; unused slots
-// hold 0.  Each of the two parts is one bulk copy.
+// hold 0.  The first part is one bulk copy, the second read field by field.
 constexpr int kConstStressFields = 8;
 constexpr int kConstFields = kConstStressFields + kTmaStepuFields;
 constexpr int kConstTileSlots = kTileOwned;
@@ -137,9 +137,8 @@ struct TmaArgs {
   // velocities stay in memory (the adjoint's tape entries); the stresses
   // still alternate between s[0] and s[1].
   size_t uv_step = 0;
-  // A launch of several subcycles: per tile a counter that each consumer warp
-  // raises by one when it is done with the tile in a subcycle (zeroed before
-  // the launch), and the tiles each tile waits for (evp_tiles.h dep_off /
+  // A launch of several subcycles: per tile a counter that its CTA raises by
+  // one when the tile's subcycle is stored (zeroed before the launch), and the tiles each tile waits for (evp_tiles.h dep_off /
   // dep_idx) before it loads the next subcycle's state.
   unsigned *epoch = nullptr;
   const int32_t *dep_off = nullptr, *dep_idx = nullptr;
@@ -157,9 +156,9 @@ struct TmaArgs {
   bool compact = false;
   const int *cflags = nullptr;
   // optional timing trace of block 0 (debug): per tile 8 %globaltimer stamps
-  // [0] producers issued all copies, [1] consumer 0 has the stress part,
-  // [2] stress done (consumer barrier), [3] bulk warp has the tile record,
-  // [4] stress slot free, [5] consumer warp 0 done with stepu, [6] bulk
+  // [0] producers issued all copies, [1] stress warp 0 has the stress part,
+  // [2] its str is in the table, [3] bulk warp has the tile record,
+  // [4] stress slot free, [5] stepu warp 0 done, [6] bulk
   // copies issued, [7] gathers issued; kTraceTiles tiles at most
   long long *trace = nullptr;
 };

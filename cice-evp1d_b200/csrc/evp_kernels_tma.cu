@@ -5,41 +5,52 @@
 // in order.  A tile's stress inputs (geometry, strength, packed index words,
 // the 12 stresses, u and v of the owned points and of the stencil's extra
 // points, and the recomputed forward halo) are staged in shared memory in a
-// two-slot ring, so one later tile loads while one computes.  The owned
-// points of a tile are contiguous slots and its per-call constants one
-// contiguous block, so the owned data arrive by cp.async.bulk (TMA) copies
-// completing on the slot's mbarrier (complete_tx); the halo and the extra
-// velocities are gathered with 4/8-byte cp.async, whose completion arrives on
-// the same mbarrier (cp.async.mbarrier.arrive).
-// Producer warps: the bulk warp (the bulk copies) and kGatherWarps gather
-// warps issuing the cp.async gathers side by side with it.  The producers'
-// own inputs -- the tile's slot range and gather lists -- are one 1.3 KB
-// record per tile that a bulk copy brings kRecRing tiles ahead, so no
-// producer waits on a global load.
-// Eight consumer warps (one thread per compute-set point: the tile's owned
-// points, then its forward halo, 256 at most) compute stress from shared
-// memory into the tile's str table, then stepu for the owned points, writing
-// the new stresses and velocities to the other ping-pong buffer.  Stepu reads
-// str from the tile's own table and from the previous tile's, which stays
-// alive: three str tables rotate, so that one tile's stress can start while
-// stepu still reads the two before it (six of the eight str, in pairs read
-// together; str1 and str5 are read by their own point alone and stay in its
-// registers: 26.3 -> 25.9 us a subcycle at 296k points against tables of
-// eight).  The 13 stepu inputs of a tile (the
-// second part of its constant block) arrive by one more bulk copy into a
-// stepu slot, which the consumers release as soon as each has its point's
-// inputs in registers.  Where every Tbu of the call is +0, every uinit and
-// vinit finite and revp == 0, the part stops after its tenth field: Tbu is
-// +0, and revp*uinit a signed zero whose sign comes from the packed word.
+// two-slot ring.  The owned points of a tile are contiguous slots and its
+// per-call constants one contiguous block, so the owned data arrive by
+// cp.async.bulk (TMA) copies completing on the slot's mbarrier (complete_tx);
+// the halo and the extra velocities are gathered with 4/8-byte cp.async, whose
+// completion arrives on the same mbarrier (cp.async.mbarrier.arrive).
+//
+// Three roles, each a number of warpgroups with registers of its own:
+//   producers (4 warps): the bulk warp writes the slot's header, arms its
+//     barrier and copies the constants, u and v; three gather warps copy four
+//     stresses each and gather a third of the halo.  Each waits for the slot
+//     and the record by itself.  (One warp issuing all 15 bulk copies took
+//     1.3 us a tile, of a period of 2.5; four take 0.5.)  Their own inputs,
+//     the tile's slot range and gather lists, are one 1.3 KB record per tile
+//     that a bulk copy brings up to kRecRing tiles ahead.
+//   stress (8 warps, one thread per compute-set point: the tile's owned points,
+//     then its forward halo, 256 at most): all inputs to registers, which
+//     frees the slot for the tile after next; the new stresses to the other
+//     ping-pong buffer; str to the tile's table, and what stepu needs of the
+//     point itself (old velocity, packed word) beside it.
+//   stepu (8 warps, the owned points): its 13 inputs (the second part of the
+//     constant block) straight to registers while stress runs (the bulk warp
+//     has prefetched them into L2), then str from the tile's own table and from
+//     the previous tile's, which stays alive: three tables rotate (six of the
+//     eight str, in pairs read together; str1 and str5 are read by their own
+//     point alone).  Where every Tbu of the call is +0, every uinit and vinit
+//     finite and revp == 0, the last three inputs are not read: Tbu is +0, and
+//     revp*uinit a signed zero whose sign comes from the packed word.
+// What bounds it: up to about 500k points stress, 2.1 us a tile: 1.45 in the
+// arithmetic, at 85 % of the FP64 pipe with stepu beside it, 0.65 in moving
+// its inputs and results, when the pipe idles (three warps per scheduler do
+// not fit the registers); above that HBM (1.18M points: 81 % of the measured
+// copy rate).  us a subcycle, against eight warps that did stress and stepu one
+// after the other with a shared-memory slot for stepu's inputs: 124k points
+// 12.4 -> 11.25, 190k 17.1 -> 15.6, 296k 25.9 -> 23.3, 460k 36.5 -> 33.1, 1.18M
+// 91.5 -> 83.  (With a single slot for stepu's inputs, freed when stepu began,
+// the copies' latency of 2 us a tile set the pace: 12.0, 25.0, 86.)
 // Consecutive one-subcycle launches overlap: each CTA lets the next launch
 // start at once (griddepcontrol.launch_dependents), and a launch started that
-// way loads its first tile's records, constants and stepu part while the
+// way loads its first tile's records, constants and stepu inputs while the
 // previous one finishes, reading the state only after griddepcontrol.wait.
 //
-// Every mbarrier wait is bounded by %globaltimer (kWaitNs): on expiry the
-// kernel records an error code, every thread of the consumer group leaves the
-// tile loop together, and each producer warp waits (bounded) for the copies it
-// has issued before it exits, so nothing is left in flight.
+// Every mbarrier wait is bounded by %globaltimer (kWaitNs): on expiry the warp
+// records an error code and leaves; the waits for its arrivals run out in turn.
+// The bulk warp waits (bounded) for the copies issued before it exits, so
+// nothing is left in flight.
+#include <cstddef>
 #include <cstdint>
 
 #include "evp_kernels.cuh"
@@ -85,30 +96,37 @@ struct SSlot {
 static_assert(kConstTileSlots == kTileOwned, "constant blocks hold one tile");
 static_assert(kConstFields == kConstStressFields + kTmaStepuFields, "constant block layout");
 
-// Stepu part of a tile: constant block fields 8..20 (one bulk copy).
-struct USlot {
-  double cu[kTmaStepuFields][kTileOwned];
-};
-
 struct Smem {
   SSlot ss[kSSlots];
-  USlot us;
   // rotating str tables of what other points read: (str2, str7), (str3, str6),
   // (str4, str8); position kZeroSlot holds 0
   double2 str[3][3][kStrRow];
-  double2 own_str[2][kTileOwned];  // (str1, str5), read by their own point only
-  int32_t rec[kRecRing][kRecInts];
+  // what stepu needs of its own point, from stress: (str1, str5); the old
+  // velocity, the packed word with uinit's and vinit's signs, the slot offset
+  double2 own_str[2][kTileOwned];
+  double2 old[3][kTileOwned];
+  uint2 word[3][kTileOwned];
+  int off[3];
+  alignas(16) int32_t rec[kRecRing][kRecInts];  // bulk copies' destination
   unsigned long long sfull[kSSlots];
   unsigned long long sempty[kSSlots];
   unsigned long long rec_full[kRecRing], rec_empty[kRecRing];
-  unsigned long long ufull, uempty;
   unsigned long long strfull[2];  // stress of a step is in the str tables (even, odd steps)
   unsigned long long strread[2];  // stepu of a step has read them
+  volatile int done[kStepuThreads / 32];  // several subcycles: steps each stepu warp has stored
   volatile int prod_ok;  // several subcycles: no producer warp's wait has run out
 };
 
 static_assert(sizeof(SSlot) % 16 == 0, "slots must keep 16-byte alignment");
 static_assert((kRecInts * 4) % 16 == 0, "records are bulk-copied");
+static_assert(offsetof(Smem, rec) % 16 == 0 && offsetof(Smem, ss) % 16 == 0 &&
+                  offsetof(Smem, str) % 16 == 0 && offsetof(Smem, own_str) % 16 == 0 &&
+                  offsetof(Smem, old) % 16 == 0 && offsetof(Smem, word) % 8 == 0 &&
+                  offsetof(Smem, sfull) % 8 == 0,
+              "alignment of bulk copies' destinations, 16-byte and mbarrier accesses");
+static_assert(offsetof(SSlot, s12) % 16 == 0 && offsetof(SSlot, u) % 16 == 0 &&
+                  offsetof(SSlot, v) % 16 == 0 && sizeof(double[kTileOwned]) % 16 == 0,
+              "bulk copies' destinations within a slot");
 static_assert(sizeof(Smem) <= 227 * 1024, "shared memory per block");
 
 // ---------------- PTX helpers -------------------------------------------------
@@ -140,19 +158,6 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, uint32_t 
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Non-blocking test whether the phase of parity `parity` has completed.
-__device__ __forceinline__ bool mbar_test_wait(unsigned long long *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(smem_addr(bar)), "r"(parity)
@@ -278,6 +283,14 @@ __device__ __forceinline__ unsigned ld_relaxed(const unsigned *p) {
   return v;
 }
 
+// Load of a constant of the call, read once (volatile: issued where it stands,
+// ahead of the waits that follow).
+__device__ __forceinline__ double ld_const(const double *p) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
 // Coherent 8-byte load (at L2) of state other CTAs may have written.
 __device__ __forceinline__ double ld_cg(const double *p) { return __ldcg(p); }
 
@@ -302,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
   if (tid == 0) {
     for (int s = 0; s < kSSlots; s++) {
       mbar_init(&S.sfull[s], 1 + 32 * kGatherWarps);  // expect_tx arrival + cp.async lanes
-      mbar_init(&S.sempty[s], kStressThreads / 32 + kStepuThreads / 32);
+      mbar_init(&S.sempty[s], kStressThreads / 32);
       mbar_init(&S.strfull[s], kStressThreads / 32);
       mbar_init(&S.strread[s], kStepuThreads / 32);
     }
@@ -310,8 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       mbar_init(&S.rec_full[r], 1);
       mbar_init(&S.rec_empty[r], kStageWarps);
     }
-    mbar_init(&S.ufull, 1);
-    mbar_init(&S.uempty, kStepuThreads / 32);
+    for (int w = 0; w < kStepuThreads / 32; w++) S.done[w] = 0;
     S.prod_ok = 1;
     mbar_fence_init();
   }
@@ -338,64 +350,38 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
   if (tid >= kStressThreads + kStepuThreads) {
     reg_dec<kStageRegs>();
     // ======================= producers ===================================
-    // The bulk warp (pw 0) waits for the tile record and the free slot,
-    // writes the slot header, arms the slot's full barrier and issues the
-    // bulk copies (TMA unit); the gather warps meanwhile gather the forward
-    // halo and the extra velocities (8-byte cp.async, or, in a launch of
-    // several subcycles, coherent loads).  Two named-barrier handshakes per
-    // step order the warps: after the first the slot is armed and the record
-    // readable, after the second every warp is done with the record, which
-    // the bulk warp then refills.  The bulk warp's waits are bounded and it
-    // reaches the first handshake on every path, so the handshakes cannot
-    // hang; a failed wait is passed on through prod_ok.
-    // Step q = (subcycle q / n, tile q % n).  In round q the bulk warp first
-    // issues step q-1's stepu part (once stepu of step q-2 has freed the
-    // stepu slot), then step q's stress part (once stress of step q-2 has
-    // freed its slot).  The TMA unit serves copies in issue order, which keeps
-    // the part needed first at the front.
+    // Each warp waits (bounded) for the tile record and the free slot.  The bulk
+    // warp (pw 0) writes the slot header, arms the slot's full barrier with the
+    // bytes of all bulk copies (the others' may land before: the phase still
+    // lacks the arrival) and issues the constants', u's and v's.  The gather
+    // warps issue the stresses' and gather the forward halo and the extra
+    // velocities (8-byte cp.async, or, in a launch of several subcycles,
+    // coherent loads).  A record is refilled once all four are done with it.
+    // Step q = (subcycle q / n, tile q % n).
     // A launch of several subcycles: step q's stress part goes out only when
-    // every tile its tile depends on has finished the previous subcycle.  Its
-    // lanes read those tiles' counters (relaxed) at the end of round q-1 and
-    // check them here, so the check usually costs no wait; the acquire fence
-    // then orders the state reads after the counters.  The bulk warp also
-    // publishes this CTA's steps: once stepu of a step is done (all consumer
-    // warps arrived on the stepu slot's barrier), it raises the tile's
-    // counter after a gpu-scope fence, at the end of a round, where the wait
-    // for the next slot absorbs the fence.  Every step's stepu part is out
-    // before a round can wait on counters, so consumers finish every earlier
-    // step without this round: no wait can depend on itself.
+    // every tile its tile depends on has finished the previous subcycle.  The
+    // bulk warp's lanes read those tiles' counters (relaxed) at the end of
+    // round q-1 and check them here, so the check usually costs no wait; the
+    // acquire fence then orders the state reads after the counters, and a
+    // barrier of the four warps the others' reads after that.  The bulk warp
+    // also publishes this CTA's steps: once every stepu warp has stored a step
+    // (S.done), it raises the tile's counter after a gpu-scope fence.  Stress
+    // and stepu finish every earlier step without this round: no wait can
+    // depend on itself.
     const int pw = (tid - kStressThreads - kStepuThreads) >> 5;
     const int lane = tid & 31;
     constexpr uint32_t kRecBytes = kRecInts * 4u;
     const uint32_t ubytes = (cpt ? kTmaStepuCompact : kTmaStepuFields) * kTileOwned * 8u;
-    int nu = 0;   // stepu parts issued (the bulk warp's lane 0 counts)
-    auto issue_stepu = [&](int q) {  // lane 0 of the bulk warp
-      mbar_arrive_expect_tx(&S.ufull, ubytes);
-      bulk_g2s(S.us.cu,
-               a.cblk + ((size_t)(T0 + (kMulti ? q % n : q)) * kConstFields + kConstStressFields) *
-                            kTileOwned,
-               ubytes, &S.ufull);
-    };
-    // issue the next one if its slot is free (stepu of the step before has its
-    // inputs)
-    auto pump_stepu = [&]() {
-      if (nu > 0 && nu < nq && mbar_test_wait(&S.uempty, (uint32_t)(nu - 1) & 1)) issue_stepu(nu++);
-    };
     int pub = 0;  // steps whose counters are raised (multi-subcycle launches)
-    // Lane 0: raise the counters of every step whose stepu has completed.
-    // Stepu phases below nu - 1 are known complete (the bulk warp waited for
-    // each before issuing a later stepu part); phase nu - 1, the last one
-    // issued, is tested: its parity is unambiguous because the phase after it
-    // cannot complete before the next part goes out.
+    // Lane 0: raise the counters of every step whose stepu has stored.
     auto publish = [&](int limit) {
       bool any = false;
-      while (pub < limit) {
-        const bool done = pub < nu - 1 || (pub == nu - 1 && mbar_test_wait(&S.uempty, (uint32_t)pub & 1));
-        if (!done) break;
+      for (; pub < limit; pub++) {
+        for (int w = 0; w < kStepuThreads / 32; w++)
+          if (S.done[w] <= pub) return;
         if (!any) __threadfence();
         any = true;
         atomicAdd(a.epoch + T0 + (kMulti ? pub % n : pub), 1u);
-        pub++;
       }
     };
     int nrec = 0;  // records issued (the bulk warp's lane 0 counts)
@@ -425,22 +411,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       if (lane == 0) {
         w = mbar_wait(&S.rec_full[r], (uint32_t)(issued / kRecRing) & 1, a.err, 6) ? 1 : 0;
         if (pw == 0) trace_stamp(a, issued, 3);
-        if (w && issued >= kSSlots) {
-          if (pw == 0) {
-            // the bulk warp also issues stepu parts as their slot comes free
-            const unsigned long long t0 = global_ns();
-            while (!mbar_test_wait(&S.sempty[s], (use - 1) & 1)) {
-              pump_stepu();
-              if (global_ns() - t0 > kWaitNs) {
-                atomicMax(a.err, 2);
-                w = 0;
-                break;
-              }
-            }
-          } else {
-            w = mbar_wait(&S.sempty[s], (use - 1) & 1, a.err, 2) ? 1 : 0;
-          }
-        }
+        if (w && issued >= kSSlots)
+          w = mbar_wait(&S.sempty[s], (use - 1) & 1, a.err, 2) ? 1 : 0;
       }
       w = __shfl_sync(0xffffffffu, w, 0);
       __syncwarp();
@@ -460,10 +432,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
                 mine = ld_relaxed(a.epoch + a.dep_idx[d]) >= need;
               }
               if (__all_sync(0xffffffffu, mine)) break;
-              if (lane == 0) {
-                pump_stepu();  // (this CTA's own finished steps need theirs)
-                publish(q);
-              }
+              if (lane == 0) publish(q);
               // one decision for the whole warp (lane 0's clock)
               if (__shfl_sync(0xffffffffu, global_ns() - t0 > kWaitNs ? 1 : 0, 0)) {
                 if (lane == 0) atomicMax(a.err, 13);
@@ -514,16 +483,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
         const uint32_t b8 = (uint32_t)((cnt + 3) & ~3) * 8u;
         if (lane == 0) {
           bulk_g2s(st.cs, a.cblk + (size_t)t * kBlk, kCsBytes, &S.sfull[s]);
-          // a programmatic dependent has the time: the first stepu part
-          // goes out before the state, while the previous launch drains
-          if (issued == 0 && a.pdl) issue_stepu(nu++);
+          // (stepu's loads of its part find it in L2)
+          bulk_prefetch_l2(a.cblk + (size_t)t * kBlk + kConstStressFields * kTileOwned, ubytes);
         }
         // the state the previous subcycle wrote
         if (issued == 0) griddep_wait();
         if (lane == 0) {
           bulk_g2s(st.u, u_in + off, b8, &S.sfull[s]);
           bulk_g2s(st.v, v_in + off, b8, &S.sfull[s]);
-          if (issued == 0 && nu == 0) issue_stepu(nu++);
           trace_stamp(a, issued, 6);
         }
       } else {
@@ -608,7 +575,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       if (pw == 0) {
         if (lane == 0) {
           trace_stamp(a, issued, 0);
-          pump_stepu();
           // the record every warp has finished with by now
           if (q >= 1 && nrec < nq) {
             if (mbar_wait(&S.rec_empty[(q - 1) % kRecRing], (uint32_t)((q - 1) / kRecRing) & 1,
@@ -644,14 +610,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       issued++;
     }
     if (pw == 0) {
-      if (ok && lane == 0) {
-        // the stepu parts of the last steps
-        while (nu < nq) {
-          if (!mbar_wait(&S.uempty, (uint32_t)(nu - 1) & 1, a.err, 9)) break;
-          issue_stepu(nu++);
-        }
-      }
-      if (lane == 0 && nu > 0) mbar_wait(&S.ufull, (uint32_t)(nu - 1) & 1, a.err, 10);
       if (multi && lane == 0) {
         // the last steps' counters (a later launch zeroes them anyway)
         const unsigned long long t0 = global_ns();
@@ -678,73 +636,50 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
   const int lane = tid & 31;
   if (tid >= kStressThreads) {
     // ======================= stepu of the owned points =====================
-    // Its inputs come to registers while stress of the same step runs: the
-    // packed word and the old velocities from the stress slot, the 13 fields
-    // from the stepu slot, which this frees for the next tile's.
+    // Its 13 fields come to registers, straight from the constant block, while
+    // stress of the same step runs; the rest is in the tables of strfull.
     reg_dec<kStepuRegs>();
     const int c = tid - kStressThreads;
-    griddep_wait();
     for (int q = 0; q < nq; q++) {
-      const int s = q % kSSlots;
       const int b = q % 3;
       const int bp = (q + 2) % 3;  // the previous tile's table
       const int sub = kMulti ? q / n : 0;
       const int to = (sub & 1) ^ 1;
       const bool wlast = kMulti ? (a.last && sub == a.nsub - 1) : kLast;
+      const double *cu = a.cblk + ((size_t)(T0 + (kMulti ? q % n : q)) * kConstFields +
+                                   kConstStressFields) * kTileOwned + c;
       StepuIn in;
-      uint32_t m = 0, sg = 0;  // sg: sign bits of uinit (bit 0) and vinit (bit 1)
-      int at = 0;
-      bool act = false;
-      bool ok = mbar_wait(&S.sfull[s], (uint32_t)(q / kSSlots) & 1, a.err, 1);
-      if (ok) {
-        const SSlot &st = S.ss[s];
-        at = st.hdr[0] + c;
-        if (c < st.hdr[1]) {
-          const unsigned long long ml = (unsigned long long)__double_as_longlong(st.cs[7][c]);
-          m = (uint32_t)ml;
-          sg = (uint32_t)(ml >> 62);
-          act = !((m >> 30) & kSkipU);
-          in.uold = st.u[c];
-          in.vold = st.v[c];
-        }
+      in.kvrel = ld_const(cu);
+      in.uocn = ld_const(cu + kTileOwned);
+      in.vocn = ld_const(cu + 2 * kTileOwned);
+      in.waterx = ld_const(cu + 3 * kTileOwned);
+      in.watery = ld_const(cu + 4 * kTileOwned);
+      in.forcex = ld_const(cu + 5 * kTileOwned);
+      in.forcey = ld_const(cu + 6 * kTileOwned);
+      in.umassdti = ld_const(cu + 7 * kTileOwned);
+      in.fm = ld_const(cu + 8 * kTileOwned);
+      in.uarear = ld_const(cu + 9 * kTileOwned);
+      in.Tbu = 0.0;
+      if (!cpt) {
+        in.Tbu = ld_const(cu + 10 * kTileOwned);
+        in.uinit = ld_const(cu + 11 * kTileOwned);
+        in.vinit = ld_const(cu + 12 * kTileOwned);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.sempty[s]);
-      ok &= mbar_wait(&S.ufull, (uint32_t)q & 1, a.err, 11);
-      act &= ok;
+      if (q == 0) griddep_wait();
+      const bool ok = mbar_wait(&S.strfull[q & 1], (uint32_t)(q >> 1) & 1, a.err, 16);
+      const uint2 word = S.word[b][c];
+      const uint32_t m = word.x;
+      const bool act = ok && !((m >> 30) & kSkipU);
+      const int at = S.off[b] + c;
       if (act) {
-        const USlot &us = S.us;
-        in.kvrel = us.cu[0][c];
-        in.uocn = us.cu[1][c];
-        in.vocn = us.cu[2][c];
-        in.waterx = us.cu[3][c];
-        in.watery = us.cu[4][c];
-        in.forcex = us.cu[5][c];
-        in.forcey = us.cu[6][c];
-        in.umassdti = us.cu[7][c];
-        in.fm = us.cu[8][c];
-        in.uarear = us.cu[9][c];
+        const double2 old = S.old[b][c];
+        in.uold = old.x;
+        in.vold = old.y;
         if (cpt) {
           // Tbu is +0; revp == 0, so revp*uinit is a zero with uinit's sign
-          in.Tbu = 0.0;
-          in.uinit = (sg & 1u) ? -1.0 : 1.0;
-          in.vinit = (sg & 2u) ? -1.0 : 1.0;
-        } else {
-          in.Tbu = us.cu[10][c];
-          in.uinit = us.cu[11][c];
-          in.vinit = us.cu[12][c];
+          in.uinit = (word.y >> 30 & 1u) ? -1.0 : 1.0;
+          in.vinit = (word.y >> 31) ? -1.0 : 1.0;
         }
-      }
-      // (In a launch of several subcycles the release also tells the bulk
-      // warp that the tile's velocities are stored, which it publishes to
-      // other CTAs: there it comes after the stores.)
-      if (!kMulti) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&S.uempty);
-      }
-      ok &= mbar_wait(&S.strfull[q & 1], (uint32_t)(q >> 1) & 1, a.err, 16);
-      act &= ok;
-      if (act) {
         // a neighbour's str: own table, or the previous tile's (kStrPrev)
         const uint32_t vnw = m & kLnbMask, vsw = (m >> kLnbBits) & kLnbMask;
         const uint32_t vsse = (m >> (2 * kLnbBits)) & kLnbMask;
@@ -777,7 +712,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       }
       if (kMulti) {
         __syncwarp();
-        if (lane == 0) mbar_arrive(&S.uempty);
+        if (lane == 0) {
+          __threadfence();
+          S.done[c >> 5] = q + 1;
+        }
       }
       if (c == 0) trace_stamp(a, q, 5);
       if (__any_sync(0xffffffffu, !ok)) return;
@@ -811,6 +749,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
     int at = 0;
     double geo[7], s12[12];
     Corners cr;
+    uint2 word = make_uint2((uint32_t)kSkipU << 30, 0u);
     if (ok) {
       const SSlot &st = S.ss[s];
       const int cnt = st.hdr[1];
@@ -824,6 +763,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
           const unsigned long long ml = (unsigned long long)__double_as_longlong(st.cs[7][c]);
           m = (uint32_t)ml;
           lc = (uint32_t)(ml >> 32);
+          word = make_uint2(m, lc);
+          S.old[b][c] = make_double2(st.u[c], st.v[c]);
         } else {
           m = st.hmeta[h];
           lc = st.hlcor[h];
@@ -852,6 +793,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
         }
       }
     }
+    S.word[b][c] = word;
+    if (tid == 0) S.off[b] = at;
     __syncwarp();
     if (lane == 0) mbar_arrive(&S.sempty[s]);
     double out[8];
@@ -917,9 +860,6 @@ const char *tma_wait_name(int code) {
     case 6: return "the producer waited for a tile record";
     case 7: return "the producer waited for records issued ahead";
     case 8: return "the dynamic shared memory was not 16-byte aligned";
-    case 9: return "the stepu-part warp waited for the stepu slot";
-    case 10: return "the stepu-part warp waited for its last copy";
-    case 11: return "a consumer waited for a tile's stepu inputs";
     case 18: return "the producer waited for its warps to finish with a record";
     case 16: return "stepu waited for a tile's stress";
     case 17: return "stress waited for stepu to read the str tables";

@@ -1,0 +1,31 @@
+"""The subcycle kernel, whose producer, stress and stepu warps go on by
+themselves, against the oracle, bit for bit (zero tolerance: the same
+operations in the same order).  Sizes: runs of no more than one tile, of two,
+three (every table in use once) and five; all 13 stepu inputs read (general)
+and ten."""
+import numpy as np
+import pytest
+
+import evp1d
+from evp1d import synth
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("general", [False, True])
+@pytest.mark.parametrize("runs,nx,ny", [(148, 3, 2), (148, 131, 77), (16, 131, 77), (10, 131, 77),
+                                        (6, 131, 77), (148, 531, 377)])
+def test_roles_bitwise(oracle_mod, monkeypatch, runs, nx, ny, general):
+    from test_gpu_parity import assert_same, gpu_run, oracle_run
+    monkeypatch.setenv("EVP1D_RESIDENT", "0")
+    monkeypatch.setenv("EVP1D_RUNS", str(runs))
+    ndte = 4
+    g = synth.make_grid(nx, ny, seed=21, ndte=ndte, curvilinear=True)
+    p = evp1d.set_evp_parameters(ndte)
+    if general:
+        p.revp, p.Ktens, p.capping = 1.0, 0.2, 0.0
+        p.cosw, p.sinw = np.cos(0.4), np.sin(0.4)
+        rng = np.random.default_rng(6)
+        g.f["Tbu"] = np.asfortranarray(rng.uniform(0.0, 5.0, g.f["Tbu"].shape))
+    pr = synth.to_1d(g)
+    fs = gpu_run(pr, ndte, params=p, explicit_init=general)
+    assert_same(fs, oracle_run(oracle_mod, pr, ndte, params=p), pr)

@@ -35,6 +35,13 @@ namespace evp {
 namespace {
 
 constexpr int kThreads = 256;
+// The two kernels of a reverse subcycle wait on memory, then on chains of FP64
+// (38 % of the FP64 pipe, 30 to 48 % of the DRAM rate).  Their registers allow 16
+// and 24 warps an SM; in blocks of two warps a finished warp's place is taken
+// at once, not when seven others have finished, and the phases mix: us a
+// subcycle against blocks of eight, 125k points 15.0 / 16.2, 295k 39.0 / 41.0,
+// 457k 62.1 / 65.3 (four warps 15.1, 39.5, 63.0; one 16.1, 38.8, 61.9).
+constexpr int kSweepThreads = 64;
 
 #define ADJ_TRY(x)                                                         \
   do {                                                                     \
@@ -133,7 +140,7 @@ __device__ __forceinline__ void str_lam(const AdjArgs &a, int t, int w, double &
 }
 
 template <bool kOne>
-__global__ void __launch_bounds__(kThreads, 3)  // 80 registers: 24 warps per SM, no spills
+__global__ void __launch_bounds__(kSweepThreads, 768 / kSweepThreads)  // 80 registers
 k_adj_stepu(AdjArgs a, Params p, const double *__restrict__ u0, const double *__restrict__ v0,
             const double *__restrict__ u1, const double *__restrict__ v1) {
   // launched as a programmatic dependent: the previous kernel's results
@@ -208,7 +215,7 @@ __device__ __forceinline__ void store_corners(const AdjArgs &a, int w, int iee, 
 }
 
 template <bool kOne>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kSweepThreads, 512 / kSweepThreads)
 k_adj_stress(AdjArgs a, Params p, const double *__restrict__ u, const double *__restrict__ v) {
   griddep_launch_dependents();
   griddep_wait();
@@ -242,7 +249,8 @@ k_adj_stress(AdjArgs a, Params p, const double *__restrict__ u, const double *__
                              a.HTNm1[w], p.deltaminEVP);
     double lc[8], lstr;
     // (the straight-line form spills at 16 warps an SM and measured slower
-    // here, 47.1 against 41.8 us a subcycle for both kernels on 294k points)
+    // here, 47.1 against 41.8 us a subcycle for both kernels on 294k points; at 12
+    // warps, where it does not, 42.3 against 39.0)
     stress_adjoint(c, g, a.strength[w], p, lo, ls, lc, lstr);
 #pragma unroll
     for (int k = 0; k < 12; k++) a.LS[k][w] = ls[k];
@@ -811,8 +819,8 @@ int evp1d_adjoint_sweep(evp1d_t *h) {
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = h->pdl ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
+  cfg.gridDim = dim3((unsigned)((d.nslots + kSweepThreads - 1) / kSweepThreads));
+  cfg.blockDim = dim3(kSweepThreads);
   cfg.stream = st;
   cfg.attrs = pdl;
   cfg.numAttrs = 1;

@@ -53,11 +53,14 @@ constexpr uint32_t kLnbMask = (1u << kLnbBits) - 1;
 // Widths (grid columns) of the strips the grid points are ordered in, chosen
 // by the points per run: wide strips recompute less of the strip's right
 // edge, narrow ones less of the row above a run's first tile, which matters
-// when runs are short (grid1600x1200, 8,000 points per run: 97.9 us per
-// subcycle at 64 columns against 100.1 at 48 and 100.3 at 80; the halo cap
-// of 64 points bounds the width).
-constexpr int kStripWide = 64, kStripNarrow = 48;
-constexpr int kStripWideRun = 4096;  // points per run from which strips are wide
+// when runs are short.  us per subcycle at 48 / 64 / 88 / 112 columns: 102k
+// points (690 a run) 9.3 / 11.2 / 11.0 / 11.0 (a tile more in the longest
+// run), 124k 11.2 / 11.2 / 11.1 / 13.0, 190k (1280) 15.5 / 15.5 / 15.3 / 17.2,
+// 296k 23.3 / 22.8 / 22.5 / 22.3, 797k 58.2 / 56.7 / 55.2 / 54.4, 1.18M 85.7 /
+// 84.3 / 81.2 / 81.6 (the caps of 64 halo points and 128 extra velocities bound
+// the width).
+constexpr int kStripWide = 88, kStripNarrow = 48;
+constexpr int kStripWideRun = 1024;  // points per run from which strips are wide
 
 struct TilePlan {
   int na = 0, navel = 0;

@@ -330,8 +330,7 @@ struct AdjointState {
   int32_t *tr_off[kNumTr] = {}, *tr_idx[kNumTr] = {};
   int32_t *tr_one[kNumTr] = {};
   bool one = false;  // every transposed list has at most one entry
-  // the neighbour relations are each other's inverse, and the resident plan's
-  // blocks can run the reverse sweep (launch_resident_adjoint)
+  // the resident plan's blocks can run the reverse sweep (launch_resident_adjoint)
   bool resident = false;
   double *Pu = nullptr, *Pv = nullptr, *Lx = nullptr, *Ly = nullptr;
   double *C8[8] = {}, *LS[12] = {}, *g[kNumGrad] = {};
@@ -429,18 +428,8 @@ int ensure_static(evp1d_t *h) {
         if (off[t][w + 1] > off[t][w]) direct[(size_t)t * S + w] = idx[t][off[t][w]];
   }
   A.one = one;
-  // nw of ee, sw of ne, sse of se and back, wherever both ends are list points
-  bool inverse = one;
-  for (int s = 0; s < S && inverse; s++) {
-    if (pos[s] < 0) continue;
-    const int pair[3][2] = {{0, 3}, {1, 4}, {2, 5}};
-    for (const auto &q : pair)
-      for (int r = 0; r < 2; r++) {
-        const int o = nbk(q[r], s);
-        if (o < S && nbk(q[1 - r], o) != s) inverse = false;
-      }
-  }
-  A.resident = inverse && h->resident && d.res_blocks > 0 && d.res_cls <= kResAdjointMax &&
+  // (a resident plan's relations are each other's inverse)
+  A.resident = h->resident && d.res_blocks > 0 && d.res_cls <= kResAdjointMax &&
                resident_adjoint_prepare(d.device, d.res_cls, d.res_blocks) != 0;
   // carve
   const size_t SD = pad256((size_t)S);

@@ -23,8 +23,9 @@
 // mailboxes, for even and odd subcycles.  One can be written again without
 // looking: a block writes number n+2 only after it has read number n+1 from
 // every block it reads from; those had then passed the barrier after their
-// stress n, and they include every block that reads this one (the plan
-// requires the symmetry).
+// stress n, and they include every block that waits for this one (the plan
+// requires inverse neighbour relations, which make waiting mutual whatever
+// the mask: inverse_relations in evp_resident.cpp).
 // The CTAs wait on one another, so the launch is cooperative (all resident or
 // none).  Every wait is bounded: on expiry the code goes to the error word,
 // the CTA leaves together at the next barrier, and its neighbours' waits run

@@ -65,6 +65,25 @@ bool cut_blocks(int na, const int32_t *const nb0[6], const TilePlan &T, int thre
   return true;
 }
 
+// Whether nw of ee, sw of ne, sse of se and back return to the point wherever
+// both ends are list points; *first: a point where they do not.  Then the
+// blocks that read a corner velocity of a T point are those that own one of
+// its corners, and every one of them computes the point: a point that is not
+// skipped makes all of them wait for one another, a skipped one none, so
+// waiting is mutual under every mask.  (Symmetry between blocks over all
+// points is not enough: a mask can leave only one side's points.)
+bool inverse_relations(int na, const int32_t *const nb0[6], int *first) {
+  for (int r = 0; r < 6; r++)
+    for (int p = 0; p < na; p++) {
+      const int q = nb0[r][p];
+      if (q < na && nb0[(r + 3) % 6][q] != p) {
+        *first = p;
+        return false;
+      }
+    }
+  return true;
+}
+
 }  // namespace
 
 bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T, int max_blocks,
@@ -72,7 +91,10 @@ bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T,
   ResidentPlan &R = *plan;
   R = ResidentPlan();
   // 17 bits of strip, row and piece in the sort key
-  if (na <= 0 || !T.from_coords || max_blocks < 1 || na > (1 << 17)) return false;
+  int one_way;
+  if (na <= 0 || !T.from_coords || max_blocks < 1 || na > (1 << 17) ||
+      !inverse_relations(na, nb0, &one_way))
+    return false;
   const double o = std::ceil((double)na / max_blocks);
   const double least = o + 1.8 * std::sqrt(o);
   Cut cut;
@@ -110,7 +132,6 @@ bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T,
   std::vector<char> exported((size_t)na, 0);
   std::vector<int32_t> pos((size_t)na, -1);       // position in the point's own block
   std::vector<int32_t> hpos((size_t)na, -1), hblk((size_t)na, -1);
-  std::vector<uint32_t> pairs;                    // (reader, owner) of polled velocities
   std::vector<std::vector<int32_t>> members((size_t)nb);
   for (int b = 0; b < nb; b++) {
     auto reads_other = [&](int p) {
@@ -159,7 +180,6 @@ bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T,
         } else {
           at = ~T.slot_of_point[q];
           exported[q] = 1;
-          pairs.push_back((uint32_t)b * (uint32_t)nb + (uint32_t)owner[q]);
         }
         R.corner[4 * (base + k) + r] = at;
       }
@@ -167,13 +187,6 @@ bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &T,
   }
   for (int p = 0; p < na; p++)
     if (exported[p]) R.str[(size_t)owner[p] * threads + pos[p]] |= kResExport;
-  std::sort(pairs.begin(), pairs.end());
-  pairs.erase(std::unique(pairs.begin(), pairs.end()), pairs.end());
-  for (uint32_t x : pairs)
-    if (!std::binary_search(pairs.begin(), pairs.end(), (x % nb) * (uint32_t)nb + x / nb)) {
-      R = ResidentPlan();
-      return false;
-    }
   return true;
 }
 
@@ -244,6 +257,9 @@ long long verify_resident_plan(const ResidentPlan &R, int na, const int32_t *con
     if (owner[p] < 0) wrong("a point no block owns", -1, p);
     if (exported[p] != wanted[p]) wrong("export mark", owner[p], p);
   }
+  int one_way;
+  if (!inverse_relations(na, nb0, &one_way))
+    wrong("neighbour relations that are not each other's inverse", -1, one_way);
   std::sort(pairs.begin(), pairs.end());
   for (uint64_t x : pairs)
     if (!std::binary_search(pairs.begin(), pairs.end(), (x & 0xffffffffu) << 32 | x >> 32))

@@ -52,9 +52,10 @@ struct ResidentPlan {
 
 // Plan for at most `max_blocks` CTAs from the problem's tile plan (its slots
 // and rebuilt coordinates) and 0-based neighbour vectors.  False where the
-// problem does not fit one point per thread, has no grid layout, or where a
-// block would read from a block that does not read from it (the kernel's
-// two-deep mailboxes need the symmetry; grids have it).
+// problem does not fit the widest blocks, has no grid layout, or where its
+// neighbour relations are not each other's inverse (ee and nw, ne and sw, se
+// and sse; grids' are): the kernels' two-deep mailboxes and their results in
+// place need every wait to be mutual, whichever points a call skips.
 // `quad`: blocks for four lanes per point where the problem is small enough.
 bool build_resident_plan(int na, const int32_t *const nb0[6], const TilePlan &tiles,
                          int max_blocks, ResidentPlan *plan, bool quad = true);

@@ -62,6 +62,21 @@ def test_plan_refuses_what_does_not_fit(shim):
     assert plan(shim, pr)[0] == -1
 
 
+@pytest.mark.parametrize("k", NEIGHBOURS)
+def test_plan_refuses_one_way_relations(shim, k):
+    """One neighbour entry led to a halo slot while the point it named still
+    points back: a mask that leaves only the other points active would make one
+    block wait for a block that does not wait for it."""
+    pr = synth.to_1d(synth.make_grid(64, 48, seed=3, ndte=2))
+    assert plan(shim, pr)[0] == 0
+    listed = np.flatnonzero(pr.idx[k] <= pr.na)
+    for p in listed[[0, len(listed) // 2, -1]]:
+        was = pr.idx[k][p]
+        pr.idx[k][p] = pr.navel
+        assert plan(shim, pr)[0] == -1, (k, p)
+        pr.idx[k][p] = was
+
+
 @pytest.mark.parametrize("plant", [1, 2, 3, 4, 5])
 def test_plan_verifier_catches(shim, plant):
     pr = synth.to_1d(synth.make_grid(131, 77, seed=3, ndte=2))
@@ -121,6 +136,32 @@ def test_same_as_one_launch_per_subcycle(monkeypatch, nx, ny, n):
     for k in ("stress", "uvel", "vvel", "strintx", "strinty", "Cb", "str"):
         a, b = (np.asarray(getattr(f, k)).view(np.int64) for f in got)
         assert np.array_equal(a, b), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mask", ["one point", "half", "sparse"])
+@pytest.mark.parametrize("one_way", [False, True])
+def test_masked_bitwise(oracle_mod, one_way, mask):
+    """Calls that skip most points: on a grid on chip (blocks without an active
+    point beside working ones), on a list with a one-way relation by a launch
+    per subcycle."""
+    from test_gpu_parity import assert_same, oracle_run
+    ndte = 6
+    pr = synth.to_1d(synth.make_grid(64, 48, seed=3, ndte=ndte))
+    w = int(np.flatnonzero((pr.idx["ee"] <= pr.na) & (pr.skipT == 0))[0])
+    if one_way:
+        pr.idx["ee"][w] = pr.navel
+    rng = np.random.default_rng(4)
+    keep = {"one point": np.arange(pr.na) == w, "half": np.arange(pr.na) < pr.na // 2,
+            "sparse": rng.random(pr.na) < 0.05}[mask]
+    pr.skipT[~keep] = 1
+    pr.skipU[~keep] = 1
+    fs = evp1d.FieldSet.from_problem(pr, want_str=True)
+    with evp1d.EVP1D.from_problem(pr, ndte=ndte) as s:
+        s.launch_count(reset=True)
+        s.run(ndte, fs)
+        assert s.launch_count() == (ndte if one_way else 1)
+    assert_same(fs, oracle_run(oracle_mod, pr, ndte), pr)
 
 
 # widths 128, 256, 384, 512 of the reverse kernel; segments of 1, 2 and more subcycles

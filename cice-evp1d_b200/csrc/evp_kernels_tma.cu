@@ -821,6 +821,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       }
     }
     if (__any_sync(0xffffffffu, !ok)) return;
+    __syncwarp();  // every lane's stores come before the arrival
     if (lane == 0) mbar_arrive(&S.strfull[q & 1]);
     if (tid == 0) trace_stamp(a, q, 2);
   }

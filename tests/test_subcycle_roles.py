@@ -3,11 +3,29 @@ themselves, against the oracle, bit for bit (zero tolerance: the same
 operations in the same order).  Sizes: runs of no more than one tile, of two,
 three (every table in use once) and five; all 13 stepu inputs read (general)
 and ten."""
+import os
+import re
+
 import numpy as np
 import pytest
 
 import evp1d
 from evp1d import synth
+
+from conftest import PKG
+
+
+def test_lane_arrivals_follow_a_warp_sync():
+    """Lane 0's arrival on an mbarrier stands for what its whole warp read or
+    wrote: the statement before it is a __syncwarp() (a vote orders no memory).
+    No execution shows the difference reliably, so the source is read."""
+    src = open(os.path.join(PKG, "csrc", "evp_kernels_tma.cu")).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    arrivals = list(re.finditer(r"if \(lane == 0\)\s*(?:\{\s*const[^;]*;\s*)?mbar_arrive", src))
+    assert len(arrivals) >= 5
+    for m in arrivals:
+        before = src[:m.start()].rstrip()
+        assert before.endswith("__syncwarp();"), before[-200:] + m.group()
 
 
 @pytest.mark.gpu

@@ -51,10 +51,11 @@ __global__ void __launch_bounds__(NT, 1) k_resident_adj(ResidentAdjArgs a, Param
   extern __shared__ __align__(16) unsigned char adj_raw[];
   AdjSmem<NT> &S = *reinterpret_cast<AdjSmem<NT> *>(adj_raw);
   const int c = threadIdx.x;
-  const size_t at = (size_t)blockIdx.x * blockDim.x + c;
-  const int slot = a.slot[at];
+  // whole warps: a plan of four lanes a point may have a width that is none
+  const size_t at = (size_t)blockIdx.x * a.width + c;
+  const int slot = c < a.width ? a.slot[at] : -1;
   const bool own = c < a.cnt[blockIdx.x];
-  const uint32_t nbr = a.str_idx[at];
+  const uint32_t nbr = own ? a.str_idx[at] : 0u;
   const uint8_t fl = slot >= 0 ? a.flags[slot] : (uint8_t)(kSkipT | kSkipU);
   const bool actT = !(fl & kSkipT), actU = own && !(fl & kSkipU);
   const bool exported = own && (nbr & kResExport);
@@ -293,10 +294,11 @@ cudaError_t launch_resident_adjoint(const ResidentAdjArgs &given, const Params &
   const AdjVariant *v = find_variant(cls);
   if (!v || nblocks <= 0 || given.nsub < 1) return cudaErrorInvalidValue;
   ResidentAdjArgs a = given;
+  a.width = threads;
   Params pp = p;
   void *args[] = {&a, &pp};
-  return cudaLaunchCooperativeKernel((const void *)v->k, dim3(nblocks), dim3(threads), args,
-                                     v->smem, st);
+  return cudaLaunchCooperativeKernel((const void *)v->k, dim3(nblocks),
+                                     dim3((threads + 31) / 32 * 32), args, v->smem, st);
 }
 
 }  // namespace evp

@@ -225,6 +225,7 @@ cudaError_t launch_resident(const ResidentArgs &a, const Params &p, bool quad, i
 // kResAdjointMax.
 struct ResidentAdjArgs {
   int nslots = 0;
+  int width = 0;  // positions per block (set by launch_resident_adjoint)
   const int32_t *slot = nullptr, *cnt = nullptr, *corner = nullptr;
   const uint32_t *str_idx = nullptr;
   const uint8_t *flags = nullptr;

@@ -196,6 +196,15 @@ def test_reverse_launch_bitwise(monkeypatch, nx, ny, ndte, interval):
         assert np.array_equal(got[0][k].view(np.int64), got[1][k].view(np.int64)), k
 
 
+# four-lane plans whose width is no whole number of warps, on which the reverse
+# kernel, a thread per position, polls by warp votes
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,width", [(131, 77, 56), (150, 110, 88)])
+def test_reverse_launch_bitwise_ragged_width(shim, monkeypatch, nx, ny, width):
+    assert plan(shim, synth.to_1d(synth.make_grid(nx, ny, seed=17, ndte=5)))[1][1] == width
+    test_reverse_launch_bitwise(monkeypatch, nx, ny, 5, 3)
+
+
 # blocks wider than a CTA: the positions beyond its 512 threads take four lanes
 # each, in one pass (400 x 300) or two (440 x 330, 460 x 345: the kernel's end);
 # more than 512 owned points a block (410 x 310 on) take two passes of stepu

@@ -48,8 +48,8 @@
 //
 // Every mbarrier wait is bounded by %globaltimer (kWaitNs): on expiry the warp
 // records an error code and leaves; the waits for its arrivals run out in turn.
-// The bulk warp waits (bounded) for the copies issued before it exits, so
-// nothing is left in flight.
+// Every producer warp waits (bounded) for the slots it has issued copies into
+// before it exits, so nothing is left in flight.
 #include <cstddef>
 #include <cstdint>
 
@@ -609,19 +609,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_tma(TmaArgs a, Params p) {
       }
       issued++;
     }
+    // No copy may target shared memory after the CTA exits: every warp waits
+    // (bounded) for the slots it has issued copies into.  A wait that ran out
+    // in one warp need not have in another: a gather warp can have issued into
+    // a slot that the bulk warp never armed, which holds it here for the limit.
+    // (Without such a failure these waits end before stress does.)
+    for (int k = issued - kSSlots; k < issued; k++)
+      if (k >= 0 && lane == 0)
+        mbar_wait(&S.sfull[k % kSSlots], (uint32_t)(k / kSSlots) & 1, a.err, 3);
     if (pw == 0) {
       if (multi && lane == 0) {
         // the last steps' counters (a later launch zeroes them anyway)
         const unsigned long long t0 = global_ns();
         while (ok && pub < issued && global_ns() - t0 < kWaitNs) publish(issued);
-      }
-      if (!ok) {
-        // Consumers stopped early: wait (bounded) until every issued slot has
-        // landed so that no copy targets shared memory after the CTA exits.
-        for (int k = issued - kSSlots; k < issued; k++) {
-          if (k < 0) continue;
-          if (lane == 0) mbar_wait(&S.sfull[k % kSSlots], (uint32_t)(k / kSSlots) & 1, a.err, 3);
-        }
       }
       // records issued ahead and never consumed must land before exit too
       if (lane == 0) {
@@ -857,7 +857,7 @@ const char *tma_wait_name(int code) {
   switch (code) {
     case 1: return "a consumer waited for a tile's stress inputs";
     case 2: return "the producer waited for a free stress slot";
-    case 3: return "the producer waited for its copies to land after an early stop";
+    case 3: return "the producer waited for its copies to land before it ended";
     case 6: return "the producer waited for a tile record";
     case 7: return "the producer waited for records issued ahead";
     case 8: return "the dynamic shared memory was not 16-byte aligned";

@@ -28,6 +28,20 @@ def test_lane_arrivals_follow_a_warp_sync():
         assert before.endswith("__syncwarp();"), before[-200:] + m.group()
 
 
+def test_every_producer_warp_waits_for_its_copies():
+    """The waits of the four producer warps can run out one without the other, so
+    that a gather warp has copies under way into a slot that the bulk warp
+    neither arms nor waits for: each warp waits for its own slots after its
+    loop, on every path.  Read in the source: no test may leave copies in
+    flight."""
+    src = open(os.path.join(PKG, "csrc", "evp_kernels_tma.cu")).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    tail = re.sub(r"\s+", " ", src[src.index("issued++;"):])
+    assert tail.startswith("issued++; } for (int k = issued - kSSlots; k < issued; k++) "
+                           "if (k >= 0 && lane == 0) mbar_wait(&S.sfull[k % kSSlots], "
+                           "(uint32_t)(k / kSSlots) & 1"), tail[:200]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("general", [False, True])
 @pytest.mark.parametrize("runs,nx,ny", [(148, 3, 2), (148, 131, 77), (16, 131, 77), (10, 131, 77),

@@ -21,6 +21,16 @@ namespace {
 thread_local std::string g_err;
 // allocations left until the injected failure (0: none armed)
 std::atomic<int> g_fail_alloc{0};
+// launches of launch_cooperative left until the injected refusal
+std::atomic<int> g_refuse_launch{0};
+
+// Counts an armed injection down; true for the operation it picks.
+bool injected(std::atomic<int> &left) {
+  int n = left.load();
+  while (n > 0 && !left.compare_exchange_weak(n, n - 1)) {
+  }
+  return n == 1;
+}
 }  // namespace
 
 namespace evp {
@@ -41,14 +51,22 @@ int timeout_error(int code) {
 }
 
 cudaError_t device_alloc(void **p, size_t bytes) {
-  int n = g_fail_alloc.load();
-  while (n > 0 && !g_fail_alloc.compare_exchange_weak(n, n - 1)) {
-  }
-  if (n == 1) {
+  if (injected(g_fail_alloc)) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
   return cudaMalloc(p, bytes);
+}
+
+cudaError_t launch_cooperative(const void *kernel, dim3 grid, dim3 block, void **args,
+                               size_t smem, cudaStream_t st) {
+  if (injected(g_refuse_launch)) return cudaErrorCooperativeLaunchTooLarge;
+  return cudaLaunchCooperativeKernel(kernel, grid, block, args, smem, st);
+}
+
+bool launch_refused(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources ||
+         e == cudaErrorNotSupported;
 }
 }  // namespace evp
 
@@ -616,11 +634,17 @@ int run_subcycles(evp1d_t *h, int ndte, bool ends) {
     // subcycle had been a launch of its own
     DeviceProblem &d = h->d;
     const int c = d.cur, to = (ndte & 1) ? 1 - c : c;
-    CUDA_TRY(evp::problem_launch_resident(&d, h->p, ndte, ends, d.stress[c], d.stress[to], d.u[c],
-                                          d.v[c], d.u[to], d.v[to], 0));
-    d.cur = to;
-    h->launches++;
-    return EVP1D_OK;
+    const cudaError_t e = evp::problem_launch_resident(&d, h->p, ndte, ends, d.stress[c],
+                                                       d.stress[to], d.u[c], d.v[c], d.u[to],
+                                                       d.v[to], 0);
+    if (!evp::launch_refused(e)) {
+      CUDA_TRY(e);
+      d.cur = to;
+      h->launches++;
+      return EVP1D_OK;
+    }
+    cudaGetLastError();
+    h->resident = false;
   }
   if (h->path == kPathTma && h->persist && ndte > 1) {
     // the whole call in one launch; the per-tile counters start at zero
@@ -798,6 +822,12 @@ int evp1d_debug_dep_wait_timeout(evp1d_t *h, long long ns) {
 int evp1d_debug_fail_alloc(int n) {
   if (n < 0) return fail(EVP1D_ERR_INVALID_ARG, "n = %d < 0", n);
   g_fail_alloc.store(n);
+  return EVP1D_OK;
+}
+
+int evp1d_debug_refuse_launch(int n) {
+  if (n < 0) return fail(EVP1D_ERR_INVALID_ARG, "n = %d < 0", n);
+  g_refuse_launch.store(n);
   return EVP1D_OK;
 }
 

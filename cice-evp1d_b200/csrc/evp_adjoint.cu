@@ -555,22 +555,26 @@ void launch_state(evp1d_t *h, double *const s_in[12], double *const s_out[12],
 
 // `len` forward subcycles from tape entry e0: the velocities of subcycle i go
 // into entry e0 + i + 1, the stresses alternate between s0 and s1 (s0 holds
-// the start).  One multi-subcycle launch where the handle runs those, else one
-// launch per subcycle.
-void launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], double *tu0,
+// the start).  One resident or multi-subcycle launch where the handle runs
+// those, else one launch per subcycle.
+cudaError_t launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], double *tu0,
                    double *tv0, size_t entry_step, int len, bool last);
 
 double *tape_u(AdjointState &A, int e) { return A.tape + (size_t)e * 2 * A.stride; }
 
-void launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], double *tu0,
-                   double *tv0, size_t entry_step, int len, bool last) {
+cudaError_t launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], double *tu0,
+                          double *tv0, size_t entry_step, int len, bool last) {
   DeviceProblem &d = h->d;
-  if (len <= 0) return;
+  if (len <= 0) return cudaSuccess;
   if (use_resident(h, len)) {
-    problem_launch_resident(&d, h->p, len, last, s0, (len & 1) ? s1 : s0, tu0, tv0, tu0, tv0,
-                            entry_step);
-    h->launches++;
-    return;
+    const cudaError_t e = problem_launch_resident(&d, h->p, len, last, s0, (len & 1) ? s1 : s0,
+                                                  tu0, tv0, tu0, tv0, entry_step);
+    if (!launch_refused(e)) {
+      h->launches++;
+      return e;
+    }
+    cudaGetLastError();
+    h->resident = false;
   }
   if (h->path == kPathTma && h->persist && len > 1) {
     cudaMemsetAsync(d.epoch, 0, sizeof(unsigned) * (size_t)d.ntiles, d.stream);
@@ -585,9 +589,8 @@ void launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], doubl
     a.nsub = len;
     a.last = last;
     a.epoch = d.epoch;
-    launch_tma(a, h->p, d.stream);
     h->launches++;
-    return;
+    return launch_tma(a, h->p, d.stream);
   }
   for (int i = 0; i < len; i++) {
     const bool odd = i & 1;
@@ -596,6 +599,7 @@ void launch_states(evp1d_t *h, double *const s0[12], double *const s1[12], doubl
                  tv0 + (size_t)(i + 1) * entry_step, last && i == len - 1, i > 0);
   }
   h->launches += len;
+  return cudaGetLastError();
 }
 
 double *tape_v(AdjointState &A, int e) { return A.tape + (size_t)e * 2 * A.stride + A.stride; }
@@ -722,8 +726,8 @@ int evp1d_record_subcycles(evp1d_t *h, int ndte, int interval) {
                             cudaMemcpyDeviceToDevice, st));
     ADJ_TRY(cudaMemcpyAsync(tape_v(A, 0), d.v[c], sizeof(double) * d.nuv,
                             cudaMemcpyDeviceToDevice, st));
-    launch_states(h, d.stress[c], d.stress[1 - c], tape_u(A, 0), tape_v(A, 0), 2 * A.stride,
-                  ndte - n_cp, true);
+    ADJ_TRY(launch_states(h, d.stress[c], d.stress[1 - c], tape_u(A, 0), tape_v(A, 0),
+                          2 * A.stride, ndte - n_cp, true));
     const int b = ((ndte - n_cp) & 1) ? 1 - c : c;
     // the final state back into the handle's buffers for evp1d_download
     ADJ_TRY(cudaMemcpyAsync(d.u[b], tape_u(A, ndte - n_cp), sizeof(double) * d.nslots,
@@ -869,9 +873,15 @@ int evp1d_adjoint_sweep(evp1d_t *h) {
       r.seq = d.res_seq;
       r.err = d.err;
       d.res_seq += (unsigned)len;
-      keep(launch_resident_adjoint(r, h->p, d.res_cls, d.res_threads, d.res_blocks, st));
-      launches++;
-      return;
+      const cudaError_t e =
+          launch_resident_adjoint(r, h->p, d.res_cls, d.res_threads, d.res_blocks, st);
+      if (!launch_refused(e)) {
+        keep(e);
+        launches++;
+        return;
+      }
+      cudaGetLastError();
+      h->resident = false;
     }
     for (int i = len - 1; i >= 0; i--)
       reverse_step(tape_u(A, e0 + i), tape_v(A, e0 + i), tape_u(A, e0 + i + 1),
@@ -902,8 +912,8 @@ int evp1d_adjoint_sweep(evp1d_t *h) {
     const bool end_stored = j + 1 < A.nck || A.n_cp < A.ndte;
     const int nrec = end_stored ? len - 1 : len;
     const long long before = h->launches;
-    launch_states(h, A.spp[0], A.spp[1], tape_u(A, e0), tape_v(A, e0), 2 * A.stride, nrec,
-                  false);
+    keep(launch_states(h, A.spp[0], A.spp[1], tape_u(A, e0), tape_v(A, e0), 2 * A.stride, nrec,
+                       false));
     launches += h->launches - before;
     h->launches = before;
     if (end_stored) {

@@ -28,8 +28,7 @@
 #include <cstdint>
 
 #include "evp_adjoint_math.cuh"
-#include "evp_kernels.cuh"
-#include "evp_resident.h"
+#include "evp_internal.h"
 #include "evp_resident_mail.cuh"
 
 namespace evp {
@@ -297,8 +296,8 @@ cudaError_t launch_resident_adjoint(const ResidentAdjArgs &given, const Params &
   a.width = threads;
   Params pp = p;
   void *args[] = {&a, &pp};
-  return cudaLaunchCooperativeKernel((const void *)v->k, dim3(nblocks),
-                                     dim3((threads + 31) / 32 * 32), args, v->smem, st);
+  return launch_cooperative((const void *)v->k, dim3(nblocks), dim3((threads + 31) / 32 * 32), args,
+                            v->smem, st);
 }
 
 }  // namespace evp

@@ -42,7 +42,8 @@ struct evp1d_handle {
   // (cooperative), instead of one launch per subcycle in CUDA graphs
   bool persist = false;
   // TMA path: calls of at least kResidentMin subcycles in one launch that
-  // keeps the state on chip (d.res_blocks > 0)
+  // keeps the state on chip (d.res_blocks > 0); false once such a launch was
+  // refused
   bool resident = false;
   // TMA path: each subcycle's launch after the first of a call (and of a
   // captured chunk) is a programmatic dependent of the one before, so that

@@ -38,6 +38,13 @@ cudaError_t device_alloc(T **p, size_t bytes) {
   return device_alloc(reinterpret_cast<void **>(p), bytes);
 }
 
+// A launch whose blocks wait on one another, so all must be resident at once.
+// Refused (launch_refused of its result; nothing has been launched) where less
+// of the device is free to this context, and by evp1d_debug_refuse_launch.
+cudaError_t launch_cooperative(const void *kernel, dim3 grid, dim3 block, void **args,
+                               size_t smem, cudaStream_t st);
+bool launch_refused(cudaError_t e);
+
 // Per-call input fields in the order they are staged and scattered.
 enum DynField {
   kStrength, kCw, kAiu, kUocn, kVocn, kWaterx, kWatery, kForcex, kForcey,
@@ -167,7 +174,7 @@ FusedArgs problem_fused_args(const DeviceProblem &d, int from);
 TmaArgs problem_tma_args(const DeviceProblem &d, int from);
 // One resident launch of nsub subcycles from the state (u_in, v_in, s_in) to
 // s_out and, uv_step == 0, (u_out, v_out); see ResidentArgs.  Takes nsub
-// mailbox numbers.
+// mailbox numbers (a refused launch too, which changes nothing else).
 cudaError_t problem_launch_resident(DeviceProblem *d, const Params &p, int nsub, bool last,
                                     double *const s_in[12], double *const s_out[12],
                                     const double *u_in, const double *v_in, double *u_out,

@@ -50,8 +50,7 @@
 #include <algorithm>
 #include <cstdint>
 
-#include "evp_kernels.cuh"
-#include "evp_resident.h"
+#include "evp_internal.h"
 #include "evp_resident_mail.cuh"
 
 namespace evp {
@@ -617,8 +616,9 @@ cudaError_t launch_resident(const ResidentArgs &given, const Params &p, bool qua
   a.width = threads;
   Params pp = p;
   void *args[] = {&a, &pp};
-  return cudaLaunchCooperativeKernel((const void *)v->k[std_params(p) ? 1 : 0], dim3(nblocks),
-                                     dim3(quad ? 4 * threads : std::min(threads, v->threads)), args, v->smem, st);
+  return launch_cooperative((const void *)v->k[std_params(p) ? 1 : 0], dim3(nblocks),
+                            dim3(quad ? 4 * threads : std::min(threads, v->threads)), args,
+                            v->smem, st);
 }
 
 }  // namespace evp

@@ -375,8 +375,8 @@ bool launch_na_run(const NaArgs &given, const Params &given_p, int ndte, int *st
   void *args[] = {&a, &p, &ndte, &status};
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess ||
-      cudaLaunchCooperativeKernel(k, dim3(one ? blocks : (blocks < sms ? blocks : sms)), dim3(kRunThreads), args, smem,
-                                  st) != cudaSuccess) {
+      launch_cooperative(k, dim3(one ? blocks : (blocks < sms ? blocks : sms)), dim3(kRunThreads),
+                         args, smem, st) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -155,6 +155,12 @@ def debug_fail_alloc(n: int) -> None:
     check(_lib.load().evp1d_debug_fail_alloc(int(n)), "evp1d_debug_fail_alloc")
 
 
+def debug_refuse_launch(n: int) -> None:
+    """Host-side fault injection (evp1d_debug_refuse_launch): the n-th launch
+    from now on whose blocks must all be resident is refused; 0 disarms."""
+    check(_lib.load().evp1d_debug_refuse_launch(int(n)), "evp1d_debug_refuse_launch")
+
+
 def plan_check(na: int, navel: int, idx: dict) -> None:
     """Build the tile plan for these 1-based neighbour vectors and verify
     every index the kernels gather through (evp1d_plan_check; host only).

@@ -135,6 +135,8 @@ def load() -> C.CDLL:
     L.evp1d_get_tile_points.restype = C.c_int
     L.evp1d_debug_fail_alloc.argtypes = [C.c_int]
     L.evp1d_debug_fail_alloc.restype = C.c_int
+    L.evp1d_debug_refuse_launch.argtypes = [C.c_int]
+    L.evp1d_debug_refuse_launch.restype = C.c_int
     L.evp1d_exchange_setup.argtypes = [H, C.c_int, _I, C.c_int, _I]
     L.evp1d_exchange_pack.argtypes = [H, C.c_void_p]
     L.evp1d_exchange_unpack.argtypes = [H, C.c_void_p]

@@ -194,6 +194,13 @@ int evp1d_debug_dep_wait_timeout(evp1d_t *handle, long long ns);
  * instead (integration/ice_dyn_evp1d.F90:394-460). */
 int evp1d_debug_fail_alloc(int n);
 
+/* Debug: host-side injection of a refused launch.  The n-th launch after this
+ * call (1 = the next one) whose blocks must all be resident at once is refused
+ * as if less of the device were free to this context: nothing is launched, and
+ * the call goes on with a launch per subcycle, with the same results.  0
+ * disarms.  Process-wide.  No counterpart in the reference. */
+int evp1d_debug_refuse_launch(int n);
+
 /* Debug: timing trace of the TMA kernel's block 0 in the last launch
  * (recorded only when EVP1D_TRACE is set at evp1d_init).  Up to 256 tiles x 8
  * %globaltimer stamps (ns): [0] the bulk-copy warp is done with the tile,

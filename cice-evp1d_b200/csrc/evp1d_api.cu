@@ -819,6 +819,20 @@ int evp1d_debug_dep_wait_timeout(evp1d_t *h, long long ns) {
   return EVP1D_OK;
 }
 
+int evp1d_debug_mail_wait_timeout(evp1d_t *h, long long ns) {
+  if (!h) return fail(EVP1D_ERR_INVALID_ARG, "NULL handle");
+  if (ns < 1000000 || ns > 1000000000)
+    return fail(EVP1D_ERR_INVALID_ARG, "wait limit %lld ns outside [1e6, 1e9]", ns);
+  if (h->d.res_blocks == 0) return fail(EVP1D_ERR_STATE, "the problem has no mailboxes");
+  CUDA_TRY(cudaSetDevice(h->d.device));
+  // a number of no message, which the next launch's do not reach either
+  const unsigned seq = h->d.res_seq - 1u + 0x80000000u;
+  evp::launch_mail_probe(h->d.err, h->d.res_mail, h->d.nslots, seq, (unsigned long long)ns,
+                         h->d.stream);
+  CUDA_TRY(cudaGetLastError());
+  return EVP1D_OK;
+}
+
 int evp1d_debug_fail_alloc(int n) {
   if (n < 0) return fail(EVP1D_ERR_INVALID_ARG, "n = %d < 0", n);
   g_fail_alloc.store(n);

@@ -216,6 +216,10 @@ struct ResidentArgs {
 // whether `nblocks` of its CTAs are resident at once (1) or the plan cannot run
 // here (0).  `threads`: the plan's, compute positions per block.
 int resident_prepare(int device, bool quad, int cls, int nblocks);
+// Queue the two mailbox waits for messages numbered `seq`, which nobody sends,
+// limited to limit_ns each: error word, kMailProbeCode.
+void launch_mail_probe(int *err, const double4 *mail, int nslots, unsigned seq,
+                       unsigned long long limit_ns, cudaStream_t st);
 cudaError_t launch_resident(const ResidentArgs &a, const Params &p, bool quad, int cls, int threads,
                             int nblocks, cudaStream_t st);
 

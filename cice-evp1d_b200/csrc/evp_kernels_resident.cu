@@ -113,27 +113,8 @@ __device__ __forceinline__ double2 quad_velocity(const double2 *uv, const Reside
   double2 w = make_double2(0.0, 0.0);
   const bool wait = act && sub > 0 && ref < 0 && ~ref < a.nslots;
   if (act && !wait) w = ref >= 0 ? uv[ref] : make_double2(a.u_in[~ref], a.v_in[~ref]);
-  const unsigned seq = a.seq + (unsigned)sub;
   const double4 *box = a.mail + (size_t)(sub & 1) * (size_t)a.nslots + (wait ? ~ref : 0);
-  bool left = wait;
-  unsigned long long t0 = 0;
-  for (unsigned tries = 1; __any_sync(0xffffffffu, left); tries++) {
-    if (left) {
-      const Mail m = mail_get(box);
-      if (mail_is(m, seq)) {
-        w = mail_value(m);
-        left = false;
-      }
-    }
-    if ((tries & 63u) == 0) {
-      const unsigned long long t = res_ns();
-      if (t0 == 0) t0 = t;
-      if (__any_sync(0xffffffffu, t - t0 > kResWaitNs)) {
-        fail = fail || left;
-        break;
-      }
-    }
-  }
+  fail |= mail_wait_one(w, box, wait, a.seq + (unsigned)sub);
   return w;
 }
 
@@ -574,6 +555,21 @@ const ResVariant kVariants[] = {variant<128, 0>(), variant<256, 0>(), variant<38
                                 variant<kResMaxThreads, kResMaxWidth - kResMaxThreads>()};
 static_assert(sizeof(ResSmem<kResMaxThreads, kResMaxWidth - kResMaxThreads>) <= 227 * 1024, "shared memory per block");
 
+// One warp waits, as the resident kernels do, for messages that nobody sends:
+// lane l's velocities are those of slots 0 .. nslots - 1 in turn.  Both forms of
+// the wait must run out.
+__global__ void k_mail_probe(int *err, const double4 *mail, int nslots, unsigned seq,
+                             unsigned long long limit_ns) {
+  const int l = threadIdx.x;
+  int ref[4];
+  for (int k = 0; k < 4; k++) ref[k] = ~((4 * l + k) % nslots);
+  Mail m[4];
+  const bool came = mail_wait(m, mail, ref, l < 8 ? 15u : 0u, seq, limit_ns);
+  double2 w = make_double2(0.0, 0.0);
+  const bool out = mail_wait_one(w, mail + ~ref[0], l < 8, seq, limit_ns);
+  if (!came && out) atomicMax(err, kMailProbeCode);
+}
+
 // The class of a quad plan is kQuadMaxWidth, of four threads a point.
 const ResVariant kQuad = {kQuadMaxWidth, 4 * kQuadMaxWidth,
                           {k_resident_quad<4 * kQuadMaxWidth, false>,
@@ -588,6 +584,11 @@ const ResVariant *find_variant(bool quad, int cls) {
 }
 
 }  // namespace
+
+void launch_mail_probe(int *err, const double4 *mail, int nslots, unsigned seq,
+                       unsigned long long limit_ns, cudaStream_t st) {
+  k_mail_probe<<<1, 32, 0, st>>>(err, mail, nslots, seq, limit_ns);
+}
 
 int resident_prepare(int device, bool quad, int cls, int nblocks) {
   const ResVariant *v = find_variant(quad, cls);

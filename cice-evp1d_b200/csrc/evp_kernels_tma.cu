@@ -54,6 +54,7 @@
 #include <cstdint>
 
 #include "evp_kernels.cuh"
+#include "evp_resident_mail.cuh"
 #include "evp_tiles.h"
 
 namespace evp {
@@ -865,7 +866,8 @@ const char *tma_wait_name(int code) {
     case 16: return "stepu waited for a tile's stress";
     case 17: return "stress waited for stepu to read the str tables";
     case 13: return "the producer waited for neighbouring tiles to finish a subcycle";
-    case 15: return "a resident block waited for another block's velocities";
+    case kResCode: return "a resident block waited for another block's velocities";
+    case kMailProbeCode: return "the mailbox-wait probe (evp1d_debug_mail_wait_timeout)";
     case kProbeCode: return "the wait probe (evp1d_debug_wait_timeout)";
     case kDepProbeCode: return "the dependency-wait probe (evp1d_debug_dep_wait_timeout)";
     default: return "unknown";

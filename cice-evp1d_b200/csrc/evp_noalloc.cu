@@ -145,15 +145,16 @@ __device__ __forceinline__ unsigned long long na_ns() {
   return t;
 }
 
-// Every block of the (cooperative) grid has reached its barrier number `k`
-// (1, 2, ...) and what its threads wrote before is visible at L2.  Bounded:
+// Each of the (cooperative) grid's `blocks` blocks has reached its barrier number
+// `k` (1, 2, ...) and what its threads wrote before is visible at L2.  Bounded:
 // false, for the whole block, when the wait ran out.
-__device__ __forceinline__ bool grid_barrier(int *status, unsigned k) {
+__device__ __forceinline__ bool grid_barrier(int *status, unsigned k, unsigned blocks = gridDim.x,
+                                             unsigned long long limit_ns = kRunWaitNs) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned *count = reinterpret_cast<unsigned *>(status) + 2;
-    const unsigned need = k * gridDim.x;
+    const unsigned need = k * blocks;
     __threadfence();
     atomicAdd(count, 1u);
     int good = 1;
@@ -165,7 +166,7 @@ __device__ __forceinline__ bool grid_barrier(int *status, unsigned k) {
       if ((tries & 63u) == 0) {
         const unsigned long long t = na_ns();
         if (t0 == 0) t0 = t;
-        if (t - t0 > kRunWaitNs) {
+        if (t - t0 > limit_ns) {
           status[1] = 1;
           good = 0;
           break;
@@ -176,6 +177,11 @@ __device__ __forceinline__ bool grid_barrier(int *status, unsigned k) {
   }
   __syncthreads();
   return ok != 0;
+}
+
+// A barrier of two blocks at which one arrives.
+__global__ void k_na_barrier_probe(int *status, unsigned long long limit_ns) {
+  grid_barrier(status, 1, 2, limit_ns);
 }
 
 // Velocities and str of other points are read past L1 (__ldcg): other blocks
@@ -439,6 +445,17 @@ Params kernel_params(const evp1d_params &q) {
   return p;
 }
 
+// Waits for the stream; EVP1D_ERR_TIMEOUT where a barrier has run out.
+int check_barriers(const int *status, cudaStream_t st) {
+  int ran_out = 0;
+  NA_TRY(cudaMemcpyAsync(&ran_out, status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  NA_TRY(cudaStreamSynchronize(st));
+  if (ran_out)
+    return error(EVP1D_ERR_TIMEOUT, "a bounded device-side wait ran out (a barrier over the "
+                 "grid); the results of this call are not valid");
+  return EVP1D_OK;
+}
+
 int grid_for(int n) {
   const int b = (n + kThreads - 1) / kThreads;
   return b < 1 ? 1 : b;
@@ -577,12 +594,20 @@ extern "C" int evp1d_run_device_noalloc(int na, int navel, const int32_t *ee,
     if (io->str[k])
       NA_TRY(cudaMemcpyAsync(io->str[k], a.str[k], sizeof(double) * navel,
                              cudaMemcpyDeviceToDevice, st));
-  int ran_out = 0;
-  if (run)
-    NA_TRY(cudaMemcpyAsync(&ran_out, status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-  NA_TRY(cudaStreamSynchronize(st));
-  if (ran_out)
-    return error(EVP1D_ERR_TIMEOUT, "a bounded device-side wait ran out (a barrier over the "
-                 "grid); the results of this call are not valid");
-  return EVP1D_OK;
+  return check_barriers(status, st);  // (0 where the pairs of kernels ran)
+}
+
+extern "C" int evp1d_debug_grid_wait_timeout(long long ns, void *stream) {
+  using namespace evp;
+  if (ns < 1000000 || ns > 1000000000)
+    return error(EVP1D_ERR_INVALID_ARG, "wait limit %lld ns outside [1e6, 1e9]", ns);
+  double *scratch = nullptr;
+  int *status = nullptr;
+  const int rc = scratch_in_context(&scratch, &status);
+  if (rc != EVP1D_OK) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  NA_TRY(cudaMemsetAsync(status + 1, 0, 2 * sizeof(int), st));
+  k_na_barrier_probe<<<1, 32, 0, st>>>(status, (unsigned long long)ns);
+  NA_TRY(cudaGetLastError());
+  return check_barriers(status, st);
 }

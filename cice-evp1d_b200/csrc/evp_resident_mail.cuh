@@ -8,6 +8,7 @@ namespace evp {
 
 constexpr unsigned long long kResWaitNs = 2000000000ull;  // 2 s
 constexpr int kResCode = 15;
+constexpr int kMailProbeCode = 19;  // evp1d_debug_mail_wait_timeout
 
 // Two doubles of one point, each 32-bit half beside the message's number.
 __device__ __forceinline__ void mail_put(double4 *box, double u, double v, unsigned seq) {
@@ -65,7 +66,8 @@ __device__ __forceinline__ unsigned long long res_ns() {
 // a warp whose lanes left one by one would go through what follows in as many
 // parts.  Returns false in every lane when the wait ran out.
 __device__ __forceinline__ bool mail_wait(Mail (&m)[4], const double4 *box, const int (&ref)[4],
-                                          unsigned polled, unsigned seq) {
+                                          unsigned polled, unsigned seq,
+                                          unsigned long long limit_ns = kResWaitNs) {
   unsigned left = polled;
   unsigned long long t0 = 0;
   for (unsigned tries = 1; __any_sync(0xffffffffu, left != 0); tries++) {
@@ -78,10 +80,33 @@ __device__ __forceinline__ bool mail_wait(Mail (&m)[4], const double4 *box, cons
     if ((tries & 63u) == 0) {
       const unsigned long long t = res_ns();
       if (t0 == 0) t0 = t;
-      if (__any_sync(0xffffffffu, t - t0 > kResWaitNs)) return false;
+      if (__any_sync(0xffffffffu, t - t0 > limit_ns)) return false;
     }
   }
   return true;
+}
+
+// The same for at most one mailbox a lane (`left`: it waits for its own, whose
+// velocity goes to `w`).  Returns true in the lanes whose wait ran out.
+__device__ __forceinline__ bool mail_wait_one(double2 &w, const double4 *box, bool left,
+                                              unsigned seq,
+                                              unsigned long long limit_ns = kResWaitNs) {
+  unsigned long long t0 = 0;
+  for (unsigned tries = 1; __any_sync(0xffffffffu, left); tries++) {
+    if (left) {
+      const Mail m = mail_get(box);
+      if (mail_is(m, seq)) {
+        w = mail_value(m);
+        left = false;
+      }
+    }
+    if ((tries & 63u) == 0) {
+      const unsigned long long t = res_ns();
+      if (t0 == 0) t0 = t;
+      if (__any_sync(0xffffffffu, t - t0 > limit_ns)) break;
+    }
+  }
+  return left;
 }
 
 }  // namespace evp

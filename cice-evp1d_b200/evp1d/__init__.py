@@ -445,6 +445,13 @@ class EVP1D:
         check(self._L.evp1d_debug_dep_wait_timeout(self.h, int(ns)),
               "evp1d_debug_dep_wait_timeout")
 
+    def debug_mail_wait_timeout(self, ns: int) -> None:
+        """Queue the bounded waits of a resident launch, for messages nobody
+        sends (evp1d_debug_mail_wait_timeout): the next synchronize raises the
+        timeout."""
+        check(self._L.evp1d_debug_mail_wait_timeout(self.h, int(ns)),
+              "evp1d_debug_mail_wait_timeout")
+
     @property
     def path(self) -> str:
         """Name of the kernel path the library runs."""

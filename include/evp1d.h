@@ -186,6 +186,19 @@ int evp1d_debug_wait_timeout(evp1d_t *handle, long long ns);
  * naming it.  No counterpart in the reference. */
 int evp1d_debug_dep_wait_timeout(evp1d_t *handle, long long ns);
 
+/* Debug: the same for the waits of a resident launch (a call's subcycles on
+ * chip, problems of up to about 98k points; EVP1D_ERR_STATE for other handles),
+ * whose blocks wait for one another's velocities in mailboxes: both forms of
+ * the wait, for messages that nobody sends, limited to `ns` nanoseconds each
+ * (1e6 to 1e9). */
+int evp1d_debug_mail_wait_timeout(evp1d_t *handle, long long ns);
+
+/* Debug: the same for the barrier over the grid of evp1d_run_device_noalloc: a
+ * barrier at which one block of two arrives, limited to `ns` nanoseconds (1e6 to
+ * 1e9).  Waits for it and returns what that call returns then,
+ * EVP1D_ERR_TIMEOUT. */
+int evp1d_debug_grid_wait_timeout(long long ns, void *stream);
+
 /* Debug: host-side injection of an out-of-memory failure.  The n-th device
  * allocation of the library after this call (1 = the next one) fails as if
  * the device were full: it allocates nothing, and the call that made it

@@ -186,6 +186,13 @@ cudaError_t launch_tma(const TmaArgs &a, const Params &p, cudaStream_t st);
 // with one CTA per run resident on every SM).
 bool tma_can_persist(int device, int nruns);
 
+// Whether a barrier's running count of arrivals, modulo 2^32, has reached `need`:
+// it is never further from it than one barrier's blocks (148 blocks, two barriers
+// a subcycle, pass 2^32 after 14.5 million subcycles).
+__host__ __device__ __forceinline__ bool barrier_complete(unsigned count, unsigned need) {
+  return (int)(count - need) >= 0;
+}
+
 // ---- a call's subcycles in one launch, state on chip (evp_kernels_resident.cu)
 struct ResidentArgs {
   int nslots = 0;

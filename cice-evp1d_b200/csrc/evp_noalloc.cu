@@ -154,7 +154,7 @@ __device__ __forceinline__ bool grid_barrier(int *status, unsigned k, unsigned b
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned *count = reinterpret_cast<unsigned *>(status) + 2;
-    const unsigned need = k * blocks;
+    const unsigned need = k * blocks;  // as the count, modulo 2^32
     __threadfence();
     atomicAdd(count, 1u);
     int good = 1;
@@ -162,7 +162,7 @@ __device__ __forceinline__ bool grid_barrier(int *status, unsigned k, unsigned b
     for (unsigned tries = 1;; tries++) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-      if (v >= need) break;
+      if (barrier_complete(v, need)) break;
       if ((tries & 63u) == 0) {
         const unsigned long long t = na_ns();
         if (t0 == 0) t0 = t;

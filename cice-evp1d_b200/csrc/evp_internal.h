@@ -73,6 +73,7 @@ struct DeviceProblem {
   // page-locked copy of the error word (pinned_word; null: none was left)
   int *err_host = nullptr;
   bool pins = false;        // holds a reference to the page-locked pool
+  unsigned pin_gen = 0;     // as it was then
   int32_t *nb[6] = {};  // ee ne se nw sw sse, slot space
   uint32_t *lnb = nullptr;   // static packed stepu neighbours
   uint32_t *meta = nullptr;  // lnb | skip flags << 30 (per call)

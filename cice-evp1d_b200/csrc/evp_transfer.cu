@@ -204,6 +204,7 @@ PtrAttrs ptr_attrs() {
 struct PinnedPool {
   static constexpr int kWords = 1024;
   std::mutex m;
+  unsigned gen = 0;  // counts the pool's memory: handles of an older one hold nothing
   int refs = 0;
   int *words = nullptr;
   bool used[kWords] = {};
@@ -241,8 +242,22 @@ void return_stage() {
 void pinned_hold(DeviceProblem *d) {
   PinnedPool &p = pool();
   std::lock_guard<std::mutex> lock(p.m);
+  // A reset of the device (cudaDeviceReset) takes the memory away from under
+  // handles that were not finalized: the pool starts anew.
+  cudaPointerAttributes at;
+  if (p.words && (cudaPointerGetAttributes(&at, p.words) != cudaSuccess ||
+                  at.type != cudaMemoryTypeHost)) {
+    cudaGetLastError();
+    p.gen++;
+    p.refs = 0;
+    p.words = nullptr;
+    p.stage = nullptr;
+    p.lent = false;
+    for (bool &u : p.used) u = false;
+  }
   p.refs++;
   d->pins = true;
+  d->pin_gen = p.gen;
   if (!p.words && cudaHostAlloc((void **)&p.words, sizeof(int) * PinnedPool::kWords,
                                 cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
@@ -262,6 +277,7 @@ void pinned_release(DeviceProblem *d) {
   PinnedPool &p = pool();
   std::lock_guard<std::mutex> lock(p.m);
   d->pins = false;
+  if (d->pin_gen != p.gen) return;
   if (d->err_host) p.used[d->err_host - p.words] = false;
   d->err_host = nullptr;
   if (--p.refs > 0) return;

@@ -601,6 +601,7 @@ int upload_fields(evp1d_handle *h, const evp1d_fields *io, bool wait) {
     CHECK(problem_upload(&d, f, h->p.rhow, wait));
   }
   h->uploaded = true;
+  h->sets_differ = false;
   return EVP1D_OK;
 }
 
@@ -612,7 +613,7 @@ int settle(evp1d_handle *h, int rc) {
 }
 
 bool use_resident(const evp1d_handle *h, int n) {
-  if (h->path != kPathTma || !h->resident || n < kResidentMin) return false;
+  if (h->path != kPathTma || !h->resident || h->sets_differ || n < kResidentMin) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(h->d.stream, &cs) == cudaSuccess &&
          cs == cudaStreamCaptureStatusNone;

@@ -156,6 +156,7 @@ int evp1d_dyn_run(evp1d_dyn_t *d, int ndte, const evp1d_dyn_fields *io) {
   int rc = evp::settle(h, evp::problem_upload(&P, f, h->p.rhow, false));
   if (rc != EVP1D_OK) return rc;
   h->uploaded = true;
+  h->sets_differ = false;
   rc = evp::settle(h, evp1d_subcycles(h, ndte));
   if (rc != EVP1D_OK) return rc;
   int code = 0;

@@ -154,6 +154,7 @@ int evp1d_exchange_unpack(evp1d_t *h, const double *buf) {
   k_exchange_unpack<<<blocks_for(h->nrecv), kBlock, 0, h->d.stream>>>(
       h->nrecv, h->xpos + h->nsend, buf, h->d.u[c], h->d.v[c]);
   h->launches++;
+  h->sets_differ = true;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? EVP1D_OK : cuda_fail(e, "k_exchange_unpack");
 }

@@ -26,7 +26,10 @@ int settle(evp1d_handle *h, int rc);
 constexpr int kResidentMin = 2;
 // Whether a call of n subcycles, queued now on the handle's stream, takes the
 // resident launch.  Not under stream capture: its mailbox numbers are launch
-// arguments, and a replay would find the previous replay's messages.
+// arguments, and a replay would find the previous replay's messages.  Not after
+// an evp1d_exchange_unpack either: a point that the subcycles do not write then
+// has one velocity in each buffer set, which subcycle after subcycle reads in
+// turn, where a resident launch knows the first alone.
 bool use_resident(const evp1d_handle *h, int n);
 }  // namespace evp
 
@@ -52,6 +55,7 @@ struct evp1d_handle {
   bool pdl = true;
   long long *trace = nullptr;  // device timing trace (EVP1D_TRACE, debug)
   bool uploaded = false;
+  bool sets_differ = false;  // velocities received since the upload
   bool uinit_explicit = false;  // the last upload gave uvel_init/vvel_init
   long long launches = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // by starting buffer

@@ -164,6 +164,36 @@ def test_masked_bitwise(oracle_mod, one_way, mask):
     assert_same(fs, oracle_run(oracle_mod, pr, ndte), pr)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3])
+def test_after_an_exchange(monkeypatch, n):
+    """Received velocities are those of the current state: points that a
+    subcycle does not write keep others in the second buffer set.  Several
+    subcycles after an unpack give what a launch per subcycle gives."""
+    import torch
+    pr = synth.to_1d(synth.make_grid(64, 48, seed=6, ndte=n, curvilinear=True))
+    still = 1 + np.concatenate([np.flatnonzero(pr.skipU), np.arange(pr.na, pr.navel)])
+    buf = torch.from_numpy(np.random.default_rng(1).normal(0.0, 0.1, 2 * len(still))).cuda()
+    got = []
+    for resident in ("1", "0"):
+        monkeypatch.setenv("EVP1D_RESIDENT", resident)
+        fs = evp1d.FieldSet.from_problem(pr, want_str=True)
+        with evp1d.EVP1D.from_problem(pr, ndte=n) as s:
+            s.exchange_setup([1], still.tolist())
+            s.upload(fs)
+            s.subcycles_inner(2)
+            s.exchange_unpack(buf.data_ptr())
+            s.subcycles_inner(n)
+            s.subcycles(n)
+            s.download(fs)
+            got.append([np.array(getattr(fs, k)) for k in ("stress", "uvel", "vvel", "strintx", "str")])
+            s.launch_count(reset=True)
+            s.run(n, fs)  # an upload makes the sets equal again
+            assert s.launch_count() == (1 if resident == "1" else n)
+    for a, b in zip(*got):
+        assert np.array_equal(a.view(np.int64), b.view(np.int64))
+
+
 # widths 128, 256, 384, 512 of the reverse kernel; segments of 1, 2 and more subcycles
 @pytest.mark.gpu
 @pytest.mark.parametrize("nx,ny,ndte,interval", [(3, 2, 3, 0), (64, 48, 11, 0), (64, 48, 11, 5),

@@ -164,8 +164,10 @@ struct TmaArgs {
 };
 constexpr int kTraceTiles = 256;
 
-// Allow the kernel's dynamic shared memory (call once per device).
-int tma_prepare(int device);
+// Allow the kernel's dynamic shared memory (call once per device).  *short_of:
+// the registers a thread that its roles need, where it was compiled with fewer
+// (cudaErrorInvalidKernelImage), else 0.
+cudaError_t tma_prepare(int *short_of);
 // binaryVersion of the subcycle kernel on the current device (100 = sm_100a).
 cudaError_t tma_binary_version(int *version);
 // What the wait that left `code` in the error word was waiting for.

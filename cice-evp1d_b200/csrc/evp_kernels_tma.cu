@@ -891,23 +891,24 @@ void launch_dep_probe(int *err, const unsigned *counter, unsigned long long limi
 }
 
 using TmaKernel = void (*)(TmaArgs, Params);
-constexpr int kTmaKernels = 6;
-const TmaKernel kTmaAll[kTmaKernels] = {
+const TmaKernel kTmaAll[] = {
     k_tma<false, false, false>, k_tma<true, false, false>, k_tma<false, true, false>,
     k_tma<true, true, false>,   k_tma<false, false, true>, k_tma<false, true, true>};
 
-int tma_prepare(int device) {
-  const int bytes = (int)smem_bytes();
-  cudaError_t e = cudaSuccess;
-  for (int i = 0; i < kTmaKernels && e == cudaSuccess; i++) {
+cudaError_t tma_prepare(int *short_of) {
+  *short_of = 0;
+  for (TmaKernel k : kTmaAll) {
     cudaFuncAttributes at;
-    e = cudaFuncGetAttributes(&at, kTmaAll[i]);
-    if (e == cudaSuccess && at.numRegs < kLaunchRegs) e = cudaErrorInvalidKernelImage;
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kTmaAll[i], cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e = cudaFuncGetAttributes(&at, k);
+    if (e != cudaSuccess) return e;
+    if (at.numRegs < kLaunchRegs) {
+      *short_of = kLaunchRegs;
+      return cudaErrorInvalidKernelImage;
+    }
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes());
+    if (e != cudaSuccess) return e;
   }
-  (void)device;
-  return e == cudaSuccess ? 0 : (int)e;
+  return cudaSuccess;
 }
 
 bool tma_can_persist(int device, int nruns) {

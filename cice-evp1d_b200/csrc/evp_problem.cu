@@ -110,8 +110,12 @@ int problem_create(DeviceProblem *d, int device, const TilePlan &plan,
   CUDA_TRY(cudaSetDevice(device));
   CUDA_TRY(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking));
   CUDA_TRY(cudaDeviceGetAttribute(&d->nctas, cudaDevAttrMultiProcessorCount, device));
-  if (tma_prepare(device) != 0)
-    return error(EVP1D_ERR_CUDA, "cannot enable %d bytes of shared memory", 0);
+  int short_of;
+  const cudaError_t e = tma_prepare(&short_of);
+  if (short_of)
+    return error(EVP1D_ERR_CUDA, "the subcycle kernel was compiled with fewer than the %d "
+                 "registers a thread that its roles share out", short_of);
+  if (e != cudaSuccess) return error(EVP1D_ERR_CUDA, "subcycle kernel: %s", cudaGetErrorString(e));
   if (res.nblocks > 0 && resident_prepare(device, res.quad, res.cls, res.nblocks)) {
     d->res_quad = res.quad;
     d->res_blocks = res.nblocks;

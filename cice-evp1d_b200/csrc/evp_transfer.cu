@@ -16,7 +16,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -399,6 +401,23 @@ cudaError_t copy_chunked(const std::vector<CopyItem> &items, bool up, char *stag
   return (cudaError_t)failed.load();
 }
 
+// One item by the copy engine's own call.  It refuses ordinary memory of which
+// a part is registered: that goes by way of other memory.
+cudaError_t copy_plain(const CopyItem &it, bool up, cudaStream_t st) {
+  cudaError_t e = up ? cudaMemcpyAsync(it.dev, it.host, it.bytes, cudaMemcpyHostToDevice, st)
+                     : cudaMemcpyAsync(it.host, it.dev, it.bytes, cudaMemcpyDeviceToHost, st);
+  if (e != cudaErrorInvalidValue || it.kind != kPageable) return e;
+  cudaGetLastError();
+  std::unique_ptr<char[]> way(new (std::nothrow) char[it.bytes]);
+  if (!way) return cudaErrorMemoryAllocation;
+  if (up) memcpy(way.get(), it.host, it.bytes);
+  e = up ? cudaMemcpyAsync(it.dev, way.get(), it.bytes, cudaMemcpyHostToDevice, st)
+         : cudaMemcpyAsync(way.get(), it.dev, it.bytes, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && !up) memcpy(it.host, way.get(), it.bytes);
+  return e;
+}
+
 // Every item: pageable ones in chunks where the staging buffer is free and
 // they are large, the others by the copy engine's own call.  Up: queued on
 // return, and pageable memory is no longer read; down: queued (pageable:
@@ -412,9 +431,7 @@ cudaError_t copy_items(const std::vector<CopyItem> &items, bool up, int device, 
       total += it.bytes;
       continue;
     }
-    const cudaError_t e =
-        up ? cudaMemcpyAsync(it.dev, it.host, it.bytes, cudaMemcpyHostToDevice, st)
-           : cudaMemcpyAsync(it.host, it.dev, it.bytes, cudaMemcpyDeviceToHost, st);
+    const cudaError_t e = copy_plain(it, up, st);
     if (e != cudaSuccess) return e;
   }
   if (own.empty()) return cudaSuccess;
@@ -425,9 +442,7 @@ cudaError_t copy_items(const std::vector<CopyItem> &items, bool up, int device, 
     return e;
   }
   for (const CopyItem &it : own) {
-    const cudaError_t e =
-        up ? cudaMemcpyAsync(it.dev, it.host, it.bytes, cudaMemcpyHostToDevice, st)
-           : cudaMemcpyAsync(it.host, it.dev, it.bytes, cudaMemcpyDeviceToHost, st);
+    const cudaError_t e = copy_plain(it, up, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -84,6 +84,37 @@ def test_partly_registered_arrays_are_copied():
         assert np.array_equal(a[k], b[k]), k
 
 
+def test_partly_registered_arrays_without_the_staging():
+    """The same where the staging buffer is not used (device memory among the
+    arrays): cudaMemcpyAsync refuses such ranges."""
+    import torch
+    rt = torch.cuda.cudart()
+    pr = problem(131, 77)
+    ref = evp1d.FieldSet.from_problem(pr, want_str=True)
+    fs = evp1d.FieldSet.from_problem(pr, want_str=True)
+    there = torch.from_numpy(fs.dyn["uocn"]).cuda()
+    fs.c.uocn = C.cast(C.c_void_p(there.data_ptr()), _D)
+    torch.cuda.synchronize()
+    big = np.zeros(1 << 16)
+    at = (-big.ctypes.data // 8) % 512
+    first = big[at:at + pr.na]
+    first[:] = pr.f["strength"]
+    fs.c.strength = first.ctypes.data_as(_D)
+    mid = (fs.uvel.ctypes.data + 4095) // 4096 * 4096
+    assert int(rt.cudaHostRegister(first.ctypes.data, 4096, 0)) == 0
+    assert int(rt.cudaHostRegister(mid, 4096, 0)) == 0
+    try:
+        with evp1d.EVP1D.from_problem(pr, ndte=3) as s:
+            s.run(3, ref)
+            s.run(3, fs)
+    finally:
+        rt.cudaHostUnregister(first.ctypes.data)
+        rt.cudaHostUnregister(mid)
+    a, b = bits(ref), bits(fs)
+    for k in FIELDS:
+        assert np.array_equal(a[k], b[k]), k
+
+
 @pytest.mark.parametrize("pinned", [False, True])
 def test_batched_positions(pinned):
     """A batched call's velocities and str, halo slots between the members."""

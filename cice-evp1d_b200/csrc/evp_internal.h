@@ -70,8 +70,7 @@ struct DeviceProblem {
   int32_t *tile_of_quad = nullptr;  // tile of slots 4q..4q+3
   // batched: caller's position of each list point, then each halo slot
   int32_t *uv_pos = nullptr;
-  // page-locked copy of the error word (pinned_word; null: none was left)
-  int *err_host = nullptr;
+  int *err_host = nullptr;  // page-locked copy of the error word (pinned_word)
   bool pins = false;        // holds a reference to the page-locked pool
   unsigned pin_gen = 0;     // as it was then
   int32_t *nb[6] = {};  // ee ne se nw sw sse, slot space
@@ -148,12 +147,13 @@ struct DownloadFields {
 // order); waits for the stream.
 int problem_gather_to_host(DeviceProblem *d, int n, const double *const *src,
                            double *const *host);
-// Page-locked memory shared by the handles of the process, allocated on first
-// use (a page-locking call takes 2.5 ms, however small) and freed with the
-// last handle: a page of words, one per handle, and one staging buffer of
+// Page-locked memory shared by the handles of the process, allocated once
+// their calls have made enough copies without it and freed with the last
+// handle: a page of words, one per handle, and one staging buffer of
 // kPinnedStage bytes that a call borrows.  All are safe from several threads.
-void pinned_hold(DeviceProblem *d);     // takes a reference and a word
+void pinned_hold(DeviceProblem *d);  // takes a reference
 void pinned_release(DeviceProblem *d);
+int *pinned_word(DeviceProblem *d);  // the handle's word; null: none (yet)
 // Whether the GPU can address the `bytes` bytes of host memory at p
 // (page-locked or managed, the whole range, `align`ed); *dev: at which address.
 bool device_view(const void *p, size_t bytes, size_t align, void **dev);

@@ -427,7 +427,7 @@ cudaError_t problem_launch_resident(DeviceProblem *d, const Params &p, int nsub,
 
 int problem_take_error(DeviceProblem *d, int *code) {
   int v = 0;
-  int *to = d->err_host ? d->err_host : &v;
+  int *word = pinned_word(d), *to = word ? word : &v;
   CUDA_TRY(cudaMemcpyAsync(to, d->err, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
   CUDA_TRY(cudaStreamSynchronize(d->stream));
   v = *to;

@@ -6,9 +6,10 @@
 // once, in the caller's order: k_upload takes a point's 29 values, skip flags
 // included, and writes every place they go to (both state sets, the
 // slot-ordered inputs, the constant blocks); k_download gathers the results.
-// Other arrays pass through page-locked staging: a small call's by one copy by
-// the host and the same kernels; a large call's in chunks that several host
-// threads copy while the copy engine moves others to or from device staging.
+// Other arrays pass through page-locked staging, once a program's calls have
+// paid for it: a small call's by one copy by the host and the same kernels; a
+// large call's in chunks that several host threads copy while the copy engine
+// moves others to or from device staging.  Before that they go by cudaMemcpyAsync.
 //
 // What bounds it: the host link for large calls; for small ones it was the
 // number of copies (31 up, 17 down, about 2 us each, and a dozen kernels
@@ -203,34 +204,65 @@ PtrAttrs ptr_attrs() {
   return f;
 }
 
+// One page-locked block: kWords error words, then the staging buffer.
+// Page-locking it takes 4 to 10 ms (one page: 2.5), during which no other CUDA
+// call of the process gets on, so a program's first calls go without it: copies
+// by cudaMemcpyAsync from and to ordinary memory, each about 5 us dearer (and 5
+// us per 128 KB), and the block comes once they would have paid for it.  First
+// transfers of a handle in ordinary memory, 64x48 and 400x300, ms: 4 and 9 with
+// the block, 0.8 and 2.7 without; a handle's creation 7 and 4 ms at 64x48.
 struct PinnedPool {
   static constexpr int kWords = 1024;
+  static constexpr size_t kPays = 1000, kItem = 128u << 10;
   std::mutex m;
-  unsigned gen = 0;  // counts the pool's memory: handles of an older one hold nothing
+  unsigned gen = 0;  // counts the blocks: handles of an older one hold nothing
   int refs = 0;
-  int *words = nullptr;
+  size_t owed = 0;   // copies made without the block, in units of 5 us
+  char *block = nullptr;
   bool used[kWords] = {};
-  void *stage = nullptr;
   bool lent = false;
+
+  int *words() { return reinterpret_cast<int *>(block); }
+  char *stage() { return block + kWords * sizeof(int); }
+  // Whether the block is there, for a call that would make `copies` copies of
+  // `bytes` in all without it.
+  bool ready(size_t copies, size_t bytes) {
+    if (block || refs == 0) return block != nullptr;
+    owed += copies + bytes / kItem;
+    if (owed < kPays) return false;
+    owed = 0;
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, kWords * sizeof(int) + kPinnedStage, cudaHostAllocPortable) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    block = static_cast<char *>(p);
+    return true;
+  }
+  void forget() {
+    gen++;
+    refs = 0;
+    owed = 0;
+    block = nullptr;
+    lent = false;
+    for (bool &u : used) u = false;
+  }
 };
 PinnedPool &pool() {
   static PinnedPool p;
   return p;
 }
 
-// The staging buffer, or null while another call has it (the caller then
-// takes device staging).
-void *borrow_stage() {
+// The staging buffer for a call of so many copies and bytes, or null where it
+// does not pay yet or while another call has it (the caller then takes device
+// staging).
+char *borrow_stage(size_t copies, size_t bytes) {
   PinnedPool &p = pool();
   std::lock_guard<std::mutex> lock(p.m);
-  if (p.lent) return nullptr;
-  if (!p.stage && cudaHostAlloc(&p.stage, kPinnedStage, cudaHostAllocPortable) != cudaSuccess) {
-    cudaGetLastError();
-    p.stage = nullptr;
-    return nullptr;
-  }
+  if (p.lent || !p.ready(copies, bytes)) return nullptr;
   p.lent = true;
-  return p.stage;
+  return p.stage();
 }
 
 void return_stage() {
@@ -247,31 +279,14 @@ void pinned_hold(DeviceProblem *d) {
   // A reset of the device (cudaDeviceReset) takes the memory away from under
   // handles that were not finalized: the pool starts anew.
   cudaPointerAttributes at;
-  if (p.words && (cudaPointerGetAttributes(&at, p.words) != cudaSuccess ||
+  if (p.block && (cudaPointerGetAttributes(&at, p.block) != cudaSuccess ||
                   at.type != cudaMemoryTypeHost)) {
     cudaGetLastError();
-    p.gen++;
-    p.refs = 0;
-    p.words = nullptr;
-    p.stage = nullptr;
-    p.lent = false;
-    for (bool &u : p.used) u = false;
+    p.forget();
   }
   p.refs++;
   d->pins = true;
   d->pin_gen = p.gen;
-  if (!p.words && cudaHostAlloc((void **)&p.words, sizeof(int) * PinnedPool::kWords,
-                                cudaHostAllocPortable) != cudaSuccess) {
-    cudaGetLastError();
-    p.words = nullptr;
-    return;
-  }
-  for (int k = 0; k < PinnedPool::kWords; k++)
-    if (!p.used[k]) {
-      p.used[k] = true;
-      d->err_host = p.words + k;
-      return;
-    }
 }
 
 void pinned_release(DeviceProblem *d) {
@@ -280,15 +295,24 @@ void pinned_release(DeviceProblem *d) {
   std::lock_guard<std::mutex> lock(p.m);
   d->pins = false;
   if (d->pin_gen != p.gen) return;
-  if (d->err_host) p.used[d->err_host - p.words] = false;
+  if (d->err_host) p.used[d->err_host - p.words()] = false;
   d->err_host = nullptr;
   if (--p.refs > 0) return;
-  if (p.words) cudaFreeHost(p.words);
-  if (p.stage && !p.lent) {
-    cudaFreeHost(p.stage);
-    p.stage = nullptr;
-  }
-  p.words = nullptr;
+  if (p.block) cudaFreeHost(p.block);
+  p.forget();
+}
+
+int *pinned_word(DeviceProblem *d) {
+  if (d->err_host || !d->pins) return d->err_host;
+  PinnedPool &p = pool();
+  std::lock_guard<std::mutex> lock(p.m);
+  if (d->pin_gen != p.gen || !p.ready(1, sizeof(int))) return nullptr;
+  for (int k = 0; k < PinnedPool::kWords && !d->err_host; k++)
+    if (!p.used[k]) {
+      p.used[k] = true;
+      d->err_host = p.words() + k;
+    }
+  return d->err_host;
 }
 
 namespace {
@@ -435,7 +459,7 @@ cudaError_t copy_items(const std::vector<CopyItem> &items, bool up, int device, 
     if (e != cudaSuccess) return e;
   }
   if (own.empty()) return cudaSuccess;
-  char *stage = total >= kThreadBytes ? static_cast<char *>(borrow_stage()) : nullptr;
+  char *stage = total >= kThreadBytes ? borrow_stage(own.size(), total) : nullptr;
   if (stage) {
     const cudaError_t e = copy_chunked(own, up, stage, device, st);
     return_stage();
@@ -507,7 +531,7 @@ struct Placer {
       return;
     }
     if (staged.empty() || foreign || total > kStagedDirect) return;
-    char *base = static_cast<char *>(borrow_stage());
+    char *base = borrow_stage(staged.size(), total);
     if (!base) return;
     pinned = true;
     for (Item &it : staged) *it.dev = base + it.off;

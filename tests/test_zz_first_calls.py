@@ -1,0 +1,62 @@
+"""Page-locked memory that handles share comes once a program's calls pay for it.
+
+A first call on a new handle must not wait for it (4 to 10 ms, with every other
+CUDA call of the process); calls before, at and after it must give the same
+bits, small (staged whole), in chunks, with an error word of either kind."""
+import time
+
+import numpy as np
+import pytest
+
+import evp1d
+from evp1d import synth
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("stress", "uvel", "vvel", "strintx", "strinty", "Cb", "str")
+
+
+def _problem(nx, ny):
+    return synth.to_1d(synth.make_grid(nx, ny, seed=8, ndte=3, curvilinear=True))
+
+
+def _lock_ms():
+    t0 = time.perf_counter()
+    evp1d.pinned_empty(1 << 20)  # 8 MiB
+    return 1e3 * (time.perf_counter() - t0)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+def test_first_call_does_not_page_lock(pinned):
+    """The quickest of ten first calls against the quickest of ten page-locks
+    (the calls take a tenth of it)."""
+    pr = _problem(64, 48)
+    fs = evp1d.FieldSet.from_problem(pr, pinned=pinned)
+    first = []
+    for _ in range(10):
+        with evp1d.EVP1D.from_problem(pr, ndte=3) as s:
+            t0 = time.perf_counter()
+            s.run(3, fs)
+            first.append(1e3 * (time.perf_counter() - t0))
+    assert min(first) < 0.5 * min(_lock_ms() for _ in range(10)), first
+
+
+@pytest.mark.parametrize("nx,ny,calls", [(97, 61, 40), (203, 151, 24), (400, 300, 10)])
+def test_same_bits_before_and_after(nx, ny, calls):
+    pr = _problem(nx, ny)
+    fs = evp1d.FieldSet.from_problem(pr, want_str=True)
+    ref = None
+    with evp1d.EVP1D.from_problem(pr, ndte=3) as s:
+        for k in range(calls):
+            fs.refill(pr)
+            fs.str[:] = 7.0
+            s.run(3, fs)
+            got = {f: np.asarray(getattr(fs, f)).view(np.int64).copy() for f in FIELDS}
+            ref = ref or got
+            for f in FIELDS:
+                assert np.array_equal(got[f], ref[f]), (k, f)
+        s.debug_wait_timeout(5_000_000)  # by now reported through the shared word
+        with pytest.raises(evp1d.EVP1DError) as e:
+            s.synchronize()
+        assert e.value.code == -5
+        s.synchronize()

@@ -140,7 +140,7 @@ __device__ __forceinline__ void str_lam(const AdjArgs &a, int t, int w, double &
 }
 
 template <bool kOne>
-__global__ void __launch_bounds__(kSweepThreads, 768 / kSweepThreads)  // 80 registers
+__global__ void __launch_bounds__(kSweepThreads, 768 / kSweepThreads)  // 80 registers, 40 bytes spilled
 k_adj_stepu(AdjArgs a, Params p, const double *__restrict__ u0, const double *__restrict__ v0,
             const double *__restrict__ u1, const double *__restrict__ v1) {
   // launched as a programmatic dependent: the previous kernel's results

@@ -24,7 +24,11 @@
 // loads complete.
 //
 // What bounds it: the dependent chain through both reversals and one exchange
-// a subcycle, 3 us where the two kernels of a subcycle took 8 (18.7k points).
+// a subcycle, 3.3 us where the two kernels of a subcycle took 8 (18.7k points).
+// Blocks of 512 hold 128 registers a thread, too few for the 12 stress adjoints
+// beside a corner's reversal: 580 bytes of a thread are spilled, to L1 (blocks
+// of 384: 44 bytes); 7.3 us a subcycle at 54k points, against 10.3 in the two
+// kernels.
 #include <cstdint>
 
 #include "evp_adjoint_math.cuh"

@@ -1,8 +1,9 @@
 // evp_resident.h -- host-side plan of the resident solver (internal).
 //
-// Where a problem is small enough for one point per thread, a call's
-// subcycles run in one launch whose CTAs keep their points on chip from the
-// first subcycle to the last (evp_kernels_resident.cu).  The list is cut into
+// Where a problem fits the SMs' registers and shared memory (up to about 98k
+// points on 148), a call's subcycles run in one launch whose CTAs keep their
+// points on chip from the first subcycle to the last
+// (evp_kernels_resident.cu).  The list is cut into
 // blocks, one per CTA.  A block owns its points and recomputes `stress` at
 // its forward halo, the nw/sw/sse neighbours other blocks own, so that only
 // velocities travel between blocks: those of points that another block's

@@ -129,7 +129,7 @@ int evp1d_init_batched(evp1d_t **handle, int nmembers, const int32_t *na,
                        const evp1d_params *params, int device);
 
 /* Time the kernel variants (TMA-fed with and without L2 prefetch, plain
- * loads) for `nsub` subcycles on the uploaded state, keep the fastest for
+ * loads, on chip where the problem fits) for `nsub` subcycles on the uploaded state, keep the fastest for
  * this handle and restore the state.  `chosen` (may be NULL) receives a
  * description of the choice.  Needs a prior evp1d_upload. */
 int evp1d_autotune(evp1d_t *handle, int nsub, char *chosen, int len);
@@ -225,7 +225,9 @@ int evp1d_debug_trace(evp1d_t *handle, long long *out, int n);
 
 /* Name of the subcycle kernel the handle runs: "fused-tile-tma" (default,
  * TMA-fed persistent kernel) or "fused-tile" (plain loads; selected by the
- * environment variable EVP1D_PATH=fused at evp1d_init). */
+ * environment variable EVP1D_PATH=fused at evp1d_init).  The first is also the
+ * answer for a handle whose calls of two or more subcycles run on chip in one
+ * launch (problems of up to about 98k points): it runs its single subcycles. */
 const char *evp1d_kernel_path(evp1d_t *handle);
 
 /* The handle's CUDA stream (a cudaStream_t), for event timing by callers. */
@@ -252,7 +254,14 @@ int evp1d_binary_version(int device);
  * asynchronous; pageable arrays work too, at lower speed.  A caller that keeps
  * its fields in such memory across timesteps (as CICE keeps its module
  * arrays) saves most of the transfer time of evp1d_run.  No counterpart in the
- * reference. */
+ * reference.
+ *
+ * For arrays elsewhere (the skip flags among them) the library keeps one block
+ * of 8 MiB page-locked, shared by the process's handles, from the call on at
+ * which the copies made without it would have paid for it (that call takes 4
+ * to 10 ms more) until the last handle is finalized.  Pageable transfers of
+ * 2 MiB and more then run on up to eight host threads each, this one and
+ * others that end with the transfer. */
 int evp1d_host_alloc(void **ptr, size_t bytes);
 int evp1d_host_free(void *ptr);
 

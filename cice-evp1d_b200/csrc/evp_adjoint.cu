@@ -955,13 +955,13 @@ int evp1d_adjoint_gradients(evp1d_t *h, const evp1d_grads *g) {
                  "a bounded device-side wait ran out (code %d: %s); the gradients are not valid",
                  code, tma_wait_name(code));
   const size_t bn = sizeof(double) * (size_t)d.na;
-  struct Out {
-    const double *src;
-    double *host;
-  };
-  std::vector<Out> outs;
-  auto want = [&](double *host, const double *src) {
-    if (host) outs.push_back({src, host});
+  const double *src[20];  // all that evp1d_grads names
+  double *host[20];
+  int n = 0;
+  auto want = [&](double *to, const double *from) {
+    if (!to) return;
+    src[n] = from;
+    host[n++] = to;
   };
   want(g->strength, A.g[kGStrength]);
   want(g->Cw, A.g[kGCw]);
@@ -977,13 +977,7 @@ int evp1d_adjoint_gradients(evp1d_t *h, const evp1d_grads *g) {
     if (g->uvel_init) memset(g->uvel_init, 0, bn);
     if (g->vvel_init) memset(g->vvel_init, 0, bn);
   }
-  std::vector<const double *> src;
-  std::vector<double *> host;
-  for (const Out &o : outs) {
-    src.push_back(o.src);
-    host.push_back(o.host);
-  }
-  return problem_gather_to_host(&d, (int)outs.size(), src.data(), host.data());
+  return problem_gather_to_host(&d, n, src, host);
 }
 
 int evp1d_adjoint(evp1d_t *h, const double *lam_uvel, const double *lam_vvel,

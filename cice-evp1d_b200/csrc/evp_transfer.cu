@@ -459,12 +459,13 @@ cudaError_t copy_items(const std::vector<CopyItem> &items, bool up, int device, 
     if (e != cudaSuccess) return e;
   }
   if (own.empty()) return cudaSuccess;
-  char *stage = total >= kThreadBytes ? borrow_stage(own.size(), total) : nullptr;
-  if (stage) {
-    const cudaError_t e = copy_chunked(own, up, stage, device, st);
-    return_stage();
-    return e;
-  }
+  struct Loan {
+    char *stage;
+    ~Loan() {
+      if (stage) return_stage();
+    }
+  } loan{total >= kThreadBytes ? borrow_stage(own.size(), total) : nullptr};
+  if (loan.stage) return copy_chunked(own, up, loan.stage, device, st);
   for (const CopyItem &it : own) {
     const cudaError_t e = copy_plain(it, up, st);
     if (e != cudaSuccess) return e;
@@ -544,9 +545,16 @@ struct Placer {
   }
 };
 
+// The lists of a call's arrays could not grow (no exception may leave a C entry
+// point).  The copies queued so far end first.
+int no_memory(DeviceProblem *d) {
+  cudaStreamSynchronize(d->stream);
+  return error(EVP1D_ERR_NOMEM, "out of memory");
+}
+
 }  // namespace
 
-int problem_upload(DeviceProblem *d, const UploadFields &f, double rhow, bool wait) {
+int problem_upload(DeviceProblem *d, const UploadFields &f, double rhow, bool wait) try {
   if (d->na == 0) return EVP1D_OK;
   cudaStream_t st = d->stream;
   UploadArgs a;
@@ -616,9 +624,11 @@ int problem_upload(DeviceProblem *d, const UploadFields &f, double rhow, bool wa
   if (wait || P.pinned) CUDA_TRY(cudaStreamSynchronize(st));
   d->cur = 0;
   return EVP1D_OK;
+} catch (const std::bad_alloc &) {
+  return no_memory(d);
 }
 
-int problem_download(DeviceProblem *d, const DownloadFields &f, int *code) {
+int problem_download(DeviceProblem *d, const DownloadFields &f, int *code) try {
   *code = 0;
   if (d->na == 0) return EVP1D_OK;
   cudaStream_t st = d->stream;
@@ -664,10 +674,12 @@ int problem_download(DeviceProblem *d, const DownloadFields &f, int *code) {
   if (P.pinned)
     for (const Placer::Item &it : P.staged) memcpy(const_cast<void *>(it.host), *it.dev, it.bytes);
   return EVP1D_OK;
+} catch (const std::bad_alloc &) {
+  return no_memory(d);
 }
 
 int problem_gather_to_host(DeviceProblem *d, int n, const double *const *src,
-                           double *const *host) {
+                           double *const *host) try {
   const size_t bytes = (size_t)d->na * sizeof(double);
   cudaStream_t st = d->stream;
   for (int at = 0; at < n; at += kMaxBatch) {
@@ -692,6 +704,8 @@ int problem_gather_to_host(DeviceProblem *d, int n, const double *const *src,
         memcpy(const_cast<void *>(it.host), *it.dev, it.bytes);
   }
   return EVP1D_OK;
+} catch (const std::bad_alloc &) {
+  return no_memory(d);
 }
 
 }  // namespace evp

@@ -19,8 +19,9 @@
 // sweep in 80-bit arithmetic on the same velocities (relative 2-norm, 203 x 151,
 // 120 subcycles, two seeds): 0.8 to 1.4e-15 in every gradient, where the
 // compiler's own contraction of these expressions gave 2.0 to 3.9e-15 and plain
-// operations 2.9 to 5.1e-15.  (A restatement in plain 64-bit arithmetic is itself
-// 3 to 5e-15 off, which is what a comparison with it shows.)
+// operations 2.9 to 5.1e-15; on 800 x 600, 500 subcycles, 1.8 to 3.1e-15 against
+// 0.9 to 2.0e-14.  (A restatement in plain 64-bit arithmetic is itself 3 to 5e-15
+// off in the first case, which is what a comparison with it shows.)
 //
 // The forward values that choose a branch -- Delta against DminTarea and 0,
 // |u| and |u_ocn - u| against 0 -- are recomputed with every +, -, * rounded
